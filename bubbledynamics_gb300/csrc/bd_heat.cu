@@ -216,6 +216,47 @@ __global__ void __launch_bounds__(128) heat_step4_kernel(const HeatArgs<float> a
     }
 }
 
+// Initial fields and outputs are formed on the device: the callers' arrays are
+// double, the FP32 run keeps floats, and one host thread needs 118 ms for the
+// 25 M cells that these kernels convert in under a millisecond (bound by the
+// copies over the host link).  One thread per cell; host rows are nx long.
+
+// T(0) and the dose before the first step (T:232-257).  T_src (nullable) holds
+// this slab's initial temperatures; T_init / d_init are the per-material values.
+struct HeatInit {
+    double T_init[BD_MAX_MATERIALS], d_init[BD_MAX_MATERIALS];
+};
+
+template <class real>
+__global__ void heat_init_T_kernel(real* __restrict__ Ta, real* __restrict__ Tb, const double* __restrict__ T_src,
+                                   const HeatInit in, const int* __restrict__ plane_mat,
+                                   const uint8_t* __restrict__ matmap, long long plane, long long n, double T_ref) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int m = matmap ? matmap[i] : (plane_mat ? plane_mat[i / plane] : 0);
+    const double T = T_src ? T_src[i] : in.T_init[m];
+    const real v = (real)(T - T_ref);
+    Ta[i] = v;
+    Tb[i] = v;
+}
+
+__global__ void heat_init_dose_kernel(double* __restrict__ TD, const HeatInit in, const int* __restrict__ plane_mat,
+                                      const uint8_t* __restrict__ matmap, long long plane, long long n) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    TD[i] = in.d_init[matmap ? matmap[i] : (plane_mat ? plane_mat[i / plane] : 0)];
+}
+
+__global__ void heat_narrow_kernel(float* __restrict__ dst, const double* __restrict__ src, long long n) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i < n) dst[i] = (float)src[i];
+}
+
+__global__ void heat_widen_kernel(double* __restrict__ dst, const float* __restrict__ src, long long n, double T_ref) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i < n) dst[i] = T_ref + (double)src[i];
+}
+
 __global__ void heat_advance_kernel(long long* step_base, int n) {
     if (threadIdx.x == 0 && blockIdx.x == 0) *step_base += n;
 }
@@ -299,7 +340,7 @@ struct HeatPlan {
     int64_t step = 0;                              // steps done
     static constexpr int leg_cap = 4096;
     std::vector<int64_t> leg_end;
-    PoolBuf pm, mm, shd, sb;
+    PoolBuf pm, mm, shd, sb, stage;                // stage: doubles of the largest slab, for conversions
     std::vector<HeatSlab> sl;
     HeatArgs<float> af{};
     HeatArgs<double> ad{};
@@ -343,23 +384,20 @@ struct HeatPlan {
         if (max_steps > 0 && max_steps < nsteps) nsteps = max_steps;
         std::vector<int2> sh(std::max<int64_t>(nsteps, 1));
         for (int64_t s = 0; s < nsteps; ++s) sh[s] = make_int2(sx[s], sy[s]);
-        // initial fields (T:232-257)
-        auto mat_of = [&](long long i) -> int {
-            int iz = (int)(i / plane);
-            int m = th->material_map ? th->material_map[i] : (th->plane_material ? th->plane_material[iz] : 0);
-            if (m < 0 || m >= th->n_materials) fail(BD_ERR_INVALID_ARG, "material index out of range");
-            return m;
-        };
-        T_ref = f64 ? 0.0 : th->T_ref;
-        std::vector<double> T0(n), TD0(n);
-        for (long long i = 0; i < n; ++i) {
-            const bd_thermal_material& mt = th->mat[mat_of(i)];
-            T0[i] = th->T_start ? th->T_start[i] : mt.T_init;
-            TD0[i] = th->dose_start ? th->dose_start[i]
-                                    : (th->dose_init ? std::pow(4.0, mt.T_init - 273.15 - 43.0) * th->dt : 0.0);   // T:246, T:252
+        // material of every cell (or plane) in range
+        if (th->material_map) {
+            uint8_t top = 0;
+            for (long long i = 0; i < n; ++i) top = std::max(top, th->material_map[i]);
+            if (top >= th->n_materials) fail(BD_ERR_INVALID_ARG, "material index out of range");
+        } else if (th->plane_material) {
+            for (int iz = 0; iz < nz; ++iz)
+                if (th->plane_material[iz] < 0 || th->plane_material[iz] >= th->n_materials)
+                    fail(BD_ERR_INVALID_ARG, "material index out of range");
         }
+        T_ref = f64 ? 0.0 : th->T_ref;
         esz = f64 ? 8 : 4;
         std::vector<HeatSlab>(owned.size()).swap(sl);
+        long long most = 0;
         for (size_t k = 0; k < owned.size(); ++k) {
             HeatSlab& S = sl[k];
             S.zb = owned[k].first;
@@ -368,41 +406,75 @@ struct HeatPlan {
             S.hi = S.ze < nz ? S.ze + 1 : nz;
             S.nzl = S.hi - S.lo;
             S.nl = plane * S.nzl;
+            most = std::max(most, S.nl);
         }
+        cudaStream_t q = ctx->stream;
+        // whatever ends this block, the copies from the callers' arrays and from sh are done by then
+        struct Drain {
+            cudaStream_t s;
+            ~Drain() { cudaStreamSynchronize(s); }
+        } drain{q};
         shd.alloc(ctx, sh.size() * sizeof(int2));
         sb.alloc(ctx, 64);
-        BD_CUDA(cudaMemcpy(shd.p, sh.data(), sh.size() * sizeof(int2), cudaMemcpyHostToDevice));
-        for (HeatSlab& S : sl) {
-            S.Ta.alloc(ctx, S.nl * esz); S.Tb.alloc(ctx, S.nl * esz); S.Qd.alloc(ctx, S.nl * esz);
-            S.TDd.alloc(ctx, S.nl * 8);
-            const long long o = plane * S.lo;
-            if (f64) {
-                BD_CUDA(cudaMemcpy(S.Ta.p, T0.data() + o, S.nl * 8, cudaMemcpyHostToDevice));
-                BD_CUDA(cudaMemcpy(S.Tb.p, T0.data() + o, S.nl * 8, cudaMemcpyHostToDevice));
-                BD_CUDA(cudaMemcpy(S.Qd.p, Q + o, S.nl * 8, cudaMemcpyHostToDevice));
-            } else {
-                std::vector<float> tf(S.nl), qf(S.nl);
-                for (long long i = 0; i < S.nl; ++i) {
-                    tf[i] = (float)(T0[o + i] - T_ref);
-                    qf[i] = (float)Q[o + i];
-                }
-                BD_CUDA(cudaMemcpy(S.Ta.p, tf.data(), S.nl * 4, cudaMemcpyHostToDevice));
-                BD_CUDA(cudaMemcpy(S.Tb.p, tf.data(), S.nl * 4, cudaMemcpyHostToDevice));
-                BD_CUDA(cudaMemcpy(S.Qd.p, qf.data(), S.nl * 4, cudaMemcpyHostToDevice));
-            }
-            BD_CUDA(cudaMemcpy(S.TDd.p, TD0.data() + o, S.nl * 8, cudaMemcpyHostToDevice));
-        }
+        if (!f64) stage.alloc(ctx, most * 8);
+        BD_CUDA(cudaMemcpyAsync(shd.p, sh.data(), sh.size() * sizeof(int2), cudaMemcpyHostToDevice, q));
         has_pm = th->plane_material != nullptr;
         has_mm = th->material_map != nullptr;
         if (has_pm) {
             pm.alloc(ctx, nz * 4);
-            BD_CUDA(cudaMemcpy(pm.p, th->plane_material, nz * 4, cudaMemcpyHostToDevice));
+            BD_CUDA(cudaMemcpyAsync(pm.p, th->plane_material, nz * 4, cudaMemcpyHostToDevice, q));
         }
         if (has_mm) {
             mm.alloc(ctx, n);
-            BD_CUDA(cudaMemcpy(mm.p, th->material_map, n, cudaMemcpyHostToDevice));
+            BD_CUDA(cudaMemcpyAsync(mm.p, th->material_map, n, cudaMemcpyHostToDevice, q));
         }
-        BD_CUDA(cudaMemset(sb.p, 0, 64));
+        BD_CUDA(cudaMemsetAsync(sb.p, 0, 64, q));
+        // initial fields (T:232-257)
+        HeatInit in;
+        std::memset(&in, 0, sizeof in);
+        for (int k = 0; k < th->n_materials; ++k) {
+            in.T_init[k] = th->mat[k].T_init;
+            in.d_init[k] = th->dose_init ? std::pow(4.0, th->mat[k].T_init - 273.15 - 43.0) * th->dt : 0.0;   // T:246, T:252
+        }
+        for (HeatSlab& S : sl) {
+            S.Ta.alloc(ctx, S.nl * esz); S.Tb.alloc(ctx, S.nl * esz); S.Qd.alloc(ctx, S.nl * esz);
+            S.TDd.alloc(ctx, S.nl * 8);
+            const long long o = plane * S.lo;
+            const int* spm = has_pm ? pm.as<int>() + S.lo : nullptr;
+            const uint8_t* smm = has_mm ? mm.as<uint8_t>() + o : nullptr;
+            const unsigned blocks = (unsigned)((S.nl + 255) / 256);
+            const double* T_src = nullptr;
+            if (th->T_start) {
+                void* to = f64 ? S.Tb.p : stage.p;
+                BD_CUDA(cudaMemcpyAsync(to, th->T_start + o, S.nl * 8, cudaMemcpyHostToDevice, q));
+                T_src = static_cast<const double*>(to);
+            }
+            if (f64 && T_src) {
+                BD_CUDA(cudaMemcpyAsync(S.Ta.p, S.Tb.p, S.nl * 8, cudaMemcpyDeviceToDevice, q));
+            } else if (f64) {
+                heat_init_T_kernel<double><<<blocks, 256, 0, q>>>(S.Ta.as<double>(), S.Tb.as<double>(), nullptr, in, spm,
+                                                                  smm, plane, S.nl, 0.0);
+                BD_LAUNCHED(ctx);
+            } else {
+                heat_init_T_kernel<float><<<blocks, 256, 0, q>>>(S.Ta.as<float>(), S.Tb.as<float>(), T_src, in, spm, smm,
+                                                                 plane, S.nl, T_ref);
+                BD_LAUNCHED(ctx);
+            }
+            if (f64) {
+                BD_CUDA(cudaMemcpyAsync(S.Qd.p, Q + o, S.nl * 8, cudaMemcpyHostToDevice, q));
+            } else {
+                BD_CUDA(cudaMemcpyAsync(stage.p, Q + o, S.nl * 8, cudaMemcpyHostToDevice, q));
+                heat_narrow_kernel<<<blocks, 256, 0, q>>>(S.Qd.as<float>(), stage.as<double>(), S.nl);
+                BD_LAUNCHED(ctx);
+            }
+            if (th->dose_start) {
+                BD_CUDA(cudaMemcpyAsync(S.TDd.p, th->dose_start + o, S.nl * 8, cudaMemcpyHostToDevice, q));
+            } else {
+                heat_init_dose_kernel<<<blocks, 256, 0, q>>>(S.TDd.as<double>(), in, spm, smm, plane, S.nl);
+                BD_LAUNCHED(ctx);
+            }
+        }
+        BD_CUDA(cudaStreamSynchronize(q));
         vec4 = !f64 && nx % 4 == 0;
         static int per_sm4 = 0;
         if (vec4 && !per_sm4) BD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm4, heat_step4_kernel, 128, 0));
@@ -540,24 +612,29 @@ struct HeatPlan {
         for (const HeatSlab& S : sl) {
             const PoolBuf& src = newest(S, steps);
             const long long off = plane * (S.zb - S.lo), cnt = plane * (S.ze - S.zb);
-            double* d = dst + plane * S.zb;
-            if (f64) {
-                BD_CUDA(cudaMemcpyAsync(d, static_cast<const double*>(src.p) + off, cnt * 8, cudaMemcpyDeviceToHost, s));
-                BD_CUDA(cudaStreamSynchronize(s));
-            } else {
-                std::vector<float> tf(cnt);
-                BD_CUDA(cudaMemcpyAsync(tf.data(), static_cast<const float*>(src.p) + off, cnt * 4,
-                                        cudaMemcpyDeviceToHost, s));
-                BD_CUDA(cudaStreamSynchronize(s));
-                for (long long i = 0; i < cnt; ++i) d[i] = T_ref + (double)tf[i];
+            const double* from = static_cast<const double*>(src.p) + off;
+            if (!f64) {
+                heat_widen_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, s>>>(
+                    stage.as<double>(), static_cast<const float*>(src.p) + off, cnt, T_ref);
+                BD_LAUNCHED(ctx);
+                from = stage.as<double>();
             }
+            double* d = dst + plane * S.zb;
+            host_populate(d, cnt * 8);   // while the steps before this copy run
+            BD_CUDA(cudaMemcpyAsync(d, from, cnt * 8, cudaMemcpyDeviceToHost, s));
         }
+        BD_CUDA(cudaStreamSynchronize(s));
     }
 
     void copy_dose(double* dst) {
-        for (const HeatSlab& S : sl)
-            BD_CUDA(cudaMemcpy(dst + plane * S.zb, static_cast<const double*>(S.TDd.p) + plane * (S.zb - S.lo),
-                               (size_t)plane * (S.ze - S.zb) * 8, cudaMemcpyDeviceToHost));
+        for (const HeatSlab& S : sl) {
+            double* d = dst + plane * S.zb;
+            const size_t bytes = (size_t)plane * (S.ze - S.zb) * 8;
+            host_populate(d, bytes);
+            BD_CUDA(cudaMemcpyAsync(d, static_cast<const double*>(S.TDd.p) + plane * (S.zb - S.lo), bytes,
+                                    cudaMemcpyDeviceToHost, ctx->stream));
+        }
+        BD_CUDA(cudaStreamSynchronize(ctx->stream));
     }
 };
 
@@ -597,6 +674,8 @@ static void heat_run(bd_context* ctx, const bd_thermal* th, const double* Q, con
         done = next;
     }
     BD_CUDA(cudaEventRecord(ctx->ev1, s));
+    host_populate(out->T_final, (size_t)P.n * 8);   // while the device steps
+    host_populate(out->dose, (size_t)P.n * 8);
     BD_CUDA(cudaEventSynchronize(ctx->ev1));
     float ms = 0;
     BD_CUDA(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));

@@ -989,8 +989,23 @@ __global__ void wv_q_kernel(const real* __restrict__ energy, const real* __restr
     }
 }
 
+// Pages of the output buffers that finish() writes (host_populate).
+static void populate_outputs(const WvSession& S, const bd_westervelt_outputs* o) {
+    const size_t bytes = (size_t)(S.own1 - S.own0) * S.plane * S.esz;
+    host_populate(o->p_final, bytes);
+    host_populate(o->peak, bytes);
+    host_populate(o->energy, bytes);
+    for (int j = 0; j < S.n_dft; ++j) {
+        const size_t at = ((size_t)j * S.dft_glob_cells + S.dft_glob_off) * S.esz, nb = (size_t)S.dcells * S.esz;
+        if (o->dft_re) host_populate(static_cast<char*>(o->dft_re) + at, nb);
+        if (o->dft_im) host_populate(static_cast<char*>(o->dft_im) + at, nb);
+    }
+    if (S.p.q_mode == BD_Q_REFERENCE) host_populate(o->Q, bytes / S.esz * 8);
+}
+
 static void finish(WvSession& S, bd_westervelt_outputs* o) {
     cudaStream_t st = S.ctx->stream;
+    populate_outputs(S, o);
     BD_CUDA(cudaStreamSynchronize(st));
     // owned planes only (a whole grid owns every plane)
     const size_t off = (size_t)S.own0 * S.plane * S.esz;
@@ -1757,11 +1772,13 @@ struct bd_westervelt {
 
 using namespace bd;
 
-static double timed_advance(WvSession& S, int64_t n) {
+// out: buffers whose pages are made present while the device steps (may be null)
+static double timed_advance(WvSession& S, int64_t n, const bd_westervelt_outputs* out = nullptr) {
     BD_CUDA(cudaEventRecord(S.ctx->ev0, S.ctx->stream));
     bool graph = S.p.graph_chunk >= 0;
     advance(S, n, graph);
     BD_CUDA(cudaEventRecord(S.ctx->ev1, S.ctx->stream));
+    if (out) populate_outputs(S, out);
     BD_CUDA(cudaEventSynchronize(S.ctx->ev1));
     float ms = 0;
     BD_CUDA(cudaEventElapsedTime(&ms, S.ctx->ev0, S.ctx->ev1));
@@ -2042,7 +2059,7 @@ bd_status bd_westervelt_run(bd_context* ctx, const bd_grid* grid, const bd_mediu
         ctx_check(ctx);
         bd_westervelt w;
         setup(w.S, ctx, grid, medium, source, params);
-        timed_advance(w.S, params->n_steps);
+        timed_advance(w.S, params->n_steps, out);
         finish(w.S, out);
         out->elapsed_ms = w.S.last_ms;
     });
