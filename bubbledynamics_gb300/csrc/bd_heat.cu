@@ -36,7 +36,9 @@ struct HeatMat {
 template <class real>
 struct HeatArgs {
     int nx, ny, nz, zb;
-    long long plane;
+    int px;                        // row pitch in cells (nx, or nx rounded up to whole 16-byte vectors)
+    int rev;                       // four-cell kernel: march the planes from the high end
+    long long plane;               // px * ny
     const real* __restrict__ Tin;
     real* __restrict__ Tout;
     const real* __restrict__ Q;
@@ -78,6 +80,43 @@ __device__ __forceinline__ double widen_pos(float x) {
     return __longlong_as_double(((long long)b << 29) + (896LL << 52));
 }
 
+// The FP64 adder behind a branch: asm volatile keeps the compiler from issuing it
+// on every path and selecting afterwards.
+__device__ __forceinline__ double dadd_slow(double d, double x) {
+    double r;
+    asm volatile("add.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(d), "d"(x));
+    return r;
+}
+
+// dose + inc as the FP64 adder rounds it.  An FP64 instruction holds its quarter
+// of an SM for 64 cycles a warp here (76 with all quarters busy): at one add per
+// cell and step that pipe alone needs 2.1 us per million cells.  For a dose of 1
+// to 2^30 times the increment the float's mantissa lands on whole units of the
+// dose's last place, the sum is exact unless it carries into the exponent, and
+// one integer multiply-add gives the adder's bits.  Everything else (a first
+// increment on zero, a carry, tiny increments, non-finite or negative values)
+// takes the adder.
+__device__ __forceinline__ double dose_add(double d, float inc) {
+    const long long D = __double_as_longlong(d);
+    const int b = __float_as_int(inc);
+    const int s = (b >> 23) + 925 - (int)(D >> 52);          // 29 - distance of the exponents
+    const long long sum = D + (long long)((unsigned long long)((b & 0x007fffff) | 0x00800000) * (1u << (s & 31)));
+    if ((unsigned)s <= 29u && b >= 0x00800000 && ((sum ^ D) >> 52) == 0) return __longlong_as_double(sum);
+    return dadd_slow(d, widen_pos(inc));
+}
+
+// Dose increment rate at x = T_C - 43 (T:99-102): 2x < x below 43 C
+__device__ __forceinline__ float dose_rate(float x) { return exp2f(fminf(2.0f * x, x)); }
+
+// T:85-87 (plus the Pennes term -w dt (T - T_art), zero in the reference), explicitly
+// rounded so that every FP32 kernel gives the same bits
+__device__ __forceinline__ float heat_cell(const HeatMat<float>& M, float tc, float sxy, float zz, float q) {
+    float t = __fmaf_rn(tc, M.a0, __fmul_rn(M.kxy, sxy));
+    t = __fmaf_rn(M.kz, zz, t);
+    t = __fmaf_rn(M.qc, q, t);
+    return __fadd_rn(t, M.wTa);
+}
+
 template <class real>
 __global__ void heat_step_kernel(const HeatArgs<real> a, int koff) {
     const int ix = blockIdx.x * blockDim.x + threadIdx.x;
@@ -88,8 +127,8 @@ __global__ void heat_step_kernel(const HeatArgs<real> a, int koff) {
     const int2 sh = a.shifts[step];
     const int ixa = ix - sh.x, iya = iy - sh.y;                  // T:61-62
     const bool qin = ixa >= 0 && ixa < a.nx && iya >= 0 && iya < a.ny;
-    const long long col = (long long)iy * a.nx + ix;
-    const long long colq = (long long)iya * a.nx + ixa;
+    const long long col = (long long)iy * a.px + ix;
+    const long long colq = (long long)iya * a.px + ixa;
     const int z0 = max(1, blockIdx.z * a.zb);
     const int z1 = min(a.nz - 1, blockIdx.z * a.zb + a.zb);
     if (z0 >= z1) return;
@@ -100,7 +139,9 @@ __global__ void heat_step_kernel(const HeatArgs<real> a, int koff) {
         const long long i = (long long)iz * a.plane + col;
         const int m = a.matmap ? a.matmap[i] : (a.plane_mat ? __ldg(a.plane_mat + iz) : 0);
         const HeatMat<real>& M = a.mat[m];
-        const real tn = tcv * M.a0 + M.kxy * sxy + M.kz * (tpv + tmv) + M.qc * q + M.wTa;
+        real tn;
+        if constexpr (sizeof(real) == 8) tn = tcv * M.a0 + M.kxy * sxy + M.kz * (tpv + tmv) + M.qc * q + M.wTa;
+        else tn = heat_cell(M, tcv, sxy, tpv + tmv, q);
         a.Tout[i] = tn;
         if (sizeof(real) == 8) {
             const double Tc = (double)tn - 273.15;                     // T:88
@@ -108,14 +149,14 @@ __global__ void heat_step_kernel(const HeatArgs<real> a, int koff) {
             a.TD[i] = a.TD[i] + (Tc < 43.0 ? pow(4.0, Tc - 43.0) : pow(2.0, Tc - 43.0)) * (double)a.dt;
         } else {
             const float x = (float)tn + a.T_refm43;                    // T_C - 43
-            const float inc = exp2f(x < 0.0f ? 2.0f * x : x) * (float)a.dt;
-            if (a.TD) a.TD[i] = a.TD[i] + widen_pos(inc);
+            const float inc = __fmul_rn(dose_rate(x), (float)a.dt);
+            if (a.TD) a.TD[i] = dose_add(a.TD[i], inc);
             else a.TDf[i] = df_add(a.TDf[i], inc);
         }
     };
     auto sxy_at = [&](int iz) {
         const long long i = (long long)iz * a.plane + col;
-        return __ldg(a.Tin + i - 1) + __ldg(a.Tin + i + 1) + __ldg(a.Tin + i + a.nx) + __ldg(a.Tin + i - a.nx);
+        return __ldg(a.Tin + i - 1) + __ldg(a.Tin + i + 1) + __ldg(a.Tin + i + a.px) + __ldg(a.Tin + i - a.px);
     };
     auto q_at = [&](int iz) {                                           // T:76-77
         return qin ? __ldg(a.Q + (long long)iz * a.plane + colq) : real(0);
@@ -143,33 +184,39 @@ __global__ void heat_step_kernel(const HeatArgs<real> a, int koff) {
     }
 }
 
-// FP32 step on four consecutive x cells per thread (nx % 4 == 0): theta, its
-// neighbour rows and the dose pairs move as 16-byte vectors; the source Q,
-// shifted by any whole number of cells, is read per cell.  Face cells keep
-// their value (they are written back unchanged), like the scalar kernel.
+// FP32 step on four consecutive x cells per thread (row pitch % 4 == 0): theta, its
+// neighbour rows and the doses move as 16-byte vectors; the source Q, shifted by
+// any whole number of cells, is read per cell.  Face cells keep their value
+// (they are written back unchanged), like the scalar kernel.  Every other step
+// marches the planes (and the chunks) from the high end, so that it starts on the
+// planes the step before it left in L2.  PAIR: the dose is a (hi, lo) float pair.
+template <bool PAIR>
 __global__ void __launch_bounds__(128) heat_step4_kernel(const HeatArgs<float> a, int koff) {
     const int x0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
     const int iy = blockIdx.y * blockDim.y + threadIdx.y;
     if (x0 >= a.nx || iy < 1 || iy >= a.ny - 1) return;
+    const int bz = a.rev ? gridDim.z - 1 - blockIdx.z : blockIdx.z;
+    const int z0 = max(1, bz * a.zb);
+    const int z1 = min(a.nz - 1, bz * a.zb + a.zb);
+    if (z0 >= z1) return;
     const long long step = *a.step_base + koff;
     const int2 sh = a.shifts[step];
     const int iya = iy - sh.y;                                   // T:61-62
     const bool qrow = iya >= 0 && iya < a.ny;
-    const long long col = (long long)iy * a.nx + x0;
-    const int z0 = max(1, blockIdx.z * a.zb);
-    const int z1 = min(a.nz - 1, blockIdx.z * a.zb + a.zb);
-    if (z0 >= z1) return;
-    const long long P = a.plane, NX = a.nx;
+    const long long col = (long long)iy * a.px + x0;
+    const long long P = a.plane, NX = a.px;
     auto ld4 = [](const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); };
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 tm = ld4(a.Tin + (long long)(z0 - 1) * P + col);
-    float4 tc = ld4(a.Tin + (long long)z0 * P + col);
+    const int zs = a.rev ? z1 - 1 : z0;                          // first plane of the march
+    const long long dz = a.rev ? -P : P;
+    float4 tm = ld4(a.Tin + (long long)zs * P - dz + col);       // the plane behind, this plane
+    float4 tc = ld4(a.Tin + (long long)zs * P + col);
     bool upd[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) upd[k] = x0 + k >= 1 && x0 + k < a.nx - 1;
-    for (int iz = z0; iz < z1; ++iz) {
+    for (int n = z1 - z0, iz = zs; n > 0; --n, iz += a.rev ? -1 : 1) {
         const long long i = (long long)iz * P + col;
-        const float4 tp = ld4(a.Tin + i + P);
+        const float4 tp = ld4(a.Tin + i + dz);
         const float4 L = x0 >= 4 ? ld4(a.Tin + i - 4) : zero;
         const float4 R = x0 + 4 < a.nx ? ld4(a.Tin + i + 4) : zero;
         const float4 yu = ld4(a.Tin + i + NX), yd = ld4(a.Tin + i - NX);
@@ -179,7 +226,7 @@ __global__ void __launch_bounds__(128) heat_step4_kernel(const HeatArgs<float> a
             const int ixa = x0 + k - sh.x;
             q[k] = (qrow && ixa >= 0 && ixa < a.nx) ? __ldg(a.Q + (long long)iz * P + (long long)iya * NX + ixa) : 0.f;
         }
-        double2* dp = reinterpret_cast<double2*>(a.TD + i);
+        double2* dp = PAIR ? reinterpret_cast<double2*>(a.TDf + i) : reinterpret_cast<double2*>(a.TD + i);
         double2 d01 = dp[0], d23 = dp[1];
         int mats[4];
         if (a.matmap) {
@@ -197,15 +244,19 @@ __global__ void __launch_bounds__(128) heat_step4_kernel(const HeatArgs<float> a
         float tn[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const HeatMat<float>& M = a.mat[mats[k]];
             const float sxy = xl[k] + xr[k] + su[k] + sd[k];
-            // T:85-87 (plus the Pennes term -w dt (T - T_art), zero in the reference)
-            const float t = cv[k] * M.a0 + M.kxy * sxy + M.kz * (zu[k] + zd[k]) + M.qc * q[k] + M.wTa;
+            const float t = heat_cell(a.mat[mats[k]], cv[k], sxy, zu[k] + zd[k], q[k]);
             tn[k] = upd[k] ? t : cv[k];
             if (upd[k]) {
-                const float x = t + a.T_refm43;                   // T_C - 43
-                const float inc = exp2f(x < 0.0f ? 2.0f * x : x) * a.dt;   // T:99-102
-                dose[k] = dose[k] + widen_pos(inc);
+                const float inc = __fmul_rn(dose_rate(t + a.T_refm43), a.dt);
+                if constexpr (PAIR) {
+                    float2 d;
+                    memcpy(&d, &dose[k], 8);
+                    d = df_add(d, inc);
+                    memcpy(&dose[k], &d, 8);
+                } else {
+                    dose[k] = dose_add(dose[k], inc);
+                }
             }
         }
         *reinterpret_cast<float4*>(a.Tout + i) = make_float4(tn[0], tn[1], tn[2], tn[3]);
@@ -214,6 +265,43 @@ __global__ void __launch_bounds__(128) heat_step4_kernel(const HeatArgs<float> a
         tm = tc;
         tc = tp;
     }
+}
+
+// Planes per CTA of the FP32 kernels.  A chunk costs its planes plus about 0.7 of
+// a plane's time to start; grids of several waves fill up as CTAs end and pay
+// half a chunk at the end.  Measured per step: 256 x 256 x 384 105.7 / 105.5 /
+// 117.2 us in chunks of 8 / 24 / 32 planes, 213 x 213 x 201 45.0 / 47.8 / 52.7 us
+// in 4 / 24 / 32, 96 x 96 x 78 5.5 / 10.1 / 30.5 us in 2 / 8 / 32, 72 x 72 x 60
+// 7.1 / 11.2 / 29.9 us (launch by launch) in 2 / 8 / 32.
+static int march_zb(bd_context* ctx, long long tiles, int nz, int per_sm) {
+    const double slots = (double)ctx->sm_count * std::max(per_sm, 1);
+    int best = 1;
+    double cost = 1e300;
+    for (int zb = 1; zb <= std::min(nz, 64); ++zb) {
+        const double waves = (double)(tiles * ((nz + zb - 1) / zb)) / slots;
+        const double c = (waves > 1.0 ? waves + 0.5 : 1.0) * (zb + 0.7);
+        if (c < cost) { cost = c; best = zb; }
+    }
+    return best;
+}
+static dim3 step4_grid(int px, int ny, int nz, int zb) {
+    return dim3((px / 4 + 15) / 16, (ny + 7) / 8, (nz + zb - 1) / zb);
+}
+static int step4_zb(bd_context* ctx, int px, int ny, int nz) {
+    static const int per_sm = [] {
+        int n = 0;
+        BD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_step4_kernel<false>, 128, 0));
+        return n;
+    }();
+    return march_zb(ctx, (long long)((px / 4 + 15) / 16) * ((ny + 7) / 8), nz, per_sm);
+}
+static int scalar_zb(bd_context* ctx, int nx, int ny, int nz) {
+    static const int per_sm = [] {
+        int n = 0;
+        BD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_step_kernel<float>, 256, 0));
+        return n;
+    }();
+    return march_zb(ctx, (long long)((nx + 31) / 32) * ((ny + 7) / 8), nz, per_sm);
 }
 
 // Initial fields and outputs are formed on the device: the callers' arrays are
@@ -227,34 +315,50 @@ struct HeatInit {
     double T_init[BD_MAX_MATERIALS], d_init[BD_MAX_MATERIALS];
 };
 
+// cell i of rows of nx cells, in rows of px cells
+__device__ __forceinline__ long long pitched(long long i, int nx, int px) {
+    const long long row = i / nx;
+    return row * px + (i - row * nx);
+}
+
 template <class real>
 __global__ void heat_init_T_kernel(real* __restrict__ Ta, real* __restrict__ Tb, const double* __restrict__ T_src,
                                    const HeatInit in, const int* __restrict__ plane_mat,
-                                   const uint8_t* __restrict__ matmap, long long plane, long long n, double T_ref) {
+                                   const uint8_t* __restrict__ matmap, int nx, int px, long long plane, long long n,
+                                   double T_ref) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int m = matmap ? matmap[i] : (plane_mat ? plane_mat[i / plane] : 0);
+    const long long j = pitched(i, nx, px);
+    const int m = matmap ? matmap[j] : (plane_mat ? plane_mat[j / plane] : 0);
     const double T = T_src ? T_src[i] : in.T_init[m];
     const real v = (real)(T - T_ref);
-    Ta[i] = v;
-    Tb[i] = v;
+    Ta[j] = v;
+    Tb[j] = v;
 }
 
-__global__ void heat_init_dose_kernel(double* __restrict__ TD, const HeatInit in, const int* __restrict__ plane_mat,
-                                      const uint8_t* __restrict__ matmap, long long plane, long long n) {
+__global__ void heat_init_dose_kernel(double* __restrict__ TD, const double* __restrict__ d_src, const HeatInit in,
+                                      const int* __restrict__ plane_mat, const uint8_t* __restrict__ matmap, int nx,
+                                      int px, long long plane, long long n) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    TD[i] = in.d_init[matmap ? matmap[i] : (plane_mat ? plane_mat[i / plane] : 0)];
+    const long long j = pitched(i, nx, px);
+    TD[j] = d_src ? d_src[i] : in.d_init[matmap ? matmap[j] : (plane_mat ? plane_mat[j / plane] : 0)];
 }
 
-__global__ void heat_narrow_kernel(float* __restrict__ dst, const double* __restrict__ src, long long n) {
+__global__ void heat_narrow_kernel(float* __restrict__ dst, const double* __restrict__ src, int nx, int px, long long n) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i < n) dst[i] = (float)src[i];
+    if (i < n) dst[pitched(i, nx, px)] = (float)src[i];
 }
 
-__global__ void heat_widen_kernel(double* __restrict__ dst, const float* __restrict__ src, long long n, double T_ref) {
+__global__ void heat_widen_kernel(double* __restrict__ dst, const float* __restrict__ src, int nx, int px, long long n,
+                                  double T_ref) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i < n) dst[i] = T_ref + (double)src[i];
+    if (i < n) dst[i] = T_ref + (double)src[pitched(i, nx, px)];
+}
+
+__global__ void heat_compact_kernel(double* __restrict__ dst, const double* __restrict__ src, int nx, int px, long long n) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i < n) dst[i] = src[pitched(i, nx, px)];
 }
 
 __global__ void heat_advance_kernel(long long* step_base, int n) {
@@ -333,7 +437,11 @@ struct HeatPlan {
     bd_context* ctx = nullptr;
     bool f64 = false, vec4 = false, use_graph = true, has_pm = false, has_mm = false;
     int nx = 0, ny = 0, nz = 0, n_legs = 0;
-    long long plane = 0, n = 0;
+    // device rows hold px cells: FP32 rows are padded to whole 16-byte vectors, so
+    // that odd row lengths take the four-cell kernel too (213 x 213 x 201: 45 us a
+    // step, 53 with the scalar kernel)
+    int px = 0;
+    long long plane = 0, hplane = 0, n = 0;        // px * ny, nx * ny, nx * ny * nz
     size_t esz = 4;
     double T_ref = 0.0, dt = 0.0;
     int64_t nsteps = 0;
@@ -369,8 +477,10 @@ struct HeatPlan {
             if (k > 0 && owned[k - 1].second != zb) fail(BD_ERR_INVALID_ARG, "local slabs must be contiguous");
         }
         f64 = th->precision == BD_F64;
-        plane = (long long)nx * ny;
-        n = plane * nz;
+        px = f64 ? nx : (nx + 3) / 4 * 4;
+        plane = (long long)px * ny;
+        hplane = (long long)nx * ny;
+        n = hplane * nz;
         dt = th->dt;
         use_graph = th->plain_launches == 0;
         // trajectory
@@ -406,7 +516,7 @@ struct HeatPlan {
             S.hi = S.ze < nz ? S.ze + 1 : nz;
             S.nzl = S.hi - S.lo;
             S.nl = plane * S.nzl;
-            most = std::max(most, S.nl);
+            most = std::max(most, hplane * S.nzl);
         }
         cudaStream_t q = ctx->stream;
         // whatever ends this block, the copies from the callers' arrays and from sh are done by then
@@ -425,8 +535,8 @@ struct HeatPlan {
             BD_CUDA(cudaMemcpyAsync(pm.p, th->plane_material, nz * 4, cudaMemcpyHostToDevice, q));
         }
         if (has_mm) {
-            mm.alloc(ctx, n);
-            BD_CUDA(cudaMemcpyAsync(mm.p, th->material_map, n, cudaMemcpyHostToDevice, q));
+            mm.alloc(ctx, plane * nz);
+            BD_CUDA(cudaMemcpy2DAsync(mm.p, px, th->material_map, nx, nx, (size_t)ny * nz, cudaMemcpyHostToDevice, q));
         }
         BD_CUDA(cudaMemsetAsync(sb.p, 0, 64, q));
         // initial fields (T:232-257)
@@ -439,54 +549,52 @@ struct HeatPlan {
         for (HeatSlab& S : sl) {
             S.Ta.alloc(ctx, S.nl * esz); S.Tb.alloc(ctx, S.nl * esz); S.Qd.alloc(ctx, S.nl * esz);
             S.TDd.alloc(ctx, S.nl * 8);
-            const long long o = plane * S.lo;
+            const long long o = hplane * S.lo, cells = hplane * S.nzl;
             const int* spm = has_pm ? pm.as<int>() + S.lo : nullptr;
-            const uint8_t* smm = has_mm ? mm.as<uint8_t>() + o : nullptr;
-            const unsigned blocks = (unsigned)((S.nl + 255) / 256);
-            const double* T_src = nullptr;
+            const uint8_t* smm = has_mm ? mm.as<uint8_t>() + plane * S.lo : nullptr;
+            const unsigned blocks = (unsigned)((cells + 255) / 256);
+            // FP64 rows are not padded: its arrays are copied straight in, the FP32 ones through the staging buffer
+            const double* src = nullptr;
             if (th->T_start) {
                 void* to = f64 ? S.Tb.p : stage.p;
-                BD_CUDA(cudaMemcpyAsync(to, th->T_start + o, S.nl * 8, cudaMemcpyHostToDevice, q));
-                T_src = static_cast<const double*>(to);
+                BD_CUDA(cudaMemcpyAsync(to, th->T_start + o, cells * 8, cudaMemcpyHostToDevice, q));
+                src = static_cast<const double*>(to);
             }
-            if (f64 && T_src) {
-                BD_CUDA(cudaMemcpyAsync(S.Ta.p, S.Tb.p, S.nl * 8, cudaMemcpyDeviceToDevice, q));
+            if (f64 && src) {
+                BD_CUDA(cudaMemcpyAsync(S.Ta.p, S.Tb.p, cells * 8, cudaMemcpyDeviceToDevice, q));
             } else if (f64) {
                 heat_init_T_kernel<double><<<blocks, 256, 0, q>>>(S.Ta.as<double>(), S.Tb.as<double>(), nullptr, in, spm,
-                                                                  smm, plane, S.nl, 0.0);
+                                                                  smm, nx, px, plane, cells, 0.0);
                 BD_LAUNCHED(ctx);
             } else {
-                heat_init_T_kernel<float><<<blocks, 256, 0, q>>>(S.Ta.as<float>(), S.Tb.as<float>(), T_src, in, spm, smm,
-                                                                 plane, S.nl, T_ref);
+                heat_init_T_kernel<float><<<blocks, 256, 0, q>>>(S.Ta.as<float>(), S.Tb.as<float>(), src, in, spm, smm,
+                                                                 nx, px, plane, cells, T_ref);
                 BD_LAUNCHED(ctx);
             }
             if (f64) {
-                BD_CUDA(cudaMemcpyAsync(S.Qd.p, Q + o, S.nl * 8, cudaMemcpyHostToDevice, q));
+                BD_CUDA(cudaMemcpyAsync(S.Qd.p, Q + o, cells * 8, cudaMemcpyHostToDevice, q));
             } else {
-                BD_CUDA(cudaMemcpyAsync(stage.p, Q + o, S.nl * 8, cudaMemcpyHostToDevice, q));
-                heat_narrow_kernel<<<blocks, 256, 0, q>>>(S.Qd.as<float>(), stage.as<double>(), S.nl);
+                BD_CUDA(cudaMemcpyAsync(stage.p, Q + o, cells * 8, cudaMemcpyHostToDevice, q));
+                heat_narrow_kernel<<<blocks, 256, 0, q>>>(S.Qd.as<float>(), stage.as<double>(), nx, px, cells);
                 BD_LAUNCHED(ctx);
             }
+            src = nullptr;
             if (th->dose_start) {
-                BD_CUDA(cudaMemcpyAsync(S.TDd.p, th->dose_start + o, S.nl * 8, cudaMemcpyHostToDevice, q));
-            } else {
-                heat_init_dose_kernel<<<blocks, 256, 0, q>>>(S.TDd.as<double>(), in, spm, smm, plane, S.nl);
+                void* to = f64 ? S.TDd.p : stage.p;
+                BD_CUDA(cudaMemcpyAsync(to, th->dose_start + o, cells * 8, cudaMemcpyHostToDevice, q));
+                src = static_cast<const double*>(to);
+            }
+            if (!(f64 && src)) {
+                heat_init_dose_kernel<<<blocks, 256, 0, q>>>(S.TDd.as<double>(), src, in, spm, smm, nx, px, plane, cells);
                 BD_LAUNCHED(ctx);
             }
         }
         BD_CUDA(cudaStreamSynchronize(q));
-        vec4 = !f64 && nx % 4 == 0;
-        static int per_sm4 = 0;
-        if (vec4 && !per_sm4) BD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm4, heat_step4_kernel, 128, 0));
+        vec4 = !f64;
         for (HeatSlab& S : sl) {
-            S.zbk = 32;
-            if (vec4) {
-                // four-cell kernel: z-chunk fitted to whole waves of its resident CTAs
-                const long long tiles = (long long)((nx / 4 + 15) / 16) * ((ny + 7) / 8);
-                S.zbk = wave_fitted_zb(tiles, S.nzl, (long long)ctx->sm_count * std::max(per_sm4, 1), 0.9);
-            }
+            S.zbk = vec4 ? step4_zb(ctx, px, ny, S.nzl) : 32;
             S.grid = dim3((nx + 31) / 32, (ny + 7) / 8, (S.nzl + S.zbk - 1) / S.zbk);
-            S.grid4 = dim3((nx / 4 + 15) / 16, (ny + 7) / 8, (S.nzl + S.zbk - 1) / S.zbk);
+            S.grid4 = step4_grid(px, ny, S.nzl, S.zbk);
         }
         // material constants (T:212-217, plus the Pennes term)
         std::memset(&af, 0, sizeof af);
@@ -507,7 +615,7 @@ struct HeatPlan {
 
     template <class A, class RR>
     void fill(A& a, const HeatSlab& S, bool a_to_b) const {
-        a.nx = nx; a.ny = ny; a.nz = S.nzl; a.zb = S.zbk; a.plane = plane;
+        a.nx = nx; a.ny = ny; a.nz = S.nzl; a.zb = S.zbk; a.px = px; a.rev = a_to_b ? 0 : 1; a.plane = plane;
         a.Tin = (a_to_b ? S.Ta : S.Tb).template as<RR>();
         a.Tout = (a_to_b ? S.Tb : S.Ta).template as<RR>();
         a.Q = S.Qd.template as<RR>();
@@ -545,7 +653,7 @@ struct HeatPlan {
     // steps s0 .. s0 + cnt - 1 of every local slab: the kernels read their step as
     // the device counter plus their offset, and one advance kernel moves the counter
     void issue(cudaStream_t st, int64_t s0, int cnt) {
-        const dim3 block(32, 8), block4(16, 8);
+        const dim3 block(32, 8);
         for (int k = 0; k < cnt; ++k) {
             const bool a_to_b = ((s0 + k) % 2) == 0;
             for (const HeatSlab& S : sl) {
@@ -556,8 +664,7 @@ struct HeatPlan {
                 } else {
                     HeatArgs<float> a = af;
                     fill<HeatArgs<float>, float>(a, S, a_to_b);
-                    if (vec4) heat_step4_kernel<<<S.grid4, block4, 0, st>>>(a, k);
-                    else heat_step_kernel<float><<<S.grid, block, 0, st>>>(a, k);
+                    heat_step4_kernel<false><<<S.grid4, dim3(16, 8), 0, st>>>(a, k);
                 }
                 BD_LAUNCHED(ctx);
             }
@@ -611,15 +718,15 @@ struct HeatPlan {
         cudaStream_t s = ctx->stream;
         for (const HeatSlab& S : sl) {
             const PoolBuf& src = newest(S, steps);
-            const long long off = plane * (S.zb - S.lo), cnt = plane * (S.ze - S.zb);
+            const long long off = plane * (S.zb - S.lo), cnt = hplane * (S.ze - S.zb);
             const double* from = static_cast<const double*>(src.p) + off;
             if (!f64) {
                 heat_widen_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, s>>>(
-                    stage.as<double>(), static_cast<const float*>(src.p) + off, cnt, T_ref);
+                    stage.as<double>(), static_cast<const float*>(src.p) + off, nx, px, cnt, T_ref);
                 BD_LAUNCHED(ctx);
                 from = stage.as<double>();
             }
-            double* d = dst + plane * S.zb;
+            double* d = dst + hplane * S.zb;
             host_populate(d, cnt * 8);   // while the steps before this copy run
             BD_CUDA(cudaMemcpyAsync(d, from, cnt * 8, cudaMemcpyDeviceToHost, s));
         }
@@ -627,14 +734,20 @@ struct HeatPlan {
     }
 
     void copy_dose(double* dst) {
+        cudaStream_t s = ctx->stream;
         for (const HeatSlab& S : sl) {
-            double* d = dst + plane * S.zb;
-            const size_t bytes = (size_t)plane * (S.ze - S.zb) * 8;
-            host_populate(d, bytes);
-            BD_CUDA(cudaMemcpyAsync(d, static_cast<const double*>(S.TDd.p) + plane * (S.zb - S.lo), bytes,
-                                    cudaMemcpyDeviceToHost, ctx->stream));
+            const long long off = plane * (S.zb - S.lo), cnt = hplane * (S.ze - S.zb);
+            const double* from = S.TDd.as<double>() + off;
+            if (px != nx) {
+                heat_compact_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, s>>>(stage.as<double>(), from, nx, px, cnt);
+                BD_LAUNCHED(ctx);
+                from = stage.as<double>();
+            }
+            double* d = dst + hplane * S.zb;
+            host_populate(d, cnt * 8);
+            BD_CUDA(cudaMemcpyAsync(d, from, cnt * 8, cudaMemcpyDeviceToHost, s));
         }
-        BD_CUDA(cudaStreamSynchronize(ctx->stream));
+        BD_CUDA(cudaStreamSynchronize(s));
     }
 };
 
@@ -801,7 +914,7 @@ bd_status bd_heat_slab_advance(bd_heat_slab* h, int64_t n) {
 bd_status bd_heat_slab_halo_bytes(bd_heat_slab* h, size_t* bytes) {
     return guard([&] {
         if (!h || !bytes) fail(BD_ERR_INVALID_ARG, "null argument");
-        *bytes = (size_t)h->P.plane * h->P.esz;
+        *bytes = (size_t)h->P.hplane * h->P.esz;
     });
 }
 
@@ -818,8 +931,9 @@ bd_status bd_heat_slab_halo_copy(bd_heat_slab* h, int32_t side, int32_t to_ghost
         const int local = side == 0 ? (to_ghost ? 0 : 1) : (to_ghost ? S.nzl - 1 : S.nzl - 2);
         char* plane = static_cast<char*>(h->P.newest(S, h->P.step).p) + (size_t)local * pb;
         cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : h->P.ctx->stream;
-        if (to_ghost) BD_CUDA(cudaMemcpyAsync(plane, d_buf, pb, cudaMemcpyDeviceToDevice, st));
-        else BD_CUDA(cudaMemcpyAsync(d_buf, plane, pb, cudaMemcpyDeviceToDevice, st));
+        const size_t row = (size_t)h->P.nx * h->P.esz, pitch = (size_t)h->P.px * h->P.esz;   // messages are not padded
+        if (to_ghost) BD_CUDA(cudaMemcpy2DAsync(plane, pitch, d_buf, row, row, h->P.ny, cudaMemcpyDeviceToDevice, st));
+        else BD_CUDA(cudaMemcpy2DAsync(d_buf, row, plane, pitch, row, h->P.ny, cudaMemcpyDeviceToDevice, st));
     });
 }
 
@@ -873,7 +987,7 @@ bd_status bd_heat_run_device_noalloc(bd_context* ctx, const bd_thermal* th, floa
         HeatArgs<float> a;
         std::memset(&a, 0, sizeof a);
         heat_materials<float>(th, th->T_ref, a.mat);
-        a.nx = nx; a.ny = ny; a.nz = nz; a.zb = 32; a.plane = (long long)nx * ny;
+        a.nx = nx; a.ny = ny; a.nz = nz; a.px = nx; a.plane = (long long)nx * ny;
         a.Q = d_Q;
         a.TD = nullptr;
         a.TDf = reinterpret_cast<float2*>(d_dose);
@@ -884,18 +998,18 @@ bd_status bd_heat_run_device_noalloc(bd_context* ctx, const bd_thermal* th, floa
         a.dt = (float)th->dt;
         a.T_ref = th->T_ref;
         a.T_refm43 = (float)(th->T_ref - 273.15 - 43.0);
-        dim3 block(32, 8), grid((nx + 31) / 32, (ny + 7) / 8, (nz + a.zb - 1) / a.zb);
-        const int CH = 64;
-        for (int64_t s0 = 0; s0 < n_steps; s0 += CH) {
-            const int cnt = (int)std::min<int64_t>(CH, n_steps - s0);
-            for (int k = 0; k < cnt; ++k) {
-                const bool even = ((s0 + k) % 2) == 0;   // even steps read the caller's field
-                a.Tin = even ? d_theta : sc.theta;
-                a.Tout = even ? sc.theta : d_theta;
-                heat_step_kernel<float><<<grid, block, 0, s>>>(a, k);
-                BD_LAUNCHED(ctx);
-            }
-            heat_advance_kernel<<<1, 32, 0, s>>>(sc.step, cnt);
+        // the caller's rows are not padded: whole-vector rows and 16-byte aligned buffers take the four-cell kernel
+        const bool vec = nx % 4 == 0 && (reinterpret_cast<uintptr_t>(d_theta) | reinterpret_cast<uintptr_t>(d_dose)) % 16 == 0;
+        a.zb = vec ? step4_zb(ctx, nx, ny, nz) : scalar_zb(ctx, nx, ny, nz);
+        const dim3 block(32, 8), grid((nx + 31) / 32, (ny + 7) / 8, (nz + a.zb - 1) / a.zb);
+        const dim3 grid4 = step4_grid(nx, ny, nz, a.zb);
+        for (int64_t k = 0; k < n_steps; ++k) {
+            const bool even = k % 2 == 0;                    // even steps read the caller's field
+            a.rev = even ? 0 : 1;
+            a.Tin = even ? d_theta : sc.theta;
+            a.Tout = even ? sc.theta : d_theta;
+            if (vec) heat_step4_kernel<true><<<grid4, dim3(16, 8), 0, s>>>(a, (int)k);
+            else heat_step_kernel<float><<<grid, block, 0, s>>>(a, (int)k);
             BD_LAUNCHED(ctx);
         }
         if (n_steps % 2 == 1)   // the latest field is in the partner buffer
