@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
@@ -134,12 +135,16 @@ void host_populate(void* p, size_t bytes);
 // resident CTAs (at least `fill` of the last wave busy), the largest such
 // chunk of at least 8 planes with the chunk count rounded up to cover w waves;
 // failing that, the chunk count rounded down (just under w waves); 16 if
-// neither qualifies.  down_first tries the rounded-down counts first (fewer,
-// longer chunks, for kernels with a long per-chunk prologue).
-inline int wave_fitted_zb(long long tiles, int nz, long long slots, double fill = 0.97, bool down_first = false) {
+// neither qualifies.  Grids that chunks of 8 planes do not fill one wave of take
+// the shortest chunks (2 planes or more) that still fit one.
+inline int wave_fitted_zb(long long tiles, int nz, long long slots, double fill = 0.97) {
+    if (tiles * ((nz + 7) / 8) <= slots) {
+        const long long chunks = slots / tiles;               // per tile
+        return (int)std::max<long long>(2, (nz + chunks - 1) / chunks);
+    }
     for (int pass = 0; pass < 2; ++pass)
         for (int w = 1; w <= 16; ++w) {
-            const bool down = (pass == 0) == down_first;
+            const bool down = pass == 1;
             const long long chunks = down ? (w * slots) / tiles : (w * slots + tiles - 1) / tiles;
             if (chunks > nz) break;
             if (chunks < 1) continue;

@@ -38,7 +38,8 @@ namespace bd {
 // Kernel variants: 0-7 plain (read-only-cache neighbours), 8-23 TMA-pipelined
 // (need a row pitch that is a multiple of 16 bytes).  19-23 take two adjacent
 // x cells per thread (wv_tma_pair_kernel, pointwise ring of nq slots) and are
-// built for FP32 fields with at most two relaxation processes.
+// built for FP32 fields with at most two relaxation processes.  24-28 are 19-23
+// on device rows padded to a 16-byte pitch: they serve any row length.
 struct Variant { int tx, ty, zb, tma, cpt, zu, pair, nq; };
 static const Variant kVariants[] = {
     {32, 8, 32, 0, 1, 1, 0, 3}, {32, 4, 32, 0, 1, 1, 0, 3}, {64, 4, 32, 0, 1, 1, 0, 3}, {32, 8, 64, 0, 1, 1, 0, 3},
@@ -50,8 +51,11 @@ static const Variant kVariants[] = {
     // two x cells per thread, two-slot pointwise ring
     {32, 8, -1, 1, 1, 1, 1, 2}, {32, 8, -1, 1, 1, 2, 1, 2}, {64, 8, -1, 1, 1, 1, 1, 2},
     {64, 8, -1, 1, 1, 2, 1, 2}, {32, 16, -1, 1, 1, 1, 1, 2},
+    {32, 8, -1, 1, 1, 1, 1, 2}, {32, 8, -1, 1, 1, 2, 1, 2}, {64, 8, -1, 1, 1, 1, 1, 2},
+    {64, 8, -1, 1, 1, 2, 1, 2}, {32, 16, -1, 1, 1, 1, 1, 2},
 };
 static const int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
+static const int kFirstPadded = 24, kPadOffset = 5;   // variant v + kPadOffset is v on padded rows
 
 // tuned variant per problem signature (process-wide)
 static std::mutex g_tune_mu;
@@ -65,7 +69,13 @@ struct WvSession {
     int prec = BD_F32;
     size_t esz = 4;
     int nx = 0, ny = 0, nz = 0;
-    long long plane = 0, ncell = 0;
+    // device fields have rows of px cells: nx, or nx rounded up to a 16-byte pitch
+    // (the cells in between are never read by a cell of the grid); every host array,
+    // message and checkpoint has rows of nx cells
+    int px = 0;
+    long long plane = 0, ncell = 0;          // px * ny and px * ny * nz
+    long long hplane = 0;                    // nx * ny
+    PoolBuf stage;                           // rows of nx cells between a host array and a padded field
     int max_relax = 0;
     int n_dft = 0, dz_lo = 0, dz_hi = 0;
     long long dcells = 0;
@@ -128,6 +138,7 @@ static WvArgs<real> make_args(WvSession& S, int64_t s) {
     WvArgs<real> a;
     std::memset(&a, 0, sizeof a);
     a.nx = S.nx; a.ny = S.ny; a.nz = S.nz;
+    a.px = S.px;
     a.plane = S.plane;
     const int h = head_of(s);
     a.p0 = S.P[(h + 0) % 5].as<real>();
@@ -215,7 +226,7 @@ static CUtensorMap make_map(const WvSession& S, const void* base, bool is_float,
     CUtensorMap m;
     const size_t esz = is_u8 ? 1 : is_float ? 4 : 8;
     cuuint64_t dims[3] = {(cuuint64_t)S.nx, (cuuint64_t)S.ny, (cuuint64_t)(depth > 0 ? depth : S.nz)};
-    cuuint64_t strides[2] = {(cuuint64_t)S.nx * esz, (cuuint64_t)S.nx * S.ny * esz};
+    cuuint64_t strides[2] = {(cuuint64_t)S.px * esz, (cuuint64_t)S.px * S.ny * esz};
     cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, 1};
     cuuint32_t estr[3] = {1, 1, 1};
     const CUtensorMapDataType ty = is_u8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
@@ -229,12 +240,15 @@ static CUtensorMap make_map(const WvSession& S, const void* base, bool is_float,
 }
 
 static bool tma_eligible(const WvSession& S) {
-    return (S.nx * S.esz) % 16 == 0 && S.nx >= 8;
+    return (S.px * S.esz) % 16 == 0 && S.nx >= 8;
 }
 
 // The two-cell variants are compiled for FP32 fields with at most two
-// relaxation processes; a 16-byte row pitch makes nx even.
+// relaxation processes; a 16-byte row pitch makes px even.  Grids whose rows
+// are padded take the padded variants (and the plain kernels), the others the
+// rest.
 static bool variant_ok(const WvSession& S, int v) {
+    if ((v >= kFirstPadded) != (S.px != S.nx) && kVariants[v].tma) return false;
     if (!kVariants[v].pair) return true;
     return S.prec == BD_F32 && S.max_relax <= 2 && tma_eligible(S);
 }
@@ -560,7 +574,7 @@ static void zero_state(WvSession& S) {
 
 static std::string tune_key(const WvSession& S) {
     char b[256];
-    snprintf(b, sizeof b, "%d:%d:%d:%d:%d:%d:%d:%d:%d:%d", S.nx, S.ny, S.nz, S.prec, S.max_relax, S.has_cmap ? 1 : 0,
+    snprintf(b, sizeof b, "%d:%d:%d:%d:%d:%d:%d:%d:%d:%d:%d", S.nx, S.px, S.ny, S.nz, S.prec, S.max_relax, S.has_cmap ? 1 : 0,
              S.has_matmap ? 1 : 0, S.has_planemat ? 1 : 0, S.any_mur ? 1 : 0, S.n_dft);
     return b;
 }
@@ -639,10 +653,89 @@ static void upload(WvSession& S, PoolBuf& b, const std::vector<T>& v) {
     if (!v.empty()) BD_CUDA(cudaMemcpy(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
 }
 
+// Rows of nx cells to or from rows of px cells.
+template <class T>
+__global__ void wv_repitch_kernel(T* __restrict__ dst, const T* __restrict__ src, int nx, int px, long long n,
+                                  int to_padded) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const long long row = i / nx, j = row * px + (i - row * nx);
+    if (to_padded) dst[j] = src[i];
+    else dst[i] = src[j];
+}
+
+// rows = number of nx-cell rows moved between a host array and a field
+template <class T>
+static void field_in(WvSession& S, void* dev, const void* host, long long rows) {
+    const size_t bytes = (size_t)rows * S.nx * sizeof(T);
+    if (S.px == S.nx) {
+        BD_CUDA(cudaMemcpy(dev, host, bytes, cudaMemcpyHostToDevice));
+        return;
+    }
+    cudaStream_t st = S.ctx->stream;
+    if (S.stage.bytes < bytes) S.stage.alloc(S.ctx, bytes);
+    BD_CUDA(cudaMemcpyAsync(S.stage.p, host, bytes, cudaMemcpyHostToDevice, st));
+    const long long n = rows * S.nx;
+    wv_repitch_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(static_cast<T*>(dev), S.stage.as<T>(), S.nx, S.px, n, 1);
+    BD_LAUNCHED(S.ctx);
+    BD_CUDA(cudaStreamSynchronize(st));      // the host array has been read
+}
+
+template <class T>
+static void field_out(WvSession& S, void* host, const void* dev, long long rows) {
+    const size_t bytes = (size_t)rows * S.nx * sizeof(T);
+    if (S.px == S.nx) {
+        BD_CUDA(cudaMemcpy(host, dev, bytes, cudaMemcpyDeviceToHost));
+        return;
+    }
+    cudaStream_t st = S.ctx->stream;
+    if (S.stage.bytes < bytes) S.stage.alloc(S.ctx, bytes);
+    const long long n = rows * S.nx;
+    wv_repitch_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(S.stage.as<T>(), static_cast<const T*>(dev), S.nx, S.px, n, 0);
+    BD_LAUNCHED(S.ctx);
+    BD_CUDA(cudaMemcpyAsync(host, S.stage.p, bytes, cudaMemcpyDeviceToHost, st));
+    BD_CUDA(cudaStreamSynchronize(st));
+}
+
+static void real_in(WvSession& S, void* dev, const void* host, long long rows) {
+    if (S.prec == BD_F32) field_in<float>(S, dev, host, rows);
+    else field_in<double>(S, dev, host, rows);
+}
+static void real_out(WvSession& S, void* host, const void* dev, long long rows) {
+    if (S.prec == BD_F32) field_out<float>(S, host, dev, rows);
+    else field_out<double>(S, host, dev, rows);
+}
+
 static double frac(double x) { return x - std::floor(x); }
 
+// Variant of a run that is not tuned: FP32 grids of at most two relaxation
+// processes take the two-cell kernel, in the tile whose chunks (the fewest planes
+// that still fit one wave, pair_zb) should end first: a chunk costs its planes
+// plus about six planes' time to fill the pipeline, and a plane more the more
+// warps share an SM.  48 x 48 x 80, 80 x 80 x 96 and 112 x 112 x 128 (one
+// relaxation process, c map): 6.4, 11.0 and 18.4 us a step; the one-cell kernel in
+// 16-plane chunks took 17.6, 19.1 and 25.8.
+static int untuned_variant(const WvSession& S) {
+    if (!tma_eligible(S)) return 0;
+    if (S.prec != BD_F32 || S.max_relax > 2) return 17;
+    int best = 23;
+    double cost = 1e300;
+    for (int v : {23, 21, 19}) {
+        const Variant& V = kVariants[v];
+        const double warps = V.tx * V.ty / 64.0;                      // of a CTA; 24 are resident on an SM
+        const long long tiles = (long long)((S.nx + V.tx - 1) / V.tx) * ((S.ny + V.ty - 1) / V.ty);
+        const int zb = wave_fitted_zb(tiles, S.nz, (long long)(S.ctx->sm_count * 24 / warps));
+        const double busy = std::min(3.0, (double)(tiles * ((S.nz + zb - 1) / zb)) * warps / 8.0 / S.ctx->sm_count);
+        const double waves = std::max(1.0, (double)(tiles * ((S.nz + zb - 1) / zb)) * warps / 24.0 / S.ctx->sm_count);
+        const double c = waves * (zb + 6) * (0.5 + 0.27 * busy);
+        if (c < 0.95 * cost) { cost = c; best = v; }
+    }
+    return S.px != S.nx ? best + kPadOffset : best;
+}
+
+// pad_rows: the caller takes fields with padded rows (px != nx)
 static void setup(WvSession& S, bd_context* ctx, const bd_grid* g, const bd_medium* m, const bd_source* src,
-                  const bd_westervelt_params* p) {
+                  const bd_westervelt_params* p, bool pad_rows = false) {
     if (!ctx || !g || !m || !p) fail(BD_ERR_INVALID_ARG, "null argument");
     S.ctx = ctx;
     S.g = *g;
@@ -671,8 +764,6 @@ static void setup(WvSession& S, bd_context* ctx, const bd_grid* g, const bd_medi
     for (int f = 0; f < 6; ++f) if (g->face[f] == BD_FACE_MUR) S.any_mur = true;
     if (S.any_mur && (g->mur_layers < 1 || g->mur_layers > 8)) fail(BD_ERR_INVALID_ARG, "mur_layers must be 1..8");
     if (m->n_materials < 1 || m->n_materials > BD_MAX_MATERIALS) fail(BD_ERR_INVALID_ARG, "n_materials out of range");
-    S.plane = (long long)S.nx * S.ny;
-    S.ncell = S.plane * S.nz;
     S.max_relax = 0;
     for (int k = 0; k < m->n_materials; ++k) {
         if (m->mat[k].n_relax < 0 || m->mat[k].n_relax > BD_MAX_RELAX) fail(BD_ERR_INVALID_ARG, "n_relax out of range");
@@ -680,6 +771,19 @@ static void setup(WvSession& S, bd_context* ctx, const bd_grid* g, const bd_medi
         if (!(m->mat[k].rho > 0)) fail(BD_ERR_INVALID_ARG, "material %d density must be positive", k);
         S.max_relax = std::max(S.max_relax, m->mat[k].n_relax);
     }
+    // FP32 rows that are no multiple of 16 bytes are padded to one (of 16 cells where
+    // a material map travels with them), so that they take the two-cell TMA kernel
+    // instead of the plain one (reference physics on 107 x 107 x 401 cells, 700
+    // steps: the solve took 504 ms, 149 ms with this and the one-pass Mur faces)
+    S.px = S.nx;
+    if (pad_rows && !S.slab && S.prec == BD_F32 && S.nx % 4 != 0 && S.max_relax <= 2 &&
+        (p->tile_variant < 0 || p->tile_variant >= kFirstPadded)) {
+        const int px = m->material_map ? (S.nx + 15) / 16 * 16 : (S.nx + 3) / 4 * 4;
+        if ((long long)px * S.ny < (1LL << 31)) S.px = px;
+    }
+    S.plane = (long long)S.px * S.ny;
+    S.hplane = (long long)S.nx * S.ny;
+    S.ncell = S.plane * S.nz;
     if (S.s.kind != BD_SRC_NONE) {
         if (S.s.plane_iz < 0 || S.s.plane_iz >= S.nz) fail(BD_ERR_INVALID_ARG, "source plane outside the grid");
         if (S.s.n_tones < 1 || S.s.n_tones > BD_MAX_TONES) fail(BD_ERR_INVALID_ARG, "n_tones out of range");
@@ -698,7 +802,7 @@ static void setup(WvSession& S, bd_context* ctx, const bd_grid* g, const bd_medi
         if (S.dz_hi <= S.dz_lo || p->dft_len <= 0) S.n_dft = 0;
     }
     S.dcells = S.n_dft > 0 ? (long long)(S.dz_hi - S.dz_lo) * S.plane : 0;
-    if (!S.slab) { S.dft_glob_cells = S.dcells; S.dft_glob_off = 0; }
+    if (!S.slab) { S.dft_glob_cells = S.n_dft > 0 ? (S.dz_hi - S.dz_lo) * S.hplane : 0; S.dft_glob_off = 0; }
     if (S.slab) S.pdl = false;   // the halo copies between steps are not kernels: plain stream order
     S.chunk = p->graph_chunk > 0 ? ((p->graph_chunk + 9) / 10) * 10 : 50;
 
@@ -721,16 +825,18 @@ static void setup(WvSession& S, bd_context* ctx, const bd_grid* g, const bd_medi
     S.has_planemat = m->plane_material != nullptr;
     // the paired kernel takes the material map as a uint8 TMA tile when its rows
     // (nx bytes) are a multiple of 16 bytes, else per cell through the cache
-    S.mat_tile = S.has_matmap && S.nx % 16 == 0;
+    S.mat_tile = S.has_matmap && S.px % 16 == 0;
     if (S.has_cmap) {
         S.cmap.alloc(ctx, S.ncell * 4);
-        BD_CUDA(cudaMemcpy(S.cmap.p, m->c_map, S.ncell * 4, cudaMemcpyHostToDevice));
+        field_in<float>(S, S.cmap.p, m->c_map, (long long)S.ny * S.nz);
     }
     if (S.has_matmap) {
-        for (long long i = 0; i < S.ncell; ++i)
-            if (m->material_map[i] >= m->n_materials) fail(BD_ERR_INVALID_ARG, "material_map entry out of range");
+        uint8_t top = 0;
+        for (long long i = 0; i < S.hplane * S.nz; ++i) top = std::max(top, m->material_map[i]);
+        if (top >= m->n_materials) fail(BD_ERR_INVALID_ARG, "material_map entry out of range");
         S.matmap.alloc(ctx, S.ncell);
-        BD_CUDA(cudaMemcpy(S.matmap.p, m->material_map, S.ncell, cudaMemcpyHostToDevice));
+        if (S.px != S.nx) BD_CUDA(cudaMemsetAsync(S.matmap.p, 0, S.ncell, ctx->stream));
+        field_in<uint8_t>(S, S.matmap.p, m->material_map, (long long)S.ny * S.nz);
     }
     if (S.has_planemat) {
         for (int iz = 0; iz < S.nz; ++iz)
@@ -780,7 +886,7 @@ static void setup(WvSession& S, bd_context* ctx, const bd_grid* g, const bd_medi
         const double d = S.s.focal_length;
         for (int iy = 0; iy < S.ny; ++iy)
             for (int ix = 0; ix < S.nx; ++ix) {
-                const long long j = (long long)iy * S.nx + ix;
+                const long long j = (long long)iy * S.px + ix;
                 const double X = g->x0 + ix * g->dx - S.s.cx;
                 const double Y = g->y0 + iy * g->dx - S.s.cy;
                 const double r = std::sqrt(X * X + Y * Y);
@@ -788,7 +894,7 @@ static void setup(WvSession& S, bd_context* ctx, const bd_grid* g, const bd_medi
                     const double vr = std::sqrt(1.0 + std::pow(r / d, 2));
                     double amp = S.s.p0, ph = 0.0;
                     if (S.s.kind == BD_SRC_ARRAY) {
-                        const int e = S.s.element_of_cell[j];
+                        const int e = S.s.element_of_cell[(long long)iy * S.nx + ix];
                         if (e < 0 || e >= S.s.n_elements) continue;
                         amp *= S.s.element_amp ? S.s.element_amp[e] : 1.0;
                         ph = S.s.element_phase ? S.s.element_phase[e] : 0.0;
@@ -849,12 +955,11 @@ static void setup(WvSession& S, bd_context* ctx, const bd_grid* g, const bd_medi
     if (p->tile_variant >= 0) {
         if (p->tile_variant >= kNumVariants) fail(BD_ERR_INVALID_ARG, "tile_variant out of range");
         S.variant = p->tile_variant;
-    } else if (S.ncell >= (1LL << 21) && p->n_steps >= 200) {
+        if (S.variant >= kFirstPadded && S.px == S.nx) S.variant -= kPadOffset;   // nothing to pad
+    } else if (S.hplane * S.nz >= (1LL << 21) && p->n_steps >= 200) {
         autotune(S);
     } else {
-        // short or small runs are not worth tuning: the wave-fitted TMA variant
-        // where the row pitch allows it, else the plain kernel
-        S.variant = tma_eligible(S) ? 17 : 0;
+        S.variant = untuned_variant(S);   // short or small runs are not worth tuning
     }
 }
 
@@ -991,12 +1096,13 @@ __global__ void wv_q_kernel(const real* __restrict__ energy, const real* __restr
 
 // Pages of the output buffers that finish() writes (host_populate).
 static void populate_outputs(const WvSession& S, const bd_westervelt_outputs* o) {
-    const size_t bytes = (size_t)(S.own1 - S.own0) * S.plane * S.esz;
+    const size_t bytes = (size_t)(S.own1 - S.own0) * S.hplane * S.esz;
     host_populate(o->p_final, bytes);
     host_populate(o->peak, bytes);
     host_populate(o->energy, bytes);
     for (int j = 0; j < S.n_dft; ++j) {
-        const size_t at = ((size_t)j * S.dft_glob_cells + S.dft_glob_off) * S.esz, nb = (size_t)S.dcells * S.esz;
+        const size_t at = ((size_t)j * S.dft_glob_cells + S.dft_glob_off) * S.esz;
+        const size_t nb = (size_t)(S.dz_hi - S.dz_lo) * S.hplane * S.esz;
         if (o->dft_re) host_populate(static_cast<char*>(o->dft_re) + at, nb);
         if (o->dft_im) host_populate(static_cast<char*>(o->dft_im) + at, nb);
     }
@@ -1009,19 +1115,17 @@ static void finish(WvSession& S, bd_westervelt_outputs* o) {
     BD_CUDA(cudaStreamSynchronize(st));
     // owned planes only (a whole grid owns every plane)
     const size_t off = (size_t)S.own0 * S.plane * S.esz;
-    const size_t bytes = (size_t)(S.own1 - S.own0) * S.plane * S.esz;
+    const long long rows = (long long)(S.own1 - S.own0) * S.ny;
     const int h = head_of(S.step);
     auto at = [&](const PoolBuf& b) { return static_cast<const char*>(b.p) + off; };
-    if (o->p_final) BD_CUDA(cudaMemcpy(o->p_final, at(S.P[h]), bytes, cudaMemcpyDeviceToHost));
-    if (o->peak) BD_CUDA(cudaMemcpy(o->peak, at(S.peak), bytes, cudaMemcpyDeviceToHost));
-    if (o->energy) BD_CUDA(cudaMemcpy(o->energy, at(S.energy), bytes, cudaMemcpyDeviceToHost));
+    if (o->p_final) real_out(S, o->p_final, at(S.P[h]), rows);
+    if (o->peak) real_out(S, o->peak, at(S.peak), rows);
+    if (o->energy) real_out(S, o->energy, at(S.energy), rows);
     for (int j = 0; j < S.n_dft; ++j) {
         const size_t src = (size_t)j * S.dcells * S.esz, dst = ((size_t)j * S.dft_glob_cells + S.dft_glob_off) * S.esz;
-        const size_t nb = (size_t)S.dcells * S.esz;
-        if (o->dft_re) BD_CUDA(cudaMemcpy(static_cast<char*>(o->dft_re) + dst, static_cast<const char*>(S.dre.p) + src, nb,
-                                          cudaMemcpyDeviceToHost));
-        if (o->dft_im) BD_CUDA(cudaMemcpy(static_cast<char*>(o->dft_im) + dst, static_cast<const char*>(S.dim.p) + src, nb,
-                                          cudaMemcpyDeviceToHost));
+        const long long drows = (long long)(S.dz_hi - S.dz_lo) * S.ny;
+        if (o->dft_re) real_out(S, static_cast<char*>(o->dft_re) + dst, static_cast<const char*>(S.dre.p) + src, drows);
+        if (o->dft_im) real_out(S, static_cast<char*>(o->dft_im) + dst, static_cast<const char*>(S.dim.p) + src, drows);
     }
     if (o->Q && S.p.q_mode == BD_Q_REFERENCE) {
         S.Qd.alloc(S.ctx, S.ncell * 8);
@@ -1033,7 +1137,7 @@ static void finish(WvSession& S, bd_westervelt_outputs* o) {
                                                        S.has_cmap ? S.cmap.as<float>() : nullptr,
                                                        S.has_matmap ? S.matmap.as<uint8_t>() : nullptr,
                                                        S.has_planemat ? S.planemat.as<int>() : nullptr,
-                                                       mats.as<bd_material>(), S.nx, S.ny, S.nz, S.p.q_iz_split,
+                                                       mats.as<bd_material>(), S.px, S.ny, S.nz, S.p.q_iz_split,
                                                        S.p.q_n_harm, S.n_dft, S.dz_lo, S.dz_hi, S.p.q_freq,
                                                        (double)S.p.dft_len, S.Qd.as<double>());
         else
@@ -1041,13 +1145,12 @@ static void finish(WvSession& S, bd_westervelt_outputs* o) {
                                                         S.has_cmap ? S.cmap.as<float>() : nullptr,
                                                         S.has_matmap ? S.matmap.as<uint8_t>() : nullptr,
                                                         S.has_planemat ? S.planemat.as<int>() : nullptr,
-                                                        mats.as<bd_material>(), S.nx, S.ny, S.nz, S.p.q_iz_split,
+                                                        mats.as<bd_material>(), S.px, S.ny, S.nz, S.p.q_iz_split,
                                                         S.p.q_n_harm, S.n_dft, S.dz_lo, S.dz_hi, S.p.q_freq,
                                                         (double)S.p.dft_len, S.Qd.as<double>());
         BD_LAUNCHED(S.ctx);
-        BD_CUDA(cudaMemcpyAsync(o->Q, S.Qd.as<double>() + (size_t)S.own0 * S.plane,
-                                (size_t)(S.own1 - S.own0) * S.plane * 8, cudaMemcpyDeviceToHost, st));
         BD_CUDA(cudaStreamSynchronize(st));
+        field_out<double>(S, o->Q, S.Qd.as<double>() + (size_t)S.own0 * S.plane, rows);
     }
     o->steps_done = S.step;
     o->tile_variant = S.variant;
@@ -1060,9 +1163,12 @@ struct CkHeader {
     int64_t step, dcells;
 };
 
+// cells of one DFT plane set in rows of nx
+static long long ck_dcells(const WvSession& S) { return S.n_dft > 0 ? (long long)(S.dz_hi - S.dz_lo) * S.hplane : 0; }
+
 static size_t ck_size(const WvSession& S) {
-    const size_t f = S.ncell * S.esz;
-    return sizeof(CkHeader) + f * (5 + 2 * (size_t)S.max_relax + 2) + 2 * (size_t)S.n_dft * S.dcells * S.esz;
+    const size_t f = (size_t)S.hplane * S.nz * S.esz;
+    return sizeof(CkHeader) + f * (5 + 2 * (size_t)S.max_relax + 2) + 2 * (size_t)S.n_dft * ck_dcells(S) * S.esz;
 }
 
 static void ck_save(WvSession& S, void* blob, size_t bytes) {
@@ -1072,21 +1178,22 @@ static void ck_save(WvSession& S, void* blob, size_t bytes) {
     std::memset(&h, 0, sizeof h);
     std::memcpy(h.magic, "BDCKPT01", 8);
     h.version = 1; h.precision = S.prec; h.nx = S.nx; h.ny = S.ny; h.nz = S.nz;
-    h.max_relax = S.max_relax; h.n_dft = S.n_dft; h.step = S.step; h.dcells = S.dcells;
+    h.max_relax = S.max_relax; h.n_dft = S.n_dft; h.step = S.step; h.dcells = ck_dcells(S);
     char* o = static_cast<char*>(blob);
     std::memcpy(o, &h, sizeof h);
     o += sizeof h;
-    const size_t f = S.ncell * S.esz;
+    const size_t f = (size_t)S.hplane * S.nz * S.esz;
+    const long long rows = (long long)S.ny * S.nz, drows = (long long)S.n_dft * (S.dz_hi - S.dz_lo) * S.ny;
     const int hd = head_of(S.step);
-    for (int k = 0; k < 5; ++k) { BD_CUDA(cudaMemcpy(o, S.P[(hd + k) % 5].p, f, cudaMemcpyDeviceToHost)); o += f; }
+    for (int k = 0; k < 5; ++k) { real_out(S, o, S.P[(hd + k) % 5].p, rows); o += f; }
     const int rh = (int)(S.step & 1);
     for (int v = 0; v < S.max_relax; ++v)
-        for (int k = 0; k < 2; ++k) { BD_CUDA(cudaMemcpy(o, S.R[v][rh ^ k].p, f, cudaMemcpyDeviceToHost)); o += f; }
-    BD_CUDA(cudaMemcpy(o, S.peak.p, f, cudaMemcpyDeviceToHost)); o += f;
-    BD_CUDA(cudaMemcpy(o, S.energy.p, f, cudaMemcpyDeviceToHost)); o += f;
+        for (int k = 0; k < 2; ++k) { real_out(S, o, S.R[v][rh ^ k].p, rows); o += f; }
+    real_out(S, o, S.peak.p, rows); o += f;
+    real_out(S, o, S.energy.p, rows); o += f;
     if (S.n_dft > 0) {
-        BD_CUDA(cudaMemcpy(o, S.dre.p, S.dre.bytes, cudaMemcpyDeviceToHost)); o += S.dre.bytes;
-        BD_CUDA(cudaMemcpy(o, S.dim.p, S.dim.bytes, cudaMemcpyDeviceToHost)); o += S.dim.bytes;
+        real_out(S, o, S.dre.p, drows); o += (size_t)drows * S.nx * S.esz;
+        real_out(S, o, S.dim.p, drows); o += (size_t)drows * S.nx * S.esz;
     }
 }
 
@@ -1096,22 +1203,23 @@ static void ck_load(WvSession& S, const void* blob, size_t bytes) {
     std::memcpy(&h, blob, sizeof h);
     if (std::memcmp(h.magic, "BDCKPT01", 8) != 0) fail(BD_ERR_INVALID_ARG, "not a checkpoint blob");
     if (h.precision != S.prec || h.nx != S.nx || h.ny != S.ny || h.nz != S.nz || h.max_relax != S.max_relax ||
-        h.n_dft != S.n_dft || h.dcells != S.dcells)
+        h.n_dft != S.n_dft || h.dcells != ck_dcells(S))
         fail(BD_ERR_STATE, "checkpoint geometry does not match this solve");
     if (bytes < ck_size(S)) fail(BD_ERR_INVALID_ARG, "checkpoint truncated");
     const char* in = static_cast<const char*>(blob) + sizeof h;
-    const size_t f = S.ncell * S.esz;
+    const size_t f = (size_t)S.hplane * S.nz * S.esz;
+    const long long rows = (long long)S.ny * S.nz, drows = (long long)S.n_dft * (S.dz_hi - S.dz_lo) * S.ny;
     BD_CUDA(cudaStreamSynchronize(S.ctx->stream));
     const int hd = head_of(h.step);
-    for (int k = 0; k < 5; ++k) { BD_CUDA(cudaMemcpy(S.P[(hd + k) % 5].p, in, f, cudaMemcpyHostToDevice)); in += f; }
+    for (int k = 0; k < 5; ++k) { real_in(S, S.P[(hd + k) % 5].p, in, rows); in += f; }
     const int rh = (int)(h.step & 1);
     for (int v = 0; v < S.max_relax; ++v)
-        for (int k = 0; k < 2; ++k) { BD_CUDA(cudaMemcpy(S.R[v][rh ^ k].p, in, f, cudaMemcpyHostToDevice)); in += f; }
-    BD_CUDA(cudaMemcpy(S.peak.p, in, f, cudaMemcpyHostToDevice)); in += f;
-    BD_CUDA(cudaMemcpy(S.energy.p, in, f, cudaMemcpyHostToDevice)); in += f;
+        for (int k = 0; k < 2; ++k) { real_in(S, S.R[v][rh ^ k].p, in, rows); in += f; }
+    real_in(S, S.peak.p, in, rows); in += f;
+    real_in(S, S.energy.p, in, rows); in += f;
     if (S.n_dft > 0) {
-        BD_CUDA(cudaMemcpy(S.dre.p, in, S.dre.bytes, cudaMemcpyHostToDevice)); in += S.dre.bytes;
-        BD_CUDA(cudaMemcpy(S.dim.p, in, S.dim.bytes, cudaMemcpyHostToDevice)); in += S.dim.bytes;
+        real_in(S, S.dre.p, in, drows); in += (size_t)drows * S.nx * S.esz;
+        real_in(S, S.dim.p, in, drows); in += (size_t)drows * S.nx * S.esz;
     }
     long long st = h.step;
     BD_CUDA(cudaMemcpy(S.step_base.p, &st, sizeof st, cudaMemcpyHostToDevice));
@@ -1821,7 +1929,7 @@ bd_status bd_westervelt_begin(bd_context* ctx, const bd_grid* grid, const bd_med
         ctx_check(ctx);
         auto* w = new bd_westervelt();
         try {
-            setup(w->S, ctx, grid, medium, source, params);
+            setup(w->S, ctx, grid, medium, source, params, true);
         } catch (...) {
             delete w;
             throw;
@@ -2058,7 +2166,7 @@ bd_status bd_westervelt_run(bd_context* ctx, const bd_grid* grid, const bd_mediu
         if (!out) fail(BD_ERR_INVALID_ARG, "null outputs");
         ctx_check(ctx);
         bd_westervelt w;
-        setup(w.S, ctx, grid, medium, source, params);
+        setup(w.S, ctx, grid, medium, source, params, true);
         timed_advance(w.S, params->n_steps, out);
         finish(w.S, out);
         out->elapsed_ms = w.S.last_ms;

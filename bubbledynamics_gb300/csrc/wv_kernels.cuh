@@ -38,7 +38,8 @@ template <class real>
 struct WvArgs {
     int nx, ny, nz;
     int zb;                    // z-chunk per CTA
-    long long plane;           // nx*ny
+    int px;                    // row pitch in cells
+    long long plane;           // px*ny
     // time levels: p^n (stencil), p^{n-1..n-3}, and the p^{n-4} buffer that receives p^{n+1}
     const real* __restrict__ p0;
     const real* __restrict__ p1;
@@ -174,7 +175,7 @@ __device__ __forceinline__ void accumulate(const WvArgs<real>& a, long long step
     if (step >= a.energy_start && step < a.energy_end) a.energy[i] = energy_add(a, a.energy[i], v, vm1);
     const long long ds = step - a.dft_start;
     if (a.n_dft > 0 && ds >= 0 && ds < a.dft_len && iz >= a.dz_lo && iz < a.dz_hi) {
-        const long long pl = (long long)(iz - a.dz_lo) * a.plane + (long long)iy * a.nx + ix;
+        const long long pl = (long long)(iz - a.dz_lo) * a.plane + (long long)iy * a.px + ix;
         const long long stride = (long long)(a.dz_hi - a.dz_lo) * a.plane;
         const real* tw = a.tw + ds * a.n_dft * 2;
         for (int j = 0; j < a.n_dft; ++j) {
@@ -308,11 +309,11 @@ __global__ void __launch_bounds__(TX* TY) wv_step_kernel(const WvArgs<real> a, c
         real wyk = real(1);
         if (jy < 0) { if (a.mir_y) jy = -jy; else { jy = iy; wyk = real(0); } }
         if (jy >= a.ny) { jy = iy; wyk = real(0); }
-        yo[k] = (jy - iy) * nx; yw[k] = wyk;
+        yo[k] = (jy - iy) * a.px; yw[k] = wyk;
     }
     const bool col_in_box = ix <= a.xhi && iy <= a.yhi;
     const real sw_xy = a.wx ? mul_(a.wx[ix], a.wy[iy]) : real(1);
-    const long long col = (long long)iy * nx + ix;
+    const long long col = (long long)iy * a.px + ix;
     // z window of p^n
     real w[7];
 #pragma unroll
@@ -376,7 +377,7 @@ __global__ void wv_mur_z_kernel(const WvArgs<real> a, const WvConst<real>* __res
     if ((a.mur_xp && ix >= a.nx - a.L) || (a.mur_yp && iy >= a.ny - a.L)) return;
     const WvConst<real>& K = *Kp;
     const long long step = *a.step_base + koff;
-    const long long col = (long long)iy * a.nx + ix;
+    const long long col = (long long)iy * a.px + ix;
     const real* Pn = a.p0;
     real* F = a.p4;
     if (a.mur_zm) {
@@ -411,7 +412,7 @@ __global__ void wv_mur_x_kernel(const WvArgs<real> a, const WvConst<real>* __res
     const real* Pn = a.p0;
     real* F = a.p4;
     for (int ix = a.nx - a.L; ix < a.nx; ++ix) {
-        const long long i = (long long)iz * a.plane + (long long)iy * a.nx + ix, j = i - 1;
+        const long long i = (long long)iz * a.plane + (long long)iy * a.px + ix, j = i - 1;
         const real c = cell_c(a, K, i, cell_mat(a, i, iz));
         const real v = Pn[j] + (F[j] - Pn[i]) * mur_k(c, a.dtdx);
         F[i] = v;
@@ -430,7 +431,7 @@ __global__ void wv_mur_y_kernel(const WvArgs<real> a, const WvConst<real>* __res
     const real* Pn = a.p0;
     real* F = a.p4;
     for (int iy = a.ny - a.L; iy < a.ny; ++iy) {
-        const long long i = (long long)iz * a.plane + (long long)iy * a.nx + ix, j = i - a.nx;
+        const long long i = (long long)iz * a.plane + (long long)iy * a.px + ix, j = i - a.px;
         const real c = cell_c(a, K, i, cell_mat(a, i, iz));
         const real v = Pn[j] + (F[j] - Pn[i]) * mur_k(c, a.dtdx);
         F[i] = v;

@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(TX* TY / CPT) wv_tma_kernel(const WvArgs<real>
     int own[CPT], qi[CPT];
     bool active[CPT], inbox[CPT], murxy[CPT];
     real swxy[CPT];
-    int col[CPT];                                  // column index iy * nx + ix (a plane has < 2^31 cells)
+    int col[CPT];                                  // column index iy * px + ix (a plane has < 2^31 cells)
 #pragma unroll
     for (int c = 0; c < CPT; ++c) {
         const int ty = tyt + c * RPT;
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(TX* TY / CPT) wv_tma_kernel(const WvArgs<real>
         inbox[c] = ix <= a.xhi && iy <= a.yhi;
         murxy[c] = (a.mur_yp && iy >= a.ny - a.L) || (a.mur_xp && ix >= a.nx - a.L);
         swxy[c] = (a.wx && active[c]) ? mul_(a.wx[ix], a.wy[iy]) : real(1);
-        col[c] = iy * a.nx + ix;
+        col[c] = iy * a.px + ix;
     }
     real w[CPT][7];
 #pragma unroll

@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
     int own[NC], qi[NC];
     bool active[NC], inbox[NC], murxy[NC];
     real swxy[NC];
-    int col[NC];                                   // column index iy * nx + ix (a plane has < 2^31 cells)
+    int col[NC];                                   // column index iy * px + ix (a plane has < 2^31 cells)
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
         const int ty = tyt + (c / CX) * RPT;
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
         inbox[c] = ix <= a.xhi && iy <= a.yhi;
         murxy[c] = (a.mur_yp && iy >= a.ny - a.L) || (a.mur_xp && ix >= a.nx - a.L);
         swxy[c] = (a.wx && active[c]) ? mul_(a.wx[ix], a.wy[iy]) : real(1);
-        col[c] = iy * a.nx + ix;
+        col[c] = iy * a.px + ix;
     }
     real w[NC][7];
     // p^n of this thread's cells on one plane tile into w[.][k]
