@@ -414,6 +414,28 @@ static void launch_step_t(WvSession& S, const WvArgs<real>& a, int koff, cudaStr
     BD_LAUNCHED(S.ctx);
 }
 
+// The Mur faces of a step (one kernel), after the stencil update.
+template <class real>
+static void launch_mur(WvSession& S, const WvArgs<real>& a, int koff, cudaStream_t st, int acc) {
+    const long long cx = a.mur_xp ? a.nx - a.L : a.nx, cy = a.mur_yp ? a.ny - a.L : a.ny;
+    const long long n = (a.mur_zm ? cx * cy * a.Lzm : 0) + (a.mur_zp ? cx * cy : 0) + (a.mur_xp ? cy * a.nz : 0) +
+                        (a.mur_yp ? (long long)a.nx * a.nz : 0);
+    if (n <= 0) return;
+    const unsigned groups = acc == ACC_ALL && a.n_dft > 0 ? 1 + (a.n_dft + MUR_FREQS - 1) / MUR_FREQS : 1;
+    const WvConst<real>* K = S.kconst.as<WvConst<real>>();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((n + 127) / 128), 1, groups);
+    cfg.blockDim = dim3(128);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = S.pdl ? 1 : 0;
+    BD_CUDA(cudaLaunchKernelEx(&cfg, wv_mur_kernel<real>, a, K, koff));
+    BD_LAUNCHED(S.ctx);
+}
+
 template <class real>
 static void launch_step(WvSession& S, int variant, int64_t s, int koff, cudaStream_t st, int acc) {
     WvArgs<real> a = make_args<real>(S, s);
@@ -439,24 +461,7 @@ static void launch_step(WvSession& S, int variant, int64_t s, int koff, cudaStre
         case 15: launch_tma_t<real, 32, 8, 1, 1>(S, a, s, koff, st); break;
         default: fail(BD_ERR_INVALID_ARG, "bad tile variant %d", variant);
     }
-    if (S.any_mur) {
-        const WvConst<real>* K = S.kconst.as<WvConst<real>>();
-        if (a.mur_zm || a.mur_zp) {
-            dim3 b(32, 8), gr((S.nx + 31) / 32, (S.ny + 7) / 8);
-            wv_mur_z_kernel<real><<<gr, b, 0, st>>>(a, K, koff);
-            BD_LAUNCHED(S.ctx);
-        }
-        if (a.mur_xp) {
-            dim3 b(128), gr((S.ny + 127) / 128, S.nz);
-            wv_mur_x_kernel<real><<<gr, b, 0, st>>>(a, K, koff);
-            BD_LAUNCHED(S.ctx);
-        }
-        if (a.mur_yp) {
-            dim3 b(128), gr((S.nx + 127) / 128, S.nz);
-            wv_mur_y_kernel<real><<<gr, b, 0, st>>>(a, K, koff);
-            BD_LAUNCHED(S.ctx);
-        }
-    }
+    if (S.any_mur) launch_mur<real>(S, a, koff, st, acc);
 }
 
 // Issue steps [s, s+n) on the stream (no graph): kernels read *step_base + koff,
@@ -498,15 +503,7 @@ static void build_graph(WvSession& S, int acc) {
     S.graph_variant[acc] = S.variant;
 }
 
-static int64_t launches_per_step(const WvSession& S) {
-    int64_t n = 1;
-    if (S.any_mur) {
-        if (S.g.face[4] == BD_FACE_MUR || S.g.face[5] == BD_FACE_MUR) n++;
-        if (S.g.face[1] == BD_FACE_MUR) n++;
-        if (S.g.face[3] == BD_FACE_MUR) n++;
-    }
-    return n;
-}
+static int64_t launches_per_step(const WvSession& S) { return S.any_mur ? 2 : 1; }
 
 static void probe(WvSession& S) {
     unsigned* f = S.flag.as<unsigned>();

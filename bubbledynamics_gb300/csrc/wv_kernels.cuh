@@ -368,74 +368,159 @@ __device__ __forceinline__ real mur_k(real c, real dth) {
     return (a - real(1)) / (a + real(1));
 }
 
-// Mur on the z faces (W:101-113) for columns outside the x+/y+ layers.
+// One layer of the Mur condition (W:101-133): P^{n+1} of the cell from P^{n+1} (nb)
+// and P^n (pj) of its inner neighbour and P^n of the cell.
 template <class real>
-__global__ void wv_mur_z_kernel(const WvArgs<real> a, const WvConst<real>* __restrict__ Kp, int koff) {
-    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
-    const int iy = blockIdx.y * blockDim.y + threadIdx.y;
-    if (ix >= a.nx || iy >= a.ny) return;
-    if ((a.mur_xp && ix >= a.nx - a.L) || (a.mur_yp && iy >= a.ny - a.L)) return;
-    const WvConst<real>& K = *Kp;
-    const long long step = *a.step_base + koff;
-    const long long col = (long long)iy * a.px + ix;
-    const real* Pn = a.p0;
-    real* F = a.p4;
-    if (a.mur_zm) {
-        for (int iz = 0; iz < a.Lzm; ++iz) {
-            const long long i = (long long)iz * a.plane + col, j = i + a.plane;
-            const real nb = (iz + 1 < a.Lzm) ? Pn[j] : F[j];   // pre-boundary value of P_next is p^n in W
-            const real c = cell_c(a, K, i, cell_mat(a, i, iz));
-            const real v = Pn[j] + (nb - Pn[i]) * mur_k(c, a.dtdz);
-            F[i] = v;
-            accumulate(a, step, i, ix, iy, iz, v, a.energy_mode == BD_ENERGY_DPDT2 ? a.p1[i] : real(0));
-        }
-    }
-    if (a.mur_zp) {
-        for (int iz = a.nz - a.L; iz < a.nz; ++iz) {
-            const long long i = (long long)iz * a.plane + col, j = i - a.plane;
-            const real c = cell_c(a, K, i, cell_mat(a, i, iz));
-            const real v = Pn[j] + (F[j] - Pn[i]) * mur_k(c, a.dtdz);
-            F[i] = v;
-            accumulate(a, step, i, ix, iy, iz, v, a.energy_mode == BD_ENERGY_DPDT2 ? a.p1[i] : real(0));
-        }
-    }
+__device__ __forceinline__ real mur_cell(real pj, real nb, real pi, real c, real dth) {
+    return pj + (nb - pi) * mur_k(c, dth);
 }
 
-// Mur on the x+ face (W:122-126), rows outside the y+ layers, inner layer first.
-template <class real>
-__global__ void wv_mur_x_kernel(const WvArgs<real> a, const WvConst<real>* __restrict__ Kp, int koff) {
-    const int iy = blockIdx.x * blockDim.x + threadIdx.x;
-    const int iz = blockIdx.y;
-    if (iy >= a.ny || (a.mur_yp && iy >= a.ny - a.L)) return;
-    const WvConst<real>& K = *Kp;
-    const long long step = *a.step_base + koff;
-    const real* Pn = a.p0;
-    real* F = a.p4;
-    for (int ix = a.nx - a.L; ix < a.nx; ++ix) {
-        const long long i = (long long)iz * a.plane + (long long)iy * a.px + ix, j = i - 1;
-        const real c = cell_c(a, K, i, cell_mat(a, i, iz));
-        const real v = Pn[j] + (F[j] - Pn[i]) * mur_k(c, a.dtdx);
-        F[i] = v;
-        accumulate(a, step, i, ix, iy, iz, v, a.energy_mode == BD_ENERGY_DPDT2 ? a.p1[i] : real(0));
-    }
-}
+constexpr int MUR_MAXL = 8;    // layers of an x+, y+ or z+ face
+constexpr int MUR_FREQS = 2;   // DFT frequencies per block of the Mur kernel's DFT groups
 
-// Mur on the y+ face (W:129-133), all columns, inner layer first.
+// The Mur faces of a step in one pass, in the order z-, z+, x+, y+ of a serial
+// launch of W:88-135.  Every cell's value follows from P^n and from the cells the
+// stencil update wrote, which this kernel only reads: a thread takes one run of
+// layers (or one z- cell, whose neighbour is P^n or the source plane) and, where
+// the run starts on a cell that an earlier face overwrites, forms that cell's
+// value itself.  Three kernels, one per face, whose threads re-read each layer
+// they had just written took 26 us a step on 107 x 107 x 401 cells outside the DFT
+// window and several times that inside it (FP64 64 x 64 x 201, 600 steps, 400 of
+// them in the window: the solve went from 173 to 140 ms).
+// In the DFT window blocks with blockIdx.z > 0 form the same values again and
+// add them to MUR_FREQS frequencies each (one thread adding ten frequencies in
+// turn waited for twenty dependent round trips a layer).
 template <class real>
-__global__ void wv_mur_y_kernel(const WvArgs<real> a, const WvConst<real>* __restrict__ Kp, int koff) {
-    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
-    const int iz = blockIdx.y;
-    if (ix >= a.nx) return;
+__global__ void __launch_bounds__(128) wv_mur_kernel(const WvArgs<real> a, const WvConst<real>* __restrict__ Kp, int koff) {
     const WvConst<real>& K = *Kp;
+    const int L = a.L;
+    const int cx = a.mur_xp ? a.nx - L : a.nx, cy = a.mur_yp ? a.ny - L : a.ny;   // columns outside the x+ / y+ layers
+    const long long n_zm = a.mur_zm ? (long long)cx * cy * a.Lzm : 0, n_zp = a.mur_zp ? (long long)cx * cy : 0;
+    const long long n_x = a.mur_xp ? (long long)cy * a.nz : 0, n_y = a.mur_yp ? (long long)a.nx * a.nz : 0;
+    long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    // the previous kernel's fields (a no-op for an ordinary launch); the next step's prologue may start
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (t >= n_zm + n_zp + n_x + n_y) return;
     const long long step = *a.step_base + koff;
-    const real* Pn = a.p0;
+    const real* __restrict__ Pn = a.p0;
     real* F = a.p4;
-    for (int iy = a.ny - a.L; iy < a.ny; ++iy) {
-        const long long i = (long long)iz * a.plane + (long long)iy * a.px + ix, j = i - a.px;
-        const real c = cell_c(a, K, i, cell_mat(a, i, iz));
-        const real v = Pn[j] + (F[j] - Pn[i]) * mur_k(c, a.dtdx);
-        F[i] = v;
-        accumulate(a, step, i, ix, iy, iz, v, a.energy_mode == BD_ENERGY_DPDT2 ? a.p1[i] : real(0));
+    auto c_at = [&](long long i, int iz) { return cell_c(a, K, i, cell_mat(a, i, iz)); };
+    // value of a cell of column `col` (outside the x+ / y+ layers) after the z faces
+    auto zval = [&](long long col, int iz) -> real {
+        const long long i = (long long)iz * a.plane + col;
+        if (a.mur_zm && iz < a.Lzm) {
+            const long long j = i + a.plane;
+            const real pj = Pn[j];
+            return mur_cell(pj, iz + 1 < a.Lzm ? pj : F[j], Pn[i], c_at(i, iz), a.dtdz);   // P_next is p^n in W before the face
+        }
+        if (a.mur_zp && iz >= a.nz - L) {
+            const long long i0 = (long long)(a.nz - L) * a.plane + col;
+            real f = F[i0 - a.plane];
+            for (int z = a.nz - L; z <= iz; ++z) {
+                const long long k = (long long)z * a.plane + col;
+                f = mur_cell(Pn[k - a.plane], f, Pn[k], c_at(k, z), a.dtdz);
+            }
+            return f;
+        }
+        return F[i];
+    };
+    // the run: nl cells from i0, `st` apart, the first after a cell of value f
+    long long i0 = 0, st = 0;
+    int iz = 0, nl = L, dzl = 0;
+    real f = real(0), dth = a.dtdx;
+    if (t < n_zm) {
+        const long long col0 = t % ((long long)cx * cy);
+        iz = (int)(t / ((long long)cx * cy));
+        const long long col = (col0 / cx) * a.px + col0 % cx;
+        i0 = (long long)iz * a.plane + col;
+        f = zval(col, iz);
+        nl = 0;                                     // a single cell, already formed
+    } else if ((t -= n_zm) < n_zp) {
+        const long long col = (t / cx) * a.px + t % cx;
+        iz = a.nz - L;
+        i0 = (long long)iz * a.plane + col;
+        st = a.plane;
+        dzl = 1;
+        dth = a.dtdz;
+        f = F[i0 - st];
+    } else if ((t -= n_zp) < n_x) {
+        const int iy = (int)(t % cy);
+        iz = (int)(t / cy);
+        const long long col = (long long)iy * a.px + a.nx - L;
+        i0 = (long long)iz * a.plane + col;
+        st = 1;
+        f = zval(col - 1, iz);
+    } else {
+        t -= n_x;
+        const int ix = (int)(t % a.nx);
+        iz = (int)(t / a.nx);
+        const long long col = (long long)(a.ny - L) * a.px + ix;
+        i0 = (long long)iz * a.plane + col;
+        st = a.px;
+        if (ix < cx) f = zval(col - st, iz);
+        else {                                      // the row below is an x+ run
+            long long k = (long long)iz * a.plane + (col - st) - (ix - (a.nx - L));
+            f = zval(k - (long long)iz * a.plane - 1, iz);
+            for (int x = a.nx - L; x <= ix; ++x, ++k) f = mur_cell(Pn[k - 1], f, Pn[k], c_at(k, iz), a.dtdx);
+        }
+    }
+    real v[MUR_MAXL];
+    v[0] = f;
+    if (nl > 0) {
+        real pj = Pn[i0 - st];
+#pragma unroll
+        for (int l = 0; l < MUR_MAXL; ++l) {
+            if (l >= nl) break;
+            const long long i = i0 + l * st;
+            const real pi = Pn[i];
+            f = mur_cell(pj, f, pi, c_at(i, iz + l * dzl), dth);
+            v[l] = f;
+            pj = pi;
+        }
+    } else nl = 1;
+    if (blockIdx.z == 0) {
+        const bool do_peak = step >= a.peak_start && step < a.peak_end;
+        const bool do_energy = step >= a.energy_start && step < a.energy_end;
+#pragma unroll
+        for (int l = 0; l < MUR_MAXL; ++l) {
+            if (l >= nl) break;
+            const long long i = i0 + l * st;
+            F[i] = v[l];
+            if (do_peak) {
+                const real av = fabs(v[l]), pk = a.peak[i];
+                a.peak[i] = av > pk ? av : pk;
+            }
+            if (do_energy) a.energy[i] = energy_add(a, a.energy[i], v[l], a.energy_mode == BD_ENERGY_DPDT2 ? a.p1[i] : real(0));
+        }
+        return;
+    }
+    const long long ds = step - a.dft_start;
+    if (ds < 0 || ds >= a.dft_len) return;
+    const long long stride = (long long)(a.dz_hi - a.dz_lo) * a.plane, off = (long long)a.dz_lo * a.plane;
+    const int j0 = (blockIdx.z - 1) * MUR_FREQS;
+    const real* tw = a.tw + ds * a.n_dft * 2;
+#pragma unroll
+    for (int u = 0; u < MUR_FREQS; ++u) {
+        const int j = j0 + u;
+        if (j >= a.n_dft) break;
+        real* dr = a.dre + j * stride - off;
+        real* di = a.dim + j * stride - off;
+        const real tr = tw[2 * j], ti = tw[2 * j + 1];
+        real r[MUR_MAXL], m[MUR_MAXL];
+#pragma unroll
+        for (int l = 0; l < MUR_MAXL; ++l) {        // every load before any store
+            const int z = iz + l * dzl;
+            if (l < nl && z >= a.dz_lo && z < a.dz_hi) { r[l] = dr[i0 + l * st]; m[l] = di[i0 + l * st]; }
+        }
+#pragma unroll
+        for (int l = 0; l < MUR_MAXL; ++l) {
+            const int z = iz + l * dzl;
+            if (l < nl && z >= a.dz_lo && z < a.dz_hi) {
+                dr[i0 + l * st] = fma_(v[l], tr, r[l]);
+                di[i0 + l * st] = fma_(-v[l], ti, m[l]);
+            }
+        }
     }
 }
 
