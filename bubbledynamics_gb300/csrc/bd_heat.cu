@@ -146,7 +146,11 @@ __global__ void heat_step_kernel(const HeatArgs<real> a, int koff) {
         if (sizeof(real) == 8) {
             const double Tc = (double)tn - 273.15;                     // T:88
             // T:99-102
-            a.TD[i] = a.TD[i] + (Tc < 43.0 ? pow(4.0, Tc - 43.0) : pow(2.0, Tc - 43.0)) * (double)a.dt;
+            // (one exp2 for both bases: 4^y = 2^2y, to exp2's 2 ulp as with pow's;
+            // pow took 110 of the 150 FP64 instructions of a cell; 107 x 107 x 126:
+            // 438 us a step with it, about 120 without)
+            const double y = Tc - 43.0;
+            a.TD[i] = a.TD[i] + exp2(Tc < 43.0 ? 2.0 * y : y) * (double)a.dt;
         } else {
             const float x = (float)tn + a.T_refm43;                    // T_C - 43
             const float inc = __fmul_rn(dose_rate(x), (float)a.dt);
