@@ -139,6 +139,7 @@ static WvArgs<real> make_args(WvSession& S, int64_t s) {
     std::memset(&a, 0, sizeof a);
     a.nx = S.nx; a.ny = S.ny; a.nz = S.nz;
     a.px = S.px;
+    a.rev = (int)(s & 1);
     a.plane = S.plane;
     const int h = head_of(s);
     a.p0 = S.P[(h + 0) % 5].as<real>();

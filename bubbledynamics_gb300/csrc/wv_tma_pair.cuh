@@ -78,9 +78,15 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
     const int tx = threadIdx.x, tyt = threadIdx.y;
     const int tid = tyt * TXT + tx;
     const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
-    const int z0 = blockIdx.z * a.zb;
+    // every other step marches from the high end (chunks and planes), so that it
+    // starts on what the step before it left in L2; the z stencil is symmetric, so
+    // the bits are the same
+    const int bz = a.rev ? gridDim.z - 1 - blockIdx.z : blockIdx.z;
+    const int z0 = bz * a.zb;
     const int z1 = min(a.nz, z0 + a.zb);
     const int zbn = z1 - z0;
+    const int zf = a.rev ? z1 - 1 : z0, zd = a.rev ? -1 : 1;   // first plane, direction
+    auto zof = [&](int r) { return zf + zd * r; };             // r-th plane of the march
 
     for (int e = tid; e < (int)(BD_MAX_MATERIALS * sizeof(MatConst<real>) / 4); e += NT)
         reinterpret_cast<unsigned*>(sK)[e] = reinterpret_cast<const unsigned*>(Kp)[e];
@@ -90,10 +96,10 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
     };
     auto qslot = [&](int r) { return Qring + (r % NQ) * L::QS; };
 
-    // producer (thread 0): plane q = plane - (z0 - 3) of p^n, plane r = plane - z0 of the pointwise tiles
+    // producer (thread 0): march plane q - 3 of p^n, march plane r of the pointwise tiles
     auto issueP = [&](int q) {
         if (q > zbn + 5) return;
-        const int plane = z0 - 3 + q;
+        const int plane = zof(q - 3);
         uint64_t* bar = &barP[q % TMA_NP];
         if (plane < 0 || plane >= a.nz) { mbar_arrive(bar); return; }   // read as zeros, nothing to copy
         mbar_expect_tx(bar, L::PW * L::PH * (unsigned)sizeof(real));
@@ -105,7 +111,7 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
     bool pf_dft = false;
     auto issueQ = [&](int r) {
         if (r >= zbn) return;
-        const int plane = z0 + r;
+        const int plane = zof(r);
         if (pf_dft && plane >= a.dz_lo && plane < a.dz_hi) {
             const int ndz = a.dz_hi - a.dz_lo;
             for (int j = 0; j < a.n_dft; ++j) {
@@ -182,9 +188,9 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
         }
     };
 #pragma unroll
-    for (int k = 0; k < 6; ++k) {                  // planes z0-3 .. z0+2
+    for (int k = 0; k < 6; ++k) {                  // the first plane and three on either side, but the last
         waitP(k);
-        const int plane = z0 - 3 + k;
+        const int plane = zof(k - 3);
         load_w(pslot(k), plane >= 0 && plane < a.nz, k);
     }
     // every cell of the tile inside the grid and the update box and on no x / y
@@ -195,9 +201,9 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
         bool mine = true;
 #pragma unroll
         for (int c = 0; c < NC; ++c) mine = mine && active[c] && inbox[c] && !murxy[c];
-        tile_fast = __syncthreads_and(mine) != 0;      // also: slots of planes z0-3..z0-1 are free again
+        tile_fast = __syncthreads_and(mine) != 0;      // also: the slots of the three planes before the first are free again
     } else {
-        __syncthreads();                               // slots of planes z0-3..z0-1 are free again
+        __syncthreads();                               // the slots of the three planes before the first are free again
     }
     if (tid == 0)
         for (int q = TMA_NP; q < TMA_NP + 3; ++q) issueP(q);
@@ -212,17 +218,17 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
     // the material of single-material problems, in registers
     const MatConst<real> M0 = sK[0];
 
-    for (int izg = z0; izg < z1; izg += ZU) {
+    for (int rg = 0; rg < zbn; rg += ZU) {
         // the last planes of this CTA: the next step's grid may start its prologue
-        if (izg + ZU >= z1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        if (rg + ZU >= zbn) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 #pragma unroll
     for (int u = 0; u < ZU; ++u) {
-        const int iz = izg + u;
-        if (iz >= z1) break;
-        const int qc = iz - z0 + 3;                // stencil plane
-        const int r = iz - z0;
+        const int r = rg + u;
+        if (r >= zbn) break;
+        const int iz = zof(r);
+        const int qc = r + 3;                      // stencil plane
         waitP(qc + 3);
-        load_w(pslot(qc + 3), iz + 3 < a.nz, 6);
+        load_w(pslot(qc + 3), (unsigned)zof(r + 3) < (unsigned)a.nz, 6);
         real* T = pslot(qc);
         if (fix_x || fix_y) {                      // mirror planes x = 0 / y = 0 (W:176-200)
             if (fix_x)
@@ -481,12 +487,12 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
 #pragma unroll
             for (int k = 0; k < 6; ++k) w[c][k] = w[c][k + 1];
     }
-        __syncthreads();                           // everyone is done with planes izg..izg+ZU-1 and their tiles
+        __syncthreads();                           // everyone is done with this round's planes and their tiles
         if (tid == 0) {
 #pragma unroll
             for (int u = 0; u < ZU; ++u) {
-                issueP(izg + u - z0 + 3 + TMA_NP);
-                issueQ(izg + u - z0 + NQ);
+                issueP(rg + u + 3 + TMA_NP);
+                issueQ(rg + u + NQ);
             }
         }
     }
