@@ -33,6 +33,14 @@ struct HeatMat {
     real wTa;       // w dt (T_art - T_ref)
 };
 
+// What a step does with the dose.  The dose is most of a step's traffic (16 of 28
+// bytes a cell), and a step's increment follows from its temperature alone, which
+// the next step reads anyway: of two steps the first leaves the dose alone
+// (DOSE_LATER) and the second adds both increments, in order (DOSE_BOTH), at 12 + 28
+// bytes for the two.  256 x 256 x 384: 92 us a step, 106 with DOSE_THIS alone;
+// 213 x 213 x 201: 41 and 45.
+enum HeatDose { DOSE_LATER = 0, DOSE_THIS = 1, DOSE_BOTH = 2 };
+
 template <class real>
 struct HeatArgs {
     int nx, ny, nz, zb;
@@ -117,7 +125,7 @@ __device__ __forceinline__ float heat_cell(const HeatMat<float>& M, float tc, fl
     return __fadd_rn(t, M.wTa);
 }
 
-template <class real>
+template <class real, int DOSE>
 __global__ void heat_step_kernel(const HeatArgs<real> a, int koff) {
     const int ix = blockIdx.x * blockDim.x + threadIdx.x;
     const int iy = blockIdx.y * blockDim.y + threadIdx.y;
@@ -143,19 +151,30 @@ __global__ void heat_step_kernel(const HeatArgs<real> a, int koff) {
         if constexpr (sizeof(real) == 8) tn = tcv * M.a0 + M.kxy * sxy + M.kz * (tpv + tmv) + M.qc * q + M.wTa;
         else tn = heat_cell(M, tcv, sxy, tpv + tmv, q);
         a.Tout[i] = tn;
-        if (sizeof(real) == 8) {
-            const double Tc = (double)tn - 273.15;                     // T:88
-            // T:99-102
-            // (one exp2 for both bases: 4^y = 2^2y, to exp2's 2 ulp as with pow's;
-            // pow took 110 of the 150 FP64 instructions of a cell; 107 x 107 x 126:
+        if constexpr (DOSE == DOSE_LATER) return;
+        else if constexpr (sizeof(real) == 8) {
+            // T:88, T:99-102 (one exp2 for both bases: 4^y = 2^2y, to exp2's 2 ulp as with
+            // pow's; pow took 110 of the 150 FP64 instructions of a cell; 107 x 107 x 126:
             // 438 us a step with it, about 120 without)
-            const double y = Tc - 43.0;
-            a.TD[i] = a.TD[i] + exp2(Tc < 43.0 ? 2.0 * y : y) * (double)a.dt;
+            auto add = [&](double d, double T) {
+                const double y = T - 273.15 - 43.0;
+                return d + exp2(y < 0.0 ? 2.0 * y : y) * (double)a.dt;
+            };
+            double d = a.TD[i];
+            if (DOSE == DOSE_BOTH) d = add(d, tcv);
+            a.TD[i] = add(d, tn);
         } else {
-            const float x = (float)tn + a.T_refm43;                    // T_C - 43
-            const float inc = __fmul_rn(dose_rate(x), (float)a.dt);
-            if (a.TD) a.TD[i] = dose_add(a.TD[i], inc);
-            else a.TDf[i] = df_add(a.TDf[i], inc);
+            const float inc0 = __fmul_rn(dose_rate((float)tcv + a.T_refm43), (float)a.dt);
+            const float inc = __fmul_rn(dose_rate((float)tn + a.T_refm43), (float)a.dt);   // x = T_C - 43
+            if (a.TD) {
+                double d = a.TD[i];
+                if (DOSE == DOSE_BOTH) d = dose_add(d, inc0);
+                a.TD[i] = dose_add(d, inc);
+            } else {
+                float2 d = a.TDf[i];
+                if (DOSE == DOSE_BOTH) d = df_add(d, inc0);
+                a.TDf[i] = df_add(d, inc);
+            }
         }
     };
     auto sxy_at = [&](int iz) {
@@ -194,7 +213,7 @@ __global__ void heat_step_kernel(const HeatArgs<real> a, int koff) {
 // (they are written back unchanged), like the scalar kernel.  Every other step
 // marches the planes (and the chunks) from the high end, so that it starts on the
 // planes the step before it left in L2.  PAIR: the dose is a (hi, lo) float pair.
-template <bool PAIR>
+template <bool PAIR, int DOSE>
 __global__ void __launch_bounds__(128) heat_step4_kernel(const HeatArgs<float> a, int koff) {
     const int x0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
     const int iy = blockIdx.y * blockDim.y + threadIdx.y;
@@ -231,7 +250,11 @@ __global__ void __launch_bounds__(128) heat_step4_kernel(const HeatArgs<float> a
             q[k] = (qrow && ixa >= 0 && ixa < a.nx) ? __ldg(a.Q + (long long)iz * P + (long long)iya * NX + ixa) : 0.f;
         }
         double2* dp = PAIR ? reinterpret_cast<double2*>(a.TDf + i) : reinterpret_cast<double2*>(a.TD + i);
-        double2 d01 = dp[0], d23 = dp[1];
+        double2 d01 = make_double2(0.0, 0.0), d23 = d01;
+        if constexpr (DOSE != DOSE_LATER) {
+            d01 = dp[0];
+            d23 = dp[1];
+        }
         int mats[4];
         if (a.matmap) {
             const uchar4 mm = *reinterpret_cast<const uchar4*>(a.matmap + i);
@@ -251,21 +274,27 @@ __global__ void __launch_bounds__(128) heat_step4_kernel(const HeatArgs<float> a
             const float sxy = xl[k] + xr[k] + su[k] + sd[k];
             const float t = heat_cell(a.mat[mats[k]], cv[k], sxy, zu[k] + zd[k], q[k]);
             tn[k] = upd[k] ? t : cv[k];
-            if (upd[k]) {
-                const float inc = __fmul_rn(dose_rate(t + a.T_refm43), a.dt);
-                if constexpr (PAIR) {
-                    float2 d;
-                    memcpy(&d, &dose[k], 8);
-                    d = df_add(d, inc);
-                    memcpy(&dose[k], &d, 8);
-                } else {
-                    dose[k] = dose_add(dose[k], inc);
-                }
+            if (DOSE != DOSE_LATER && upd[k]) {
+                auto add = [&](float T) {
+                    const float inc = __fmul_rn(dose_rate(T + a.T_refm43), a.dt);
+                    if constexpr (PAIR) {
+                        float2 d;
+                        memcpy(&d, &dose[k], 8);
+                        d = df_add(d, inc);
+                        memcpy(&dose[k], &d, 8);
+                    } else {
+                        dose[k] = dose_add(dose[k], inc);
+                    }
+                };
+                if (DOSE == DOSE_BOTH) add(cv[k]);               // the previous step's
+                add(t);
             }
         }
         *reinterpret_cast<float4*>(a.Tout + i) = make_float4(tn[0], tn[1], tn[2], tn[3]);
-        dp[0] = make_double2(dose[0], dose[1]);
-        dp[1] = make_double2(dose[2], dose[3]);
+        if constexpr (DOSE != DOSE_LATER) {
+            dp[0] = make_double2(dose[0], dose[1]);
+            dp[1] = make_double2(dose[2], dose[3]);
+        }
         tm = tc;
         tc = tp;
     }
@@ -288,13 +317,33 @@ static int march_zb(bd_context* ctx, long long tiles, int nz, int per_sm) {
     }
     return best;
 }
+// dose mode of step k of a run of cnt consecutive steps: pairs, and the odd one out
+static int dose_mode(int64_t k, int64_t cnt) {
+    return k % 2 == 1 ? DOSE_BOTH : k + 1 < cnt ? DOSE_LATER : DOSE_THIS;
+}
+
+template <bool PAIR>
+static void step4_launch(const HeatArgs<float>& a, int koff, int mode, dim3 grid, cudaStream_t st) {
+    const dim3 block(16, 8);
+    if (mode == DOSE_LATER) heat_step4_kernel<PAIR, DOSE_LATER><<<grid, block, 0, st>>>(a, koff);
+    else if (mode == DOSE_THIS) heat_step4_kernel<PAIR, DOSE_THIS><<<grid, block, 0, st>>>(a, koff);
+    else heat_step4_kernel<PAIR, DOSE_BOTH><<<grid, block, 0, st>>>(a, koff);
+}
+template <class real>
+static void step_launch(const HeatArgs<real>& a, int koff, int mode, dim3 grid, cudaStream_t st) {
+    const dim3 block(32, 8);
+    if (mode == DOSE_LATER) heat_step_kernel<real, DOSE_LATER><<<grid, block, 0, st>>>(a, koff);
+    else if (mode == DOSE_THIS) heat_step_kernel<real, DOSE_THIS><<<grid, block, 0, st>>>(a, koff);
+    else heat_step_kernel<real, DOSE_BOTH><<<grid, block, 0, st>>>(a, koff);
+}
+
 static dim3 step4_grid(int px, int ny, int nz, int zb) {
     return dim3((px / 4 + 15) / 16, (ny + 7) / 8, (nz + zb - 1) / zb);
 }
 static int step4_zb(bd_context* ctx, int px, int ny, int nz) {
     static const int per_sm = [] {
         int n = 0;
-        BD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_step4_kernel<false>, 128, 0));
+        BD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_step4_kernel<false, DOSE_BOTH>, 128, 0));
         return n;
     }();
     return march_zb(ctx, (long long)((px / 4 + 15) / 16) * ((ny + 7) / 8), nz, per_sm);
@@ -302,7 +351,7 @@ static int step4_zb(bd_context* ctx, int px, int ny, int nz) {
 static int scalar_zb(bd_context* ctx, int nx, int ny, int nz) {
     static const int per_sm = [] {
         int n = 0;
-        BD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_step_kernel<float>, 256, 0));
+        BD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_step_kernel<float, DOSE_BOTH>, 256, 0));
         return n;
     }();
     return march_zb(ctx, (long long)((nx + 31) / 32) * ((ny + 7) / 8), nz, per_sm);
@@ -657,18 +706,18 @@ struct HeatPlan {
     // steps s0 .. s0 + cnt - 1 of every local slab: the kernels read their step as
     // the device counter plus their offset, and one advance kernel moves the counter
     void issue(cudaStream_t st, int64_t s0, int cnt) {
-        const dim3 block(32, 8);
         for (int k = 0; k < cnt; ++k) {
+            const int mode = dose_mode(k, cnt);
             const bool a_to_b = ((s0 + k) % 2) == 0;
             for (const HeatSlab& S : sl) {
                 if (f64) {
                     HeatArgs<double> a = ad;
                     fill<HeatArgs<double>, double>(a, S, a_to_b);
-                    heat_step_kernel<double><<<S.grid, block, 0, st>>>(a, k);
+                    step_launch(a, k, mode, S.grid, st);
                 } else {
                     HeatArgs<float> a = af;
                     fill<HeatArgs<float>, float>(a, S, a_to_b);
-                    heat_step4_kernel<false><<<S.grid4, dim3(16, 8), 0, st>>>(a, k);
+                    step4_launch<false>(a, k, mode, S.grid4, st);
                 }
                 BD_LAUNCHED(ctx);
             }
@@ -1005,15 +1054,16 @@ bd_status bd_heat_run_device_noalloc(bd_context* ctx, const bd_thermal* th, floa
         // the caller's rows are not padded: whole-vector rows and 16-byte aligned buffers take the four-cell kernel
         const bool vec = nx % 4 == 0 && (reinterpret_cast<uintptr_t>(d_theta) | reinterpret_cast<uintptr_t>(d_dose)) % 16 == 0;
         a.zb = vec ? step4_zb(ctx, nx, ny, nz) : scalar_zb(ctx, nx, ny, nz);
-        const dim3 block(32, 8), grid((nx + 31) / 32, (ny + 7) / 8, (nz + a.zb - 1) / a.zb);
+        const dim3 grid((nx + 31) / 32, (ny + 7) / 8, (nz + a.zb - 1) / a.zb);
         const dim3 grid4 = step4_grid(nx, ny, nz, a.zb);
         for (int64_t k = 0; k < n_steps; ++k) {
             const bool even = k % 2 == 0;                    // even steps read the caller's field
             a.rev = even ? 0 : 1;
             a.Tin = even ? d_theta : sc.theta;
             a.Tout = even ? sc.theta : d_theta;
-            if (vec) heat_step4_kernel<true><<<grid4, dim3(16, 8), 0, s>>>(a, (int)k);
-            else heat_step_kernel<float><<<grid, block, 0, s>>>(a, (int)k);
+            const int mode = dose_mode(k, n_steps);
+            if (vec) step4_launch<true>(a, (int)k, mode, grid4, s);
+            else step_launch(a, (int)k, mode, grid, s);
             BD_LAUNCHED(ctx);
         }
         if (n_steps % 2 == 1)   // the latest field is in the partner buffer
