@@ -352,6 +352,7 @@ static void launch_tma_t(WvSession& S, const WvArgs<real>& a, int64_t s, int kof
         launch_tma_k<real, TX, TY, CPT, 1, ZU, 3>(S, a, maps, koff, st);   // one material, c map (cfg1)
     else if (sizeof(real) == 4 && S.max_relax == 1) launch_tma_k<real, TX, TY, CPT, 1, ZU>(S, a, maps, koff, st);
     else if (sizeof(real) == 4 && S.max_relax == 2) launch_tma_k<real, TX, TY, CPT, 2, ZU>(S, a, maps, koff, st);
+    else if (sizeof(real) == 8 && !S.has_cmap) launch_tma_k<real, TX, TY, CPT, -1, ZU, FL_NOC>(S, a, maps, koff, st);
     else launch_tma_k<real, TX, TY, CPT, -1, ZU>(S, a, maps, koff, st);
 }
 
@@ -399,9 +400,9 @@ static void launch_pair(WvSession& S, const WvArgs<real>& a, int64_t s, int koff
         c.ty = v.ty;
         c.zu = v.zu;
         c.nq = v.nq;
-        c.kind = S.max_relax == 0 ? 0
-                 : S.max_relax == 1 ? ((S.has_cmap && !S.has_matmap && !S.has_planemat) ? 1 : 2)
-                 : S.max_relax == 2 ? 3 : -1;
+        c.kind = S.max_relax == 0 ? (S.has_cmap ? 0 : 4)
+                 : S.max_relax == 1 ? (!S.has_cmap ? 5 : (!S.has_matmap && !S.has_planemat) ? 1 : 2)
+                 : S.max_relax == 2 ? (S.has_cmap ? 3 : 6) : -1;
         c.acc = acc;
         wv_pair_launch(c);
     }
@@ -643,6 +644,9 @@ static void upload_consts(WvSession& S, const bd_medium* m) {
     }
     S.kconst.alloc(S.ctx, sizeof K);
     BD_CUDA(cudaMemcpy(S.kconst.p, &K, sizeof K, cudaMemcpyHostToDevice));
+    const WvArgs<real> a = make_args<real>(S, 0);    // dt, dx, dz and the relaxation scheme
+    wv_derive_kernel<real><<<1, 32, 0, S.ctx->stream>>>(a, S.kconst.as<WvConst<real>>());
+    BD_LAUNCHED(S.ctx);
 }
 
 template <class T>

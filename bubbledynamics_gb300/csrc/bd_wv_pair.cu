@@ -11,8 +11,8 @@ namespace bd {
 
 template <int TX, int TY, int NREL, int ZU, int FL, int NQ, int ACC>
 static void pair_k(const PairCall& c) {
-    using L = TmaLayout<float, TX, TY, (NREL >= 0 ? NREL : BD_MAX_RELAX), NQ>;
-    auto kern = wv_tma_pair_kernel<float, TX, TY, NREL, ZU, FL, NQ, ACC>;
+    using L = TmaLayout<float, TX, TY, NREL, NQ>;
+    auto kern = wv_tma_pair_kernel<TX, TY, NREL, ZU, FL, NQ, ACC>;
     static bool attr_done = false;
     static int per_sm = 0;
     if (!attr_done) {
@@ -49,7 +49,7 @@ static void pair_k(const PairCall& c) {
 }
 
 // material layout: 0 = no relaxation, 1 = one process, one material and a c
-// map (compile-time), 2 = one process, 3 = two processes
+// map (compile-time), 2 = one process, 3 = two processes; 4-6 = 0, 2, 3 without a c map
 template <int TX, int TY, int ZU, int NQ, int ACC>
 static void pair_kind_acc(const PairCall& c) {
     switch (c.kind) {
@@ -57,6 +57,9 @@ static void pair_kind_acc(const PairCall& c) {
         case 1: pair_k<TX, TY, 1, ZU, 3, NQ, ACC>(c); break;
         case 2: pair_k<TX, TY, 1, ZU, -1, NQ, ACC>(c); break;
         case 3: pair_k<TX, TY, 2, ZU, -1, NQ, ACC>(c); break;
+        case 4: pair_k<TX, TY, 0, ZU, FL_NOC, NQ, ACC>(c); break;
+        case 5: pair_k<TX, TY, 1, ZU, FL_NOC, NQ, ACC>(c); break;
+        case 6: pair_k<TX, TY, 2, ZU, FL_NOC, NQ, ACC>(c); break;
         default: fail(BD_ERR_INVALID_ARG, "two-cell tile variants take at most two relaxation processes");
     }
 }

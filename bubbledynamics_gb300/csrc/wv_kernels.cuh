@@ -27,6 +27,12 @@ struct MatConst {
     real rb[BD_MAX_RELAX];     // tau_v / (2dt + 3 tau_v)                 (W:227)
     int n_relax;
     int pad;
+    // what cell_update() forms from c, for c = c0 (wv_derive_kernel fills these on the
+    // device with the operations of cell_coef(), so a cell without a c map reads the
+    // bits it would compute)
+    real kxy, kz, kd, kn, kr;  // stencil xy and z, diffusivity, nonlinearity, (c dt)^2
+    real xr;                   // x / (1 - x), x = 3 kr sum a (semi-implicit relaxation)
+    real av[BD_MAX_RELAX];     // a_v
 };
 
 template <class real>
@@ -204,14 +210,56 @@ __device__ __forceinline__ real d2x180(real pc, real s1, real s2, real s3) {
     return fma_(real(2), s3, fma_(real(-27), s2, fma_(real(270), s1, mul_(real(-490), pc))));
 }
 
+// Coefficients of the cell update at sound speed c, into M's derived fields.
+template <class real, int NRMAX>
+__device__ __forceinline__ void cell_coef(const WvArgs<real>& a, MatConst<real>& M, real c) {
+    const real c2 = mul_(c, c);
+    const real ic = div_(real(1), c);
+    const real ic2 = mul_(ic, ic);
+    M.kxy = mul_(c2, a.kxy180);
+    M.kz = mul_(c2, a.kz180);
+    M.kd = mul_(M.delta_2dt, ic2);
+    M.kn = mul_(M.beta2_rho, ic2);
+    M.kr = mul_(c2, a.dt2);
+    if (a.relax_scheme == BD_RELAX_SEMI_IMPLICIT) {
+        const real ic3 = mul_(ic2, ic);
+        real sa = real(0);
+#pragma unroll
+        for (int v = 0; v < NRMAX; ++v)
+            if (v < M.n_relax) {
+                M.av[v] = mul_(M.ra_num[v], ic3);
+                sa = add_(sa, M.av[v]);
+            }
+        // p = num / (1 - x) with x = 3 kr sum a small: written as num + num x / (1 - x) so
+        // the (possibly approximate) division only touches the small correction
+        const real x = mul_(mul_(real(3), M.kr), sa);
+        M.xr = div_(x, add_(real(1), -x));
+    } else {
+#pragma unroll
+        for (int v = 0; v < NRMAX; ++v)
+            if (v < M.n_relax) M.av[v] = mul_(mul_(M.ra_num[v], ic2), ic);
+    }
+}
+
+template <class real>
+__global__ void wv_derive_kernel(const WvArgs<real> a, WvConst<real>* K) {
+    const int m = threadIdx.x;
+    if (m < BD_MAX_MATERIALS && K->mat[m].c0 > real(0)) {
+        MatConst<real> M = K->mat[m];
+        cell_coef<real, BD_MAX_RELAX>(a, M, M.c0);
+        K->mat[m] = M;
+    }
+}
+
 // The update of one cell (W:203-234, or the semi-implicit relaxation coupling).
 // sx1..sy3: sums of the +-1, +-2, +-3 neighbours along x / y; w[0..6]: p^n at
-// iz-3..iz+3; q1..q4: p^{n-1..n-4}; rc / ro: R^{n-1} / R^{n-2} per process, ro
-// returns R^n.  Returns p^{n+1} before the sponge factor.
+// iz-3..iz+3 (or iz+3..iz-3); q1..q4: p^{n-1..n-4}; rc / ro: R^{n-1} / R^{n-2} per
+// process, ro returns R^n; M: material with the derived coefficients of the cell's
+// sound speed.  Returns p^{n+1} before the sponge factor.
 template <class real, int NRMAX = BD_MAX_RELAX>
-__device__ __forceinline__ real cell_update(const WvArgs<real>& a, const MatConst<real>& M, real c, real pc, real sx1,
-                                            real sx2, real sx3, real sy1, real sy2, real sy3, const real* w, real q1,
-                                            real q2, real q3, real q4, const real* rc, real* ro) {
+__device__ __forceinline__ real cell_update(const WvArgs<real>& a, const MatConst<real>& M, real pc, real sx1, real sx2,
+                                            real sx3, real sy1, real sy2, real sy3, const real* w, real q1, real q2,
+                                            real q3, real q4, const real* rc, real* ro) {
     const real Dxx = d2x180(pc, sx1, sx2, sx3);
     const real Dyy = d2x180(pc, sy1, sy2, sy3);
     const real Dzz = d2x180(pc, add_(w[4], w[2]), add_(w[5], w[1]), add_(w[6], w[0]));
@@ -220,13 +268,6 @@ __device__ __forceinline__ real cell_update(const WvArgs<real>& a, const MatCons
     const real s3 = fma_(real(3), pc, fma_(real(-4), q1, q2));
     const real D1 = mul_(mul_(s3, s3), real(0.25));                                                   // W:208
     const real D2 = mul_(pc, fma_(real(2), pc, fma_(real(-5), q1, fma_(real(4), q2, -q3))));          // W:209
-    const real c2 = mul_(c, c);
-    const real ic = div_(real(1), c);
-    const real ic2 = mul_(ic, ic);
-    const real kxy = mul_(c2, a.kxy180);
-    const real kz = mul_(c2, a.kz180);
-    const real kd = mul_(M.delta_2dt, ic2);
-    const real kn = mul_(M.beta2_rho, ic2);
     // W:234 without the relaxation term, as an increment on p^n: Y = p + V with
     // V = (p - p1) + kxy (Dxx + Dyy) + kz Dzz + kd Dttt + kn (D1 + D2).  The terms are
     // summed at the size of the increment (about a quarter of p per step at 8
@@ -234,51 +275,52 @@ __device__ __forceinline__ real cell_update(const WvArgs<real>& a, const MatCons
     // error against FP64 after 3000 cfg1 steps drops from 1.04e-5 to 8.4e-6
     // (summing 2p - p1 + ... directly rounds at the size of p five times).
     real V = add_(pc, -q1);
-    V = fma_(kxy, add_(Dxx, Dyy), V);
-    V = fma_(kz, Dzz, V);
-    V = fma_(kd, Dttt, V);
-    V = fma_(kn, add_(D1, D2), V);
+    V = fma_(M.kxy, add_(Dxx, Dyy), V);
+    V = fma_(M.kz, Dzz, V);
+    V = fma_(M.kd, Dttt, V);
+    V = fma_(M.kn, add_(D1, D2), V);
     real pn;
     if (M.n_relax > 0 && a.relax_scheme == BD_RELAX_SEMI_IMPLICIT) {
         // R_v = a_v (3 p^{n+1} + E) + b_v (4 R1 - R2) with the 2nd-order d3p/dt3 at t_n
         // through p^{n+1}..p^{n-3}; p^{n+1} = Y + (c dt)^2 sum_v R_v solved per cell
         const real E = fma_(real(-10), pc, fma_(real(12), q1, fma_(real(-6), q2, q3)));
-        const real kr = mul_(c2, a.dt2);
-        const real ic3 = mul_(ic2, ic);
-        real sa = real(0), G = real(0);
-        real av[NRMAX > 0 ? NRMAX : 1], bv[NRMAX > 0 ? NRMAX : 1];
+        real G = real(0);
+        real bv[NRMAX > 0 ? NRMAX : 1];
 #pragma unroll
         for (int v = 0; v < NRMAX; ++v) {
             if (v < M.n_relax) {
-                av[v] = mul_(M.ra_num[v], ic3);
                 bv[v] = mul_(M.rb[v], fma_(real(4), rc[v], -ro[v]));
-                sa = add_(sa, av[v]);
-                G = add_(G, fma_(av[v], E, bv[v]));
+                G = add_(G, fma_(M.av[v], E, bv[v]));
             }
         }
-        // p = num / (1 - x) with x = 3 kr sum a small: written as num + num x / (1 - x) so
-        // the (possibly approximate) division only touches the small correction
-        const real x = mul_(mul_(real(3), kr), sa);
-        const real Vn = fma_(kr, G, V);                          // num = p + Vn
-        pn = add_(pc, fma_(add_(pc, Vn), div_(x, add_(real(1), -x)), Vn));
+        const real Vn = fma_(M.kr, G, V);                        // num = p + Vn
+        pn = add_(pc, fma_(add_(pc, Vn), M.xr, Vn));
 #pragma unroll
         for (int v = 0; v < NRMAX; ++v)
-            if (v < M.n_relax) ro[v] = fma_(av[v], fma_(real(3), pn, E), bv[v]);
+            if (v < M.n_relax) ro[v] = fma_(M.av[v], fma_(real(3), pn, E), bv[v]);
     } else {
         real sumR = real(0);
 #pragma unroll
         for (int v = 0; v < NRMAX; ++v) {
             if (v < M.n_relax) {
                 // W:227: R = 2dt 2 c_v tau Dttt/(2dt^3) / ((2dt+3tau) c^3) + tau (4 R1 - R2)/(2dt+3tau)
-                const real rn = fma_(mul_(mul_(M.ra_num[v], ic2), ic), Dttt,
-                                     mul_(M.rb[v], fma_(real(4), rc[v], -ro[v])));
+                const real rn = fma_(M.av[v], Dttt, mul_(M.rb[v], fma_(real(4), rc[v], -ro[v])));
                 ro[v] = rn;
                 sumR = add_(sumR, rn);
             }
         }
-        pn = add_(pc, fma_(sumR, mul_(c2, a.dt2), V));                                       // W:234
+        pn = add_(pc, fma_(sumR, M.kr, V));                                                      // W:234
     }
     return pn;
+}
+
+// The same at sound speed c (a grid with a c map).
+template <class real, int NRMAX = BD_MAX_RELAX>
+__device__ __forceinline__ real cell_update_c(const WvArgs<real>& a, MatConst<real> M, real c, real pc, real sx1, real sx2,
+                                              real sx3, real sy1, real sy2, real sy3, const real* w, real q1, real q2,
+                                              real q3, real q4, const real* rc, real* ro) {
+    cell_coef<real, NRMAX>(a, M, c);
+    return cell_update<real, NRMAX>(a, M, pc, sx1, sx2, sx3, sy1, sy2, sy3, w, q1, q2, q3, q4, rc, ro);
 }
 
 // One time step of the stencil update.  CTA = TX x TY columns; each thread
@@ -345,10 +387,10 @@ __global__ void __launch_bounds__(TX* TY) wv_step_kernel(const WvArgs<real> a, c
             const real sy3 = yw[5] * ld(P + yo[5]) + yw[0] * ld(P + yo[0]);
             const real q1 = ld(a.p1 + i), q2 = ld(a.p2 + i), q3 = ld(a.p3 + i), q4 = a.p4[i];
             const int m = cell_mat(a, i, iz);
-            const real c = cell_c(a, K, i, m);
             real rc[BD_MAX_RELAX], ro[BD_MAX_RELAX];
             for (int v = 0; v < K.mat[m].n_relax; ++v) { rc[v] = ld(a.rcur[v] + i); ro[v] = a.rold[v][i]; }
-            pn = cell_update(a, K.mat[m], c, pc, sx1, sx2, sx3, sy1, sy2, sy3, w, q1, q2, q3, q4, rc, ro);
+            if (a.cmap) pn = cell_update_c(a, K.mat[m], cell_c(a, K, i, m), pc, sx1, sx2, sx3, sy1, sy2, sy3, w, q1, q2, q3, q4, rc, ro);
+            else pn = cell_update(a, K.mat[m], pc, sx1, sx2, sx3, sy1, sy2, sy3, w, q1, q2, q3, q4, rc, ro);
             for (int v = 0; v < K.mat[m].n_relax; ++v) a.rold[v][i] = ro[v];
             if (a.wz) pn = mul_(pn, mul_(sw_xy, a.wz[iz]));
             have = true;

@@ -28,6 +28,7 @@ constexpr int TMA_NP = 8;   // p^n plane slots (>= 7)
 // none, the peak map only, peak and energy without the DFT
 constexpr int ACC_ALL = 0, ACC_NONE = 1, ACC_PEAK = 2, ACC_PE = 3;
 constexpr int TMA_NQ = 3;   // pointwise slots
+constexpr int FL_NOC = 4;   // kernel flags: no c map, materials by plane or cell
 
 struct TmaMaps {
     CUtensorMap p0;                     // box (TX+8, TY+6, 1) on the p^n buffer
@@ -148,8 +149,8 @@ __global__ void __launch_bounds__(TX* TY / CPT) wv_tma_kernel(const WvArgs<real>
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ MatConst<real> sK[BD_MAX_MATERIALS];
     const int nrel = NREL >= 0 ? NREL : a.max_relax;
-    // FL >= 0: bit 0 = one material everywhere, bit 1 = per-cell c map (compile-time);
-    // FL = -1: both read from the arguments
+    // FL >= 0: bit 0 = one material everywhere, bit 1 = per-cell c map (compile-time),
+    // FL_NOC = no c map, materials read from the arguments; FL = -1: both read from them
     const bool has_c = FL >= 0 ? (FL & 2) != 0 : a.cmap != nullptr;
     real* Pring = reinterpret_cast<real*>(smem);
     unsigned char* Qring = smem + TMA_NP * L::PSLOT;
@@ -250,7 +251,7 @@ __global__ void __launch_bounds__(TX* TY / CPT) wv_tma_kernel(const WvArgs<real>
     const bool do_energy = step >= a.energy_start && step < a.energy_end;
     const long long ds = step - a.dft_start;
     const bool do_dft = a.n_dft > 0 && ds >= 0 && ds < a.dft_len;
-    const bool single_mat = FL >= 0 ? (FL & 1) != 0 : (!a.matmap && !a.plane_mat);
+    const bool single_mat = FL >= 0 && FL != FL_NOC ? (FL & 1) != 0 : (!a.matmap && !a.plane_mat);
     const bool dpdt = a.energy_mode == BD_ENERGY_DPDT2;
     // the material of single-material problems, in registers
     const MatConst<real> M0 = sK[0];
@@ -327,7 +328,6 @@ __global__ void __launch_bounds__(TX* TY / CPT) wv_tma_kernel(const WvArgs<real>
                 constexpr int W = L::PW;
                 const real sy1 = c0[W] + c0[-W], sy2 = c0[2 * W] + c0[-2 * W], sy3 = c0[3 * W] + c0[-3 * W];
                 auto upd = [&](const MatConst<real>& M) -> real {
-                    const real cs = has_c ? (real)ct[k] : M.c0;
                     real rc[NRMAX > 0 ? NRMAX : 1], ro[NRMAX > 0 ? NRMAX : 1];
 #pragma unroll
                     for (int v = 0; v < NRMAX; ++v) {
@@ -336,8 +336,10 @@ __global__ void __launch_bounds__(TX* TY / CPT) wv_tma_kernel(const WvArgs<real>
                             ro[v] = reinterpret_cast<const real*>(Qs + (4 + NRMAX + v) * L::QTB)[k];
                         }
                     }
-                    const real r = cell_update<real, NRMAX>(a, M, cs, pc, sx1, sx2, sx3, sy1, sy2, sy3, w[c], q1, q2t[k],
-                                                            q3t[k], q4t[k], rc, ro);
+                    const real r = has_c ? cell_update_c<real, NRMAX>(a, M, (real)ct[k], pc, sx1, sx2, sx3, sy1, sy2, sy3,
+                                                                      w[c], q1, q2t[k], q3t[k], q4t[k], rc, ro)
+                                         : cell_update<real, NRMAX>(a, M, pc, sx1, sx2, sx3, sy1, sy2, sy3, w[c], q1,
+                                                                    q2t[k], q3t[k], q4t[k], rc, ro);
 #pragma unroll
                     for (int v = 0; v < NRMAX; ++v)
                         if (v < M.n_relax) rolz[v][col[c]] = ro[v];

@@ -7,30 +7,154 @@
 
 namespace bd {
 
-// CX consecutive values along x (CX = 1 or 2): one 8- or 16-byte access for a
-// pair, whose first element sits at an even index of a buffer aligned to the
-// pair's size.
-template <class real> struct Pair;
-template <> struct Pair<float> { using T = float2; };
-template <> struct Pair<double> { using T = double2; };
+// The two cells of a thread as one 64-bit value: sm_103a's packed FP32 add, multiply
+// and fma round each half like the scalar instruction and take one issue slot.
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float a, float b) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ F2 f2(float a) { return f2(a, a); }
+__device__ __forceinline__ void f2_split(F2 a, float& x, float& y) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+// ptxas fuses a packed product into the packed add that takes it, although both
+// are .rn: a product that goes into an add is formed by f2_mul1.
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+// the product as two scalar multiplications
+__device__ __forceinline__ F2 f2_mul1(F2 a, F2 b) {
+    float a0, a1, b0, b1;
+    f2_split(a, a0, a1);
+    f2_split(b, b0, b1);
+    return f2(mul_(a0, b0), mul_(a1, b1));
+}
+// a - b in one rounding (b (-1) + a)
+__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) { return f2_fma(b, f2(-1.0f), a); }
+__device__ __forceinline__ F2 ld2(const float* p) {
+    F2 r;
+    r.v = *reinterpret_cast<const unsigned long long*>(p);
+    return r;
+}
+__device__ __forceinline__ void st2(float* p, F2 a) { *reinterpret_cast<unsigned long long*>(p) = a.v; }
 
-template <int CX, class real>
-__device__ __forceinline__ void ldx(const real* p, real* out) {
-    if constexpr (CX == 2) {
-        const typename Pair<real>::T v = *reinterpret_cast<const typename Pair<real>::T*>(p);
-        out[0] = v.x;
-        out[1] = v.y;
-    } else {
-        out[0] = *p;
-    }
+// cell_coef()'s coefficients of two cells
+template <int NR>
+struct Coef2 {
+    F2 kxy, kz, kd, kn, kr, xr, av[NR > 0 ? NR : 1], rb[NR > 0 ? NR : 1];
+};
+
+// of the cells' materials (the same one twice: one set of loads)
+template <int NR>
+__device__ __forceinline__ Coef2<NR> coef2(const MatConst<float>& A, const MatConst<float>& B) {
+    Coef2<NR> c;
+    c.kxy = f2(A.kxy, B.kxy); c.kz = f2(A.kz, B.kz); c.kd = f2(A.kd, B.kd);
+    c.kn = f2(A.kn, B.kn); c.kr = f2(A.kr, B.kr); c.xr = f2(A.xr, B.xr);
+#pragma unroll
+    for (int v = 0; v < NR; ++v) { c.av[v] = f2(A.av[v], B.av[v]); c.rb[v] = f2(A.rb[v], B.rb[v]); }
+    return c;
 }
 
-template <class real>
-__device__ __forceinline__ void st2(real* p, real v0, real v1) {
-    typename Pair<real>::T v;
-    v.x = v0;
-    v.y = v1;
-    *reinterpret_cast<typename Pair<real>::T*>(p) = v;
+// at the sound speeds c of the two cells; a process that a cell's material does not
+// have gets zero coefficients, which leave the cell's value as it is without it
+template <int NR>
+__device__ __forceinline__ Coef2<NR> coef2_c(const WvArgs<float>& a, const MatConst<float>& A, const MatConst<float>& B, F2 c) {
+    Coef2<NR> k;
+    float cx, cy;
+    f2_split(c, cx, cy);
+    const F2 c2 = f2_mul(c, c), ic = f2(div_(1.0f, cx), div_(1.0f, cy)), ic2 = f2_mul(ic, ic);
+    k.kxy = f2_mul(c2, f2(a.kxy180));
+    k.kz = f2_mul(c2, f2(a.kz180));
+    k.kd = f2_mul(f2(A.delta_2dt, B.delta_2dt), ic2);
+    k.kn = f2_mul(f2(A.beta2_rho, B.beta2_rho), ic2);
+    k.kr = f2_mul(c2, f2(a.dt2));
+    k.xr = f2(0.0f);
+    if (NR > 0) {
+        if (a.relax_scheme == BD_RELAX_SEMI_IMPLICIT) {
+            const F2 ic3 = f2_mul(ic2, ic);
+            F2 sa = f2(0.0f);
+#pragma unroll
+            for (int v = 0; v < NR; ++v) {
+                k.av[v] = f2_mul(f2(A.ra_num[v], B.ra_num[v]), ic3);
+                sa = f2_add(sa, k.av[v]);
+            }
+            const F2 x = f2_mul(f2_mul(f2(3.0f), k.kr), sa), d = f2_sub(f2(1.0f), x);
+            float x0, x1, d0, d1;
+            f2_split(x, x0, x1);
+            f2_split(d, d0, d1);
+            k.xr = f2(div_(x0, d0), div_(x1, d1));
+        } else {
+#pragma unroll
+            for (int v = 0; v < NR; ++v) k.av[v] = f2_mul(f2_mul(f2(A.ra_num[v], B.ra_num[v]), ic2), ic);
+        }
+#pragma unroll
+        for (int v = 0; v < NR; ++v) k.rb[v] = f2(A.rb[v], B.rb[v]);
+    }
+    return k;
+}
+
+__device__ __forceinline__ F2 d2x180(F2 pc, F2 s1, F2 s2, F2 s3) {
+    return f2_fma(f2(2.0f), s3, f2_fma(f2(-27.0f), s2, f2_fma(f2(270.0f), s1, f2_mul(f2(-490.0f), pc))));
+}
+
+// cell_update() of two cells: the same operations, so the same bits.  relax: either
+// cell's material has relaxation processes.
+template <int NR>
+__device__ __forceinline__ F2 cell_update2(const WvArgs<float>& a, const Coef2<NR>& k, bool relax, F2 sx1, F2 sx2, F2 sx3,
+                                           F2 sy1, F2 sy2, F2 sy3, const F2* w, F2 q1, F2 q2, F2 q3, F2 q4, const F2* rc,
+                                           F2* ro) {
+    const F2 pc = w[3];
+    const F2 Dxx = d2x180(pc, sx1, sx2, sx3);
+    const F2 Dyy = d2x180(pc, sy1, sy2, sy3);
+    const F2 Dzz = d2x180(pc, f2_add(w[4], w[2]), f2_add(w[5], w[1]), f2_add(w[6], w[0]));
+    const F2 Dttt = f2_fma(f2(3.0f), q4, f2_fma(f2(-14.0f), q3, f2_fma(f2(24.0f), q2, f2_fma(f2(-18.0f), q1, f2_mul(f2(5.0f), pc)))));
+    const F2 s3 = f2_fma(f2(3.0f), pc, f2_fma(f2(-4.0f), q1, q2));
+    const F2 D1 = f2_mul1(f2_mul(s3, s3), f2(0.25f));
+    // 4 p2 is exact, so 4 p2 - p3 takes the one rounding of the fma
+    const F2 D2 = f2_mul1(pc, f2_fma(f2(2.0f), pc, f2_fma(f2(-5.0f), q1, f2_sub(f2_mul(f2(4.0f), q2), q3))));
+    F2 V = f2_sub(pc, q1);
+    V = f2_fma(k.kxy, f2_add(Dxx, Dyy), V);
+    V = f2_fma(k.kz, Dzz, V);
+    V = f2_fma(k.kd, Dttt, V);
+    V = f2_fma(k.kn, f2_add(D1, D2), V);
+    if (NR == 0 || !relax) return f2_add(pc, V);
+    if (a.relax_scheme == BD_RELAX_SEMI_IMPLICIT) {
+        const F2 E = f2_fma(f2(-10.0f), pc, f2_fma(f2(12.0f), q1, f2_fma(f2(-6.0f), q2, q3)));
+        F2 G = f2(0.0f), bv[NR > 0 ? NR : 1];
+#pragma unroll
+        for (int v = 0; v < NR; ++v) {
+            bv[v] = f2_mul(k.rb[v], f2_sub(f2_mul(f2(4.0f), rc[v]), ro[v]));
+            G = f2_add(G, f2_fma(k.av[v], E, bv[v]));
+        }
+        const F2 Vn = f2_fma(k.kr, G, V);
+        const F2 pn = f2_add(pc, f2_fma(f2_add(pc, Vn), k.xr, Vn));
+#pragma unroll
+        for (int v = 0; v < NR; ++v) ro[v] = f2_fma(k.av[v], f2_fma(f2(3.0f), pn, E), bv[v]);
+        return pn;
+    }
+    F2 sumR = f2(0.0f);
+#pragma unroll
+    for (int v = 0; v < NR; ++v) {
+        ro[v] = f2_fma(k.av[v], Dttt, f2_mul(k.rb[v], f2_sub(f2_mul(f2(4.0f), rc[v]), ro[v])));
+        sumR = f2_add(sumR, ro[v]);
+    }
+    return f2_add(pc, f2_fma(sumR, k.kr, V));
 }
 
 // One Westervelt step, TMA-pipelined, two adjacent x cells per thread: the
@@ -51,24 +175,23 @@ __device__ __forceinline__ void st2(real* p, real v0, real v1) {
 // every cell of the tile is updated take a copy of the cell code without the
 // per-cell conditions, except in ACC_ALL, where the larger DFT code of that
 // copy would cost registers (and spills) in the whole kernel.
-template <class real, int TX, int TY, int NREL, int ZU, int FL, int NQ, int ACC = ACC_ALL>
-__global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kernel(const WvArgs<real> a,
-                                                                 const WvConst<real>* __restrict__ Kp, int koff,
+template <int TX, int TY, int NREL, int ZU, int FL, int NQ, int ACC = ACC_ALL>
+__global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kernel(const WvArgs<float> a,
+                                                                 const WvConst<float>* __restrict__ Kp, int koff,
                                                                  const __grid_constant__ TmaMaps maps,
                                                                  unsigned* __restrict__ err) {
-    constexpr int CX = 2, CPT = 1;
+    using real = float;
+    constexpr int CX = 2;
+    static_assert(NREL >= 0 && NREL <= 2, "compiled for the relaxation count");
     static_assert(NQ >= ZU, "the pointwise ring holds a whole group of planes");
-    constexpr int NRMAX = NREL >= 0 ? NREL : BD_MAX_RELAX;
+    constexpr int NRMAX = NREL, nrel = NREL;
     using L = TmaLayout<real, TX, TY, NRMAX, NQ>;
     constexpr int TXT = TX / CX;                   // thread columns
-    constexpr int RPT = TY / CPT;                  // thread rows
-    constexpr int NT = TXT * RPT;                  // threads
-    constexpr int NC = CPT * CX;                   // cells per thread
+    constexpr int NT = TXT * TY;                   // threads
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ MatConst<real> sK[BD_MAX_MATERIALS];
-    const int nrel = NREL >= 0 ? NREL : a.max_relax;
     // FL >= 0: bit 0 = one material everywhere, bit 1 = per-cell c map (compile-time);
-    // FL = -1: both read from the arguments
+    // FL_NOC = no c map, materials read from the arguments; FL = -1: both read from them
     const bool has_c = FL >= 0 ? (FL & 2) != 0 : a.cmap != nullptr;
     real* Pring = reinterpret_cast<real*>(smem);
     unsigned char* Qring = smem + TMA_NP * L::PSLOT;
@@ -157,50 +280,32 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
     auto waitP = [&](int q) { mbar_wait(&barP[q % TMA_NP], (unsigned)((q / TMA_NP) & 1), err); };
     auto waitQ = [&](int r) { mbar_wait(&barQ[r % NQ], (unsigned)((r / NQ) & 1), err); };
 
-    // per-cell constants of this thread's cells: c = cy * CX + cx is the cell in
-    // row tyt + cy * RPT and column CX * tx + cx of the tile
-    int own[NC], qi[NC];
-    bool active[NC], inbox[NC], murxy[NC];
-    real swxy[NC];
-    int col[NC];                                   // column index iy * px + ix (a plane has < 2^31 cells)
+    // this thread's two cells: row tyt, columns CX * tx and CX * tx + 1 of the tile
+    const int ix = x0 + CX * tx, iy = y0 + tyt;
+    const int own = (tyt + 3) * L::PW + CX * tx + 4, k = tyt * TX + CX * tx;
+    const int col = iy * a.px + ix;                // column index iy * px + ix (a plane has < 2^31 cells)
+    bool active[CX], inbox[CX], murxy[CX];
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-        const int ty = tyt + (c / CX) * RPT;
-        const int lx = CX * tx + c % CX;
-        const int ix = x0 + lx, iy = y0 + ty;
-        own[c] = (ty + 3) * L::PW + lx + 4;
-        qi[c] = ty * TX + lx;
-        active[c] = ix < a.nx && iy < a.ny;
-        inbox[c] = ix <= a.xhi && iy <= a.yhi;
-        murxy[c] = (a.mur_yp && iy >= a.ny - a.L) || (a.mur_xp && ix >= a.nx - a.L);
-        swxy[c] = (a.wx && active[c]) ? mul_(a.wx[ix], a.wy[iy]) : real(1);
-        col[c] = iy * a.px + ix;
+    for (int c = 0; c < CX; ++c) {
+        active[c] = ix + c < a.nx && iy < a.ny;
+        inbox[c] = ix + c <= a.xhi && iy <= a.yhi;
+        murxy[c] = (a.mur_yp && iy >= a.ny - a.L) || (a.mur_xp && ix + c >= a.nx - a.L);
     }
-    real w[NC][7];
-    // p^n of this thread's cells on one plane tile into w[.][k]
-    auto load_w = [&](const real* tile, bool in, int k) {
-#pragma unroll
-        for (int cy = 0; cy < CPT; ++cy) {
-            real v[CX];
-            ldx<CX>(tile + own[cy * CX], v);
-#pragma unroll
-            for (int cx = 0; cx < CX; ++cx) w[cy * CX + cx][k] = in ? v[cx] : real(0);
-        }
-    };
+    const F2 swxy = f2(a.wx && active[0] ? mul_(a.wx[ix], a.wy[iy]) : 1.0f, a.wx && active[1] ? mul_(a.wx[ix + 1], a.wy[iy]) : 1.0f);
+    F2 w[7];                                       // p^n of the two cells, by plane of the march
+    auto load_w = [&](const real* tile, bool in) -> F2 { return in ? ld2(tile + own) : f2(0.0f); };
 #pragma unroll
     for (int k = 0; k < 6; ++k) {                  // the first plane and three on either side, but the last
         waitP(k);
         const int plane = zof(k - 3);
-        load_w(pslot(k), plane >= 0 && plane < a.nz, k);
+        w[k] = load_w(pslot(k), plane >= 0 && plane < a.nz);
     }
     // every cell of the tile inside the grid and the update box and on no x / y
     // Mur layer: the planes of the tile inside the z range take the code without
     // per-cell conditions (the same operations on every cell, so the same bits)
     bool tile_fast = false;
     if constexpr (ACC != ACC_ALL) {
-        bool mine = true;
-#pragma unroll
-        for (int c = 0; c < NC; ++c) mine = mine && active[c] && inbox[c] && !murxy[c];
+        const bool mine = active[0] && active[1] && inbox[0] && inbox[1] && !murxy[0] && !murxy[1];
         tile_fast = __syncthreads_and(mine) != 0;      // also: the slots of the three planes before the first are free again
     } else {
         __syncthreads();                               // the slots of the three planes before the first are free again
@@ -213,10 +318,8 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
     const bool do_energy = (ACC == ACC_ALL || ACC == ACC_PE) && step >= a.energy_start && step < a.energy_end;
     const long long ds = step - a.dft_start;
     const bool do_dft = ACC == ACC_ALL && a.n_dft > 0 && ds >= 0 && ds < a.dft_len;
-    const bool single_mat = FL >= 0 ? (FL & 1) != 0 : (!a.matmap && !a.plane_mat);
+    const bool single_mat = FL >= 0 && FL != FL_NOC ? (FL & 1) != 0 : (!a.matmap && !a.plane_mat);
     const bool dpdt = a.energy_mode == BD_ENERGY_DPDT2;
-    // the material of single-material problems, in registers
-    const MatConst<real> M0 = sK[0];
 
     for (int rg = 0; rg < zbn; rg += ZU) {
         // the last planes of this CTA: the next step's grid may start its prologue
@@ -228,7 +331,7 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
         const int iz = zof(r);
         const int qc = r + 3;                      // stencil plane
         waitP(qc + 3);
-        load_w(pslot(qc + 3), (unsigned)zof(r + 3) < (unsigned)a.nz, 6);
+        w[6] = load_w(pslot(qc + 3), (unsigned)zof(r + 3) < (unsigned)a.nz);
         real* T = pslot(qc);
         if (fix_x || fix_y) {                      // mirror planes x = 0 / y = 0 (W:176-200)
             if (fix_x)
@@ -271,187 +374,141 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
         // FAST: every cell of the tile is updated and accumulates on this plane
         auto cells = [&](auto fast_tag) {
         constexpr bool FAST = decltype(fast_tag)::value;
-#pragma unroll
-        for (int cy = 0; cy < CPT; ++cy) {
-            const int c0 = cy * CX;                // first cell of this row (the CX cells share `active`)
-            if (!FAST && !active[c0]) continue;
-            const int k = qi[c0];
-            real q1[CX], pn[CX];
-            bool have[CX];
-            int nrx[CX];                           // relaxation processes of the cell's material
-            real ro[CX][NRMAX > 0 ? NRMAX : 1];
-            ldx<CX>(q1t + k, q1);
-#pragma unroll
-            for (int cx = 0; cx < CX; ++cx) { have[cx] = false; nrx[cx] = 0; }
+        {
+            if (!FAST && !active[0]) return;       // a thread's first cell is the last to leave the grid
+            const F2 q1p = ld2(q1t + k);
+            F2 pnp, ro[NRMAX > 0 ? NRMAX : 1];
+            bool have[CX] = {FAST, FAST};
+            int nrx[CX] = {0, 0};                  // relaxation processes of the cells' materials
             if (!FAST && src_plane) {
-#pragma unroll
-                for (int cx = 0; cx < CX; ++cx) {
-                    pn[cx] = source_value<real>(a, step, (int)col[c0 + cx]);
-                    have[cx] = true;
-                }
+                pnp = f2(source_value<real>(a, step, col), source_value<real>(a, step, col + 1));
+                have[0] = have[1] = true;
             } else if (FAST || zin) {
-                // x and y neighbours of the CX cells from the plane tile
-                const real* cp = T + own[c0];
+                // x and y neighbours from the plane tile
+                const real* cp = T + own;
                 constexpr int W = L::PW;
-                real sx1[CX], sx2[CX], sx3[CX], sy1[CX], sy2[CX], sy3[CX];
-                if constexpr (CX == 2) {
-                    real xr[10];                   // x offsets -4 .. +5 from the first cell
-#pragma unroll
-                    for (int j = 0; j < 5; ++j) ldx<2>(cp - 4 + 2 * j, xr + 2 * j);
-#pragma unroll
-                    for (int cx = 0; cx < 2; ++cx) {
-                        sx1[cx] = xr[5 + cx] + xr[3 + cx];
-                        sx2[cx] = xr[6 + cx] + xr[2 + cx];
-                        sx3[cx] = xr[7 + cx] + xr[1 + cx];
-                    }
-                    real ya[6][2];
-#pragma unroll
-                    for (int j = 0; j < 3; ++j) {
-                        ldx<2>(cp + (j + 1) * W, ya[2 * j]);
-                        ldx<2>(cp - (j + 1) * W, ya[2 * j + 1]);
-                    }
-#pragma unroll
-                    for (int cx = 0; cx < 2; ++cx) {
-                        sy1[cx] = ya[0][cx] + ya[1][cx];
-                        sy2[cx] = ya[2][cx] + ya[3][cx];
-                        sy3[cx] = ya[4][cx] + ya[5][cx];
-                    }
-                } else {
-                    sx1[0] = cp[1] + cp[-1]; sx2[0] = cp[2] + cp[-2]; sx3[0] = cp[3] + cp[-3];
-                    sy1[0] = cp[W] + cp[-W]; sy2[0] = cp[2 * W] + cp[-2 * W]; sy3[0] = cp[3 * W] + cp[-3 * W];
-                }
-                real q2[CX], q3[CX], q4[CX], cs[CX];
-                ldx<CX>(q2t + k, q2);
-                ldx<CX>(q3t + k, q3);
-                ldx<CX>(q4t + k, q4);
-                if (has_c) {
-                    float cf[CX];
-                    ldx<CX>(ct + k, cf);
-#pragma unroll
-                    for (int cx = 0; cx < CX; ++cx) cs[cx] = (real)cf[cx];
-                }
-                real rc[CX][NRMAX > 0 ? NRMAX : 1];
+                float e[10];                       // x offsets -4 .. +5 from the first cell
+                const F2 xm = ld2(cp - 2), xp = ld2(cp + 2);
+                f2_split(ld2(cp - 4), e[0], e[1]);
+                f2_split(xm, e[2], e[3]);
+                f2_split(w[3], e[4], e[5]);
+                f2_split(xp, e[6], e[7]);
+                f2_split(ld2(cp + 4), e[8], e[9]);
+                const F2 sx1 = f2(add_(e[5], e[3]), add_(e[6], e[4])), sx2 = f2_add(xp, xm),
+                         sx3 = f2(add_(e[7], e[1]), add_(e[8], e[2]));
+                const F2 sy1 = f2_add(ld2(cp + W), ld2(cp - W)), sy2 = f2_add(ld2(cp + 2 * W), ld2(cp - 2 * W)),
+                         sy3 = f2_add(ld2(cp + 3 * W), ld2(cp - 3 * W));
+                const F2 q2 = ld2(q2t + k), q3 = ld2(q3t + k), q4 = ld2(q4t + k);
+                F2 rc[NRMAX > 0 ? NRMAX : 1];
 #pragma unroll
                 for (int v = 0; v < NRMAX; ++v) {
-                    if (v < nrel) {
-                        real t[CX], u[CX];
-                        ldx<CX>(reinterpret_cast<const real*>(Qs + (4 + v) * L::QTB) + k, t);
-                        ldx<CX>(reinterpret_cast<const real*>(Qs + (4 + NRMAX + v) * L::QTB) + k, u);
-#pragma unroll
-                        for (int cx = 0; cx < CX; ++cx) { rc[cx][v] = t[cx]; ro[cx][v] = u[cx]; }
+                    rc[v] = ld2(reinterpret_cast<const real*>(Qs + (4 + v) * L::QTB) + k);
+                    ro[v] = ld2(reinterpret_cast<const real*>(Qs + (4 + NRMAX + v) * L::QTB) + k);
+                }
+                int m0 = 0, m1 = 0;
+                if constexpr (!(FL >= 0 && (FL & 1))) {
+                    m0 = m1 = mplane;
+                    if (a.matmap) {
+                        m0 = a.mat_tile ? (int)mtl[k] : (int)__ldg(a.matmap + zoff + col);
+                        m1 = a.mat_tile ? (int)mtl[k + 1] : active[1] ? (int)__ldg(a.matmap + zoff + col + 1) : m0;
                     }
                 }
-#pragma unroll
-                for (int cx = 0; cx < CX; ++cx) {
-                    const int c = c0 + cx;
-                    if (!FAST && !inbox[c]) continue;
-                    auto upd = [&](const MatConst<real>& M) -> real {
-                        const real r = cell_update<real, NRMAX>(a, M, has_c ? cs[cx] : M.c0, w[c][3], sx1[cx], sx2[cx],
-                                                                sx3[cx], sy1[cx], sy2[cx], sy3[cx], w[c], q1[cx],
-                                                                q2[cx], q3[cx], q4[cx], rc[cx], ro[cx]);
-                        nrx[cx] = M.n_relax;
-                        return r;
-                    };
-                    if constexpr (FL >= 0 && (FL & 1)) {
-                        pn[cx] = upd(M0);
-                    } else {
-                        const int m = !a.matmap ? mplane
-                                      : a.mat_tile ? (int)mtl[k + cx] : (int)__ldg(a.matmap + zoff + col[c]);
-                        pn[cx] = upd(sK[m]);
-                    }
-                    if (a.wz) pn[cx] = mul_(pn[cx], mul_(swxy[c], wzi));
-                    have[cx] = true;
-                }
+                const MatConst<float>&A = sK[m0], &B = sK[m1];
+                const int nr0 = A.n_relax, nr1 = B.n_relax;
+                const Coef2<NRMAX> cf = has_c ? coef2_c<NRMAX>(a, A, B, ld2(ct + k)) : coef2<NRMAX>(A, B);
+                pnp = cell_update2<NRMAX>(a, cf, NRMAX > 0 && (nr0 > 0 || nr1 > 0), sx1, sx2, sx3, sy1, sy2, sy3, w, q1p, q2,
+                                          q3, q4, rc, ro);
+                if (a.wz) pnp = f2_mul(pnp, f2_mul(swxy, f2(wzi)));
+                if (!FAST) { have[0] = inbox[0]; have[1] = inbox[1]; }
+                nrx[0] = have[0] ? nr0 : 0;
+                nrx[1] = have[1] ? nr1 : 0;
             }
+            float pn[CX], q1[CX];
+            f2_split(pnp, pn[0], pn[1]);
+            f2_split(q1p, q1[0], q1[1]);
             // stores: a pair access where both cells take part, else per cell
-            const bool pair = CX == 2 && (FAST || (have[0] && have[CX - 1]));
-            if (pair) st2(p4z + col[c0], pn[0], pn[CX - 1]);
+            if (FAST || (have[0] && have[1])) st2(p4z + col, pnp);
             else
 #pragma unroll
-                for (int cx = 0; cx < CX; ++cx)
-                    if (have[cx]) p4z[col[c0 + cx]] = pn[cx];
+                for (int c = 0; c < CX; ++c)
+                    if (have[c]) p4z[col + c] = pn[c];
             // relaxation variables of the processes of each cell's material (as in cell_update)
 #pragma unroll
             for (int v = 0; v < NRMAX; ++v) {
-                if (CX == 2 && v < nrx[0] && v < nrx[CX - 1]) st2(rolz[v] + col[c0], ro[0][v], ro[CX - 1][v]);
-                else
-#pragma unroll
-                    for (int cx = 0; cx < CX; ++cx)
-                        if (v < nrx[cx]) rolz[v][col[c0 + cx]] = ro[cx][v];
+                if (v < nrx[0] && v < nrx[1]) st2(rolz[v] + col, ro[v]);
+                else if (v < nrx[0] || v < nrx[1]) {
+                    float r0, r1;
+                    f2_split(ro[v], r0, r1);
+                    if (v < nrx[0]) rolz[v][col] = r0;
+                    if (v < nrx[1]) rolz[v][col + 1] = r1;
+                }
             }
             bool acc[CX];
 #pragma unroll
-            for (int cx = 0; cx < CX; ++cx) acc[cx] = FAST || (have[cx] && !(murz || murxy[c0 + cx]));
-            const bool acc_pair = CX == 2 && acc[0] && acc[CX - 1];
+            for (int c = 0; c < CX; ++c) acc[c] = FAST || (have[c] && !(murz || murxy[c]));
+            const bool acc_pair = acc[0] && acc[1];
             if (do_peak) {
-                real pk[CX], pv[CX];
-                ldx<CX>(pkt + k, pk);
+                float pk[CX], pv[CX];
+                f2_split(ld2(pkt + k), pk[0], pk[1]);
 #pragma unroll
-                for (int cx = 0; cx < CX; ++cx) {
-                    const real av = fabs(pn[cx]);
-                    pv[cx] = av > pk[cx] ? av : pk[cx];
+                for (int c = 0; c < CX; ++c) {
+                    const real av = fabs(pn[c]);
+                    pv[c] = av > pk[c] ? av : pk[c];
                 }
-                if (acc_pair) st2(pkz + col[c0], pv[0], pv[CX - 1]);
+                if (acc_pair) st2(pkz + col, f2(pv[0], pv[1]));
                 else
 #pragma unroll
-                    for (int cx = 0; cx < CX; ++cx)
-                        if (acc[cx]) pkz[col[c0 + cx]] = pv[cx];
+                    for (int c = 0; c < CX; ++c)
+                        if (acc[c]) pkz[col + c] = pv[c];
             }
             if (do_energy) {
-                real en[CX], ev[CX];
-                ldx<CX>(ent + k, en);
-#pragma unroll
-                for (int cx = 0; cx < CX; ++cx) {
-                    real e;
-                    if (dpdt) {
-                        const real dp = div_(add_(pn[cx], -q1[cx]), mul_(real(2.0), a.dt));
-                        e = mul_(mul_(dp, dp), a.dt);
-                    } else {
-                        e = mul_(mul_(pn[cx], pn[cx]), a.dt);
-                    }
-                    ev[cx] = add_(en[cx], e);
+                F2 d = pnp;
+                if (dpdt) {
+                    const real h = mul_(real(2.0), a.dt);
+                    d = f2(div_(add_(pn[0], -q1[0]), h), div_(add_(pn[1], -q1[1]), h));
                 }
-                if (acc_pair) st2(enz + col[c0], ev[0], ev[CX - 1]);
-                else
-#pragma unroll
-                    for (int cx = 0; cx < CX; ++cx)
-                        if (acc[cx]) enz[col[c0 + cx]] = ev[cx];
+                const F2 ev = f2_add(ld2(ent + k), f2_mul1(f2_mul(d, d), f2(a.dt)));
+                if (acc_pair) st2(enz + col, ev);
+                else {
+                    float e0, e1;
+                    f2_split(ev, e0, e1);
+                    if (acc[0]) enz[col] = e0;
+                    if (acc[1]) enz[col + 1] = e1;
+                }
             }
             if (do_dft && iz >= a.dz_lo && iz < a.dz_hi && acc_pair) {
                 // both cells accumulate: one pair load and store per accumulator
-                using P2 = typename Pair<real>::T;
-                const long long pl = (long long)(iz - a.dz_lo) * a.plane + col[c0];
+                                const long long pl = (long long)(iz - a.dz_lo) * a.plane + col;
                 const long long stride = (long long)(a.dz_hi - a.dz_lo) * a.plane;
                 const real* tw = a.tw + ds * a.n_dft * 2;
                 real* dr = a.dre + pl;
                 real* di = a.dim + pl;
                 int j = 0;
                 for (; j + 4 <= a.n_dft; j += 4) {
-                    P2 r[4], m[4];
+                    F2 r[4], m[4];
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
-                        r[u] = *reinterpret_cast<const P2*>(dr + (j + u) * stride);
-                        m[u] = *reinterpret_cast<const P2*>(di + (j + u) * stride);
+                        r[u] = ld2(dr + (j + u) * stride);
+                        m[u] = ld2(di + (j + u) * stride);
                     }
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
                         const real tr = tw[2 * (j + u)], ti = tw[2 * (j + u) + 1];
-                        st2(dr + (j + u) * stride, fma_(pn[0], tr, r[u].x), fma_(pn[1], tr, r[u].y));
-                        st2(di + (j + u) * stride, fma_(-pn[0], ti, m[u].x), fma_(-pn[1], ti, m[u].y));
+                        st2(dr + (j + u) * stride, f2_fma(pnp, f2(tr), r[u]));
+                        st2(di + (j + u) * stride, f2_fma(pnp, f2(-ti), m[u]));
                     }
                 }
                 for (; j < a.n_dft; ++j) {
-                    const P2 r = *reinterpret_cast<const P2*>(dr + j * stride);
-                    const P2 m = *reinterpret_cast<const P2*>(di + j * stride);
-                    st2(dr + j * stride, fma_(pn[0], tw[2 * j], r.x), fma_(pn[1], tw[2 * j], r.y));
-                    st2(di + j * stride, fma_(-pn[0], tw[2 * j + 1], m.x), fma_(-pn[1], tw[2 * j + 1], m.y));
+                    const F2 r = ld2(dr + j * stride), m = ld2(di + j * stride);
+                    st2(dr + j * stride, f2_fma(pnp, f2(tw[2 * j]), r));
+                    st2(di + j * stride, f2_fma(pnp, f2(-tw[2 * j + 1]), m));
                 }
             } else if (do_dft && iz >= a.dz_lo && iz < a.dz_hi) {
 #pragma unroll
                 for (int cx = 0; cx < CX; ++cx) {
                     if (!acc[cx]) continue;
                     const real pv = pn[cx];
-                    const long long pl = (long long)(iz - a.dz_lo) * a.plane + col[c0 + cx];
+                    const long long pl = (long long)(iz - a.dz_lo) * a.plane + col + cx;
                     const long long stride = (long long)(a.dz_hi - a.dz_lo) * a.plane;
                     const real* tw = a.tw + ds * a.n_dft * 2;
                     real* dr = a.dre + pl;
@@ -483,9 +540,7 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
             cells(std::false_type{});
         }
 #pragma unroll
-        for (int c = 0; c < NC; ++c)
-#pragma unroll
-            for (int k = 0; k < 6; ++k) w[c][k] = w[c][k + 1];
+        for (int j = 0; j < 6; ++j) w[j] = w[j + 1];
     }
         __syncthreads();                           // everyone is done with this round's planes and their tiles
         if (tid == 0) {
