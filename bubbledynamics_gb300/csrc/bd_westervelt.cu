@@ -366,13 +366,14 @@ static int step_acc_mode(const WvSession& S, int64_t s) {
     return ACC_NONE;
 }
 
+static int acc_rank(int m) { return m == ACC_ALL ? 3 : m == ACC_PE ? 2 : m == ACC_PEAK ? 1 : 0; }
+
 // The mode that serves every step of [s0, s0 + n): all > peak and energy > peak > none.
 static int range_acc_mode(const WvSession& S, int64_t s0, int64_t n) {
-    auto rank = [](int m) { return m == ACC_ALL ? 3 : m == ACC_PE ? 2 : m == ACC_PEAK ? 1 : 0; };
     int m = ACC_NONE;
     for (int64_t s = s0; s < s0 + n; ++s) {
         const int k = step_acc_mode(S, s);
-        if (rank(k) > rank(m)) m = k;
+        if (acc_rank(k) > acc_rank(m)) m = k;
         if (m == ACC_ALL) break;
     }
     return m;
@@ -439,8 +440,9 @@ static void launch_mur(WvSession& S, const WvArgs<real>& a, int koff, cudaStream
 }
 
 template <class real>
-static void launch_step(WvSession& S, int variant, int64_t s, int koff, cudaStream_t st, int acc) {
+static void launch_step(WvSession& S, int variant, int64_t s, int koff, cudaStream_t st, int acc, int acc_n, int mur_acc) {
     WvArgs<real> a = make_args<real>(S, s);
+    a.acc_n = acc_n;
     const Variant& v = kVariants[variant];
     a.zb = v.zb > 0 ? v.zb : (v.zb < 0 && v.tma ? -1 : S.nz);
     if (v.tma && !tma_eligible(S)) fail(BD_ERR_INVALID_ARG, "tile variant %d needs a 16-byte row pitch", variant);
@@ -463,18 +465,33 @@ static void launch_step(WvSession& S, int variant, int64_t s, int koff, cudaStre
         case 15: launch_tma_t<real, 32, 8, 1, 1>(S, a, s, koff, st); break;
         default: fail(BD_ERR_INVALID_ARG, "bad tile variant %d", variant);
     }
-    if (S.any_mur) launch_mur<real>(S, a, koff, st, acc);
+    if (S.any_mur) launch_mur<real>(S, a, koff, st, mur_acc);   // its cells accumulate every step
+}
+
+// Whether the two-cell kernel accumulates in step s for itself and the steps since
+// the last one that did: one step in five, or four, four and two in ten where the
+// energy needs levels two apart (ten steps repeat in a captured chunk).
+static bool acc_due(const WvSession& S, int64_t s) {
+    const int r = (int)(s % 10);
+    return S.p.energy_mode == BD_ENERGY_DPDT2 ? r == 3 || r == 7 || r == 9 : r == 4 || r == 9;
 }
 
 // Issue steps [s, s+n) on the stream (no graph): kernels read *step_base + koff,
-// then one advance kernel moves the counter by n.  acc < 0: each step takes the
-// paired kernel that touches only the accumulators it needs (step_acc_mode);
-// an ACC_* mode forces that one for every step (a captured chunk).
+// then one advance kernel moves the counter by n.  The two-cell kernel accumulates
+// several steps at a time; the last step issued leaves nothing pending.  acc < 0:
+// the accumulating steps take the kernel that touches only the accumulators their
+// steps need (step_acc_mode); an ACC_* mode forces that one (a captured chunk).
 static void issue_steps(WvSession& S, int variant, int64_t s, int n, cudaStream_t st, int acc = -1) {
+    int pending = 0, mode = ACC_NONE;
     for (int k = 0; k < n; ++k) {
-        const int m = acc >= 0 ? acc : step_acc_mode(S, s + k);
-        if (S.prec == BD_F32) launch_step<float>(S, variant, s + k, k, st, m);
-        else launch_step<double>(S, variant, s + k, k, st, m);
+        const int own = acc >= 0 ? acc : step_acc_mode(S, s + k);
+        if (acc_rank(own) > acc_rank(mode)) mode = own;
+        ++pending;
+        const bool now = !kVariants[variant].pair || k == n - 1 || acc_due(S, s + k);
+        const int m = now ? mode : ACC_NONE;
+        if (S.prec == BD_F32) launch_step<float>(S, variant, s + k, k, st, m, now ? pending : 0, own);
+        else launch_step<double>(S, variant, s + k, k, st, m, now ? pending : 0, own);
+        if (now) { pending = 0; mode = ACC_NONE; }
     }
     wv_advance_kernel<<<1, 32, 0, st>>>(S.step_base.as<long long>(), n);
     BD_LAUNCHED(S.ctx);

@@ -46,6 +46,7 @@ struct WvArgs {
     int zb;                    // z-chunk per CTA
     int px;                    // row pitch in cells
     int rev;                   // two-cell kernel: march from the high end
+    int acc_n;                 // two-cell kernel: steps this one accumulates (itself and acc_n - 1 before it)
     long long plane;           // px*ny
     // time levels: p^n (stencil), p^{n-1..n-3}, and the p^{n-4} buffer that receives p^{n+1}
     const real* __restrict__ p0;

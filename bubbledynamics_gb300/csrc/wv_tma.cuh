@@ -28,6 +28,10 @@ constexpr int TMA_NP = 8;   // p^n plane slots (>= 7)
 // none, the peak map only, peak and energy without the DFT
 constexpr int ACC_ALL = 0, ACC_NONE = 1, ACC_PEAK = 2, ACC_PE = 3;
 constexpr int TMA_NQ = 3;   // pointwise slots
+// steps the two-cell kernel accumulates at once, at most: their pressures are
+// p^{n+1}..p^{n-3}; the (dp/dt)^2 energy of a step also needs the level two before
+// its own, so it stops at four
+constexpr int ACC_STEPS = 5, ACC_DPDT = 4;
 constexpr int FL_NOC = 4;   // kernel flags: no c map, materials by plane or cell
 
 struct TmaMaps {

@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const long long step = *a.step_base + koff;
     if constexpr (ACC == ACC_ALL && sizeof(real) == 4)
-        pf_dft = a.n_dft > 0 && step >= a.dft_start && step < a.dft_start + a.dft_len;
+        pf_dft = a.n_dft > 0 && step >= a.dft_start && step - a.acc_n + 1 < a.dft_start + a.dft_len;
     if (tid == 0) {
         for (int q = 0; q < TMA_NP; ++q) issueP(q);
         for (int r = 0; r < NQ; ++r) issueQ(r);
@@ -314,10 +314,27 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
         for (int q = TMA_NP; q < TMA_NP + 3; ++q) issueP(q);
 
     const bool fix_x = a.mir_x && x0 == 0, fix_y = a.mir_y && y0 == 0;
-    const bool do_peak = ACC != ACC_NONE && step >= a.peak_start && step < a.peak_end;
-    const bool do_energy = (ACC == ACC_ALL || ACC == ACC_PE) && step >= a.energy_start && step < a.energy_end;
+    // Deferred accumulation: a step's peak, energy and DFT terms follow from its
+    // pressure alone, which stays in the ring, so one step in four or five adds its
+    // own terms and those of the steps since the last such step, oldest first (the
+    // same operations on every accumulator, so the same bits), and the steps between
+    // leave the accumulators alone.  Bit m: step - m is inside the window.
+    const int acc_n = ACC == ACC_NONE ? 0 : a.acc_n;
+    unsigned peak_m = 0, energy_m = 0, dft_m = 0;
+    if constexpr (ACC != ACC_NONE) {
+#pragma unroll
+        for (int m = 0; m < ACC_STEPS; ++m) {
+            const long long t = step - m;
+            if (m >= acc_n) continue;
+            if (t >= a.peak_start && t < a.peak_end) peak_m |= 1u << m;
+            if (t >= a.energy_start && t < a.energy_end) energy_m |= 1u << m;
+            if (a.n_dft > 0 && t >= a.dft_start && t < a.dft_start + a.dft_len) dft_m |= 1u << m;
+        }
+    }
+    const bool do_peak = peak_m != 0;
+    const bool do_energy = (ACC == ACC_ALL || ACC == ACC_PE) && energy_m != 0;
+    const bool do_dft = ACC == ACC_ALL && dft_m != 0;
     const long long ds = step - a.dft_start;
-    const bool do_dft = ACC == ACC_ALL && a.n_dft > 0 && ds >= 0 && ds < a.dft_len;
     const bool single_mat = FL >= 0 && FL != FL_NOC ? (FL & 1) != 0 : (!a.matmap && !a.plane_mat);
     const bool dpdt = a.energy_mode == BD_ENERGY_DPDT2;
 
@@ -378,6 +395,7 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
             if (!FAST && !active[0]) return;       // a thread's first cell is the last to leave the grid
             const F2 q1p = ld2(q1t + k);
             F2 pnp, ro[NRMAX > 0 ? NRMAX : 1];
+            const F2 q2 = ld2(q2t + k), q3 = ld2(q3t + k), q4 = ld2(q4t + k);
             bool have[CX] = {FAST, FAST};
             int nrx[CX] = {0, 0};                  // relaxation processes of the cells' materials
             if (!FAST && src_plane) {
@@ -398,7 +416,6 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
                          sx3 = f2(add_(e[7], e[1]), add_(e[8], e[2]));
                 const F2 sy1 = f2_add(ld2(cp + W), ld2(cp - W)), sy2 = f2_add(ld2(cp + 2 * W), ld2(cp - 2 * W)),
                          sy3 = f2_add(ld2(cp + 3 * W), ld2(cp - 3 * W));
-                const F2 q2 = ld2(q2t + k), q3 = ld2(q3t + k), q4 = ld2(q4t + k);
                 F2 rc[NRMAX > 0 ? NRMAX : 1];
 #pragma unroll
                 for (int v = 0; v < NRMAX; ++v) {
@@ -423,9 +440,8 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
                 nrx[0] = have[0] ? nr0 : 0;
                 nrx[1] = have[1] ? nr1 : 0;
             }
-            float pn[CX], q1[CX];
+            float pn[CX];
             f2_split(pnp, pn[0], pn[1]);
-            f2_split(q1p, q1[0], q1[1]);
             // stores: a pair access where both cells take part, else per cell
             if (FAST || (have[0] && have[1])) st2(p4z + col, pnp);
             else
@@ -447,27 +463,44 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
 #pragma unroll
             for (int c = 0; c < CX; ++c) acc[c] = FAST || (have[c] && !(murz || murxy[c]));
             const bool acc_pair = acc[0] && acc[1];
+            if constexpr (ACC != ACC_NONE) {
+            // pressures of the steps to accumulate, newest first, and what precedes the oldest
+            const F2 lev[ACC_STEPS + 1] = {pnp, w[3], q1p, q2, q3, q4};
             if (do_peak) {
-                float pk[CX], pv[CX];
+                float pk[CX];
                 f2_split(ld2(pkt + k), pk[0], pk[1]);
 #pragma unroll
-                for (int c = 0; c < CX; ++c) {
-                    const real av = fabs(pn[c]);
-                    pv[c] = av > pk[c] ? av : pk[c];
+                for (int m = ACC_STEPS - 1; m >= 0; --m) {
+                    if (!(peak_m >> m & 1u)) continue;
+                    float v[CX];
+                    f2_split(lev[m], v[0], v[1]);
+#pragma unroll
+                    for (int c = 0; c < CX; ++c) {
+                        const real av = fabs(v[c]);
+                        pk[c] = av > pk[c] ? av : pk[c];
+                    }
                 }
-                if (acc_pair) st2(pkz + col, f2(pv[0], pv[1]));
+                if (acc_pair) st2(pkz + col, f2(pk[0], pk[1]));
                 else
 #pragma unroll
                     for (int c = 0; c < CX; ++c)
-                        if (acc[c]) pkz[col + c] = pv[c];
+                        if (acc[c]) pkz[col + c] = pk[c];
             }
             if (do_energy) {
-                F2 d = pnp;
-                if (dpdt) {
-                    const real h = mul_(real(2.0), a.dt);
-                    d = f2(div_(add_(pn[0], -q1[0]), h), div_(add_(pn[1], -q1[1]), h));
+                F2 ev = ld2(ent + k);
+                const real h = mul_(real(2.0), a.dt);
+#pragma unroll
+                for (int m = ACC_STEPS - 1; m >= 0; --m) {
+                    if (!(energy_m >> m & 1u)) continue;
+                    F2 d = lev[m];
+                    if (dpdt) {                    // p^{t+1} - p^{t-1} (at most ACC_DPDT steps, so lev[m + 2] exists)
+                        float v0, v1, u0, u1;
+                        f2_split(lev[m], v0, v1);
+                        f2_split(lev[m + 2 <= ACC_STEPS ? m + 2 : ACC_STEPS], u0, u1);
+                        d = f2(div_(add_(v0, -u0), h), div_(add_(v1, -u1), h));
+                    }
+                    ev = f2_add(ev, f2_mul1(f2_mul(d, d), f2(a.dt)));
                 }
-                const F2 ev = f2_add(ld2(ent + k), f2_mul1(f2_mul(d, d), f2(a.dt)));
                 if (acc_pair) st2(enz + col, ev);
                 else {
                     float e0, e1;
@@ -476,60 +509,55 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
                     if (acc[1]) enz[col + 1] = e1;
                 }
             }
-            if (do_dft && iz >= a.dz_lo && iz < a.dz_hi && acc_pair) {
-                // both cells accumulate: one pair load and store per accumulator
-                                const long long pl = (long long)(iz - a.dz_lo) * a.plane + col;
+            if (do_dft && iz >= a.dz_lo && iz < a.dz_hi) {
+                const long long pl = (long long)(iz - a.dz_lo) * a.plane + col;
                 const long long stride = (long long)(a.dz_hi - a.dz_lo) * a.plane;
                 const real* tw = a.tw + ds * a.n_dft * 2;
                 real* dr = a.dre + pl;
                 real* di = a.dim + pl;
-                int j = 0;
-                for (; j + 4 <= a.n_dft; j += 4) {
-                    F2 r[4], m[4];
+                auto add = [&](F2& r, F2& i, int j) {
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        r[u] = ld2(dr + (j + u) * stride);
-                        m[u] = ld2(di + (j + u) * stride);
+                    for (int m = ACC_STEPS - 1; m >= 0; --m) {
+                        if (!(dft_m >> m & 1u)) continue;
+                        const float2 t = __ldg(reinterpret_cast<const float2*>(tw + 2 * (j - m * a.n_dft)));
+                        r = f2_fma(lev[m], f2(t.x), r);
+                        i = f2_fma(lev[m], f2(-t.y), i);
                     }
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const real tr = tw[2 * (j + u)], ti = tw[2 * (j + u) + 1];
-                        st2(dr + (j + u) * stride, f2_fma(pnp, f2(tr), r[u]));
-                        st2(di + (j + u) * stride, f2_fma(pnp, f2(-ti), m[u]));
-                    }
-                }
-                for (; j < a.n_dft; ++j) {
-                    const F2 r = ld2(dr + j * stride), m = ld2(di + j * stride);
-                    st2(dr + j * stride, f2_fma(pnp, f2(tw[2 * j]), r));
-                    st2(di + j * stride, f2_fma(pnp, f2(-tw[2 * j + 1]), m));
-                }
-            } else if (do_dft && iz >= a.dz_lo && iz < a.dz_hi) {
-#pragma unroll
-                for (int cx = 0; cx < CX; ++cx) {
-                    if (!acc[cx]) continue;
-                    const real pv = pn[cx];
-                    const long long pl = (long long)(iz - a.dz_lo) * a.plane + col + cx;
-                    const long long stride = (long long)(a.dz_hi - a.dz_lo) * a.plane;
-                    const real* tw = a.tw + ds * a.n_dft * 2;
-                    real* dr = a.dre + pl;
-                    real* di = a.dim + pl;
+                };
+                if (acc_pair) {
+                    // both cells accumulate: one pair load and store per accumulator, the
+                    // loads of four frequencies before any store
                     int j = 0;
-                    // four frequencies at a time: their eight loads are issued before any store
                     for (; j + 4 <= a.n_dft; j += 4) {
-                        real r[4], m[4];
+                        F2 r[4], i[4];
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) { r[u] = dr[(j + u) * stride]; m[u] = di[(j + u) * stride]; }
+                        for (int u = 0; u < 4; ++u) { r[u] = ld2(dr + (j + u) * stride); i[u] = ld2(di + (j + u) * stride); }
 #pragma unroll
                         for (int u = 0; u < 4; ++u) {
-                            dr[(j + u) * stride] = fma_(pv, tw[2 * (j + u)], r[u]);
-                            di[(j + u) * stride] = fma_(-pv, tw[2 * (j + u) + 1], m[u]);
+                            add(r[u], i[u], j + u);
+                            st2(dr + (j + u) * stride, r[u]);
+                            st2(di + (j + u) * stride, i[u]);
                         }
                     }
                     for (; j < a.n_dft; ++j) {
-                        dr[j * stride] = fma_(pv, tw[2 * j], dr[j * stride]);
-                        di[j * stride] = fma_(-pv, tw[2 * j + 1], di[j * stride]);
+                        F2 r = ld2(dr + j * stride), i = ld2(di + j * stride);
+                        add(r, i, j);
+                        st2(dr + j * stride, r);
+                        st2(di + j * stride, i);
+                    }
+                } else if (acc[0] || acc[1]) {
+                    for (int j = 0; j < a.n_dft; ++j) {
+                        real *pr = dr + j * stride, *pi = di + j * stride;
+                        F2 r = f2(acc[0] ? pr[0] : 0.0f, acc[1] ? pr[1] : 0.0f), i = f2(acc[0] ? pi[0] : 0.0f, acc[1] ? pi[1] : 0.0f);
+                        add(r, i, j);
+                        float r0, r1, i0, i1;
+                        f2_split(r, r0, r1);
+                        f2_split(i, i0, i1);
+                        if (acc[0]) { pr[0] = r0; pi[0] = i0; }
+                        if (acc[1]) { pr[1] = r1; pi[1] = i1; }
                     }
                 }
+            }
             }
         }
         };
