@@ -34,6 +34,7 @@ struct GilK {
     double n1n;        // (n-1)/n
     double irho, ilam, i3lam, nrho;   // 1/rho, 1/lambda, 1/(3 lambda), n/(rho (n-1))
     double iCinf;                     // 1/C_inf
+    double mn1n2, mn1;                // -(n-1)/(2n), -1/n
 };
 
 struct OdeK {
@@ -56,13 +57,50 @@ __constant__ double c_B[7] = {35.0 / 384.0, 0, 500.0 / 1113.0, 125.0 / 192.0, -2
 __constant__ double c_BB[7] = {5179.0 / 57600.0, 0, 7571.0 / 16695.0, 393.0 / 640.0, -92097.0 / 339200.0,
                                187.0 / 2100.0, 1.0 / 40.0};
 __constant__ double c_C[7] = {0, 0.2, 0.3, 0.8, 8.0 / 9.0, 1.0, 1.0};
+// the same at compile time for the fast path, which leaves out the zero entries
+__device__ constexpr double k_A[7][7] = {
+    {0, 0, 0, 0, 0, 0, 0},
+    {0.2, 0, 0, 0, 0, 0, 0},
+    {3.0 / 40.0, -9.0 / 40.0, 0, 0, 0, 0, 0},
+    {44.0 / 45.0, -56.0 / 15.0, 32.0 / 9.0, 0, 0, 0, 0},
+    {19372.0 / 6561.0, -25360.0 / 2187.0, 64448.0 / 6561.0, -212.0 / 729.0, 0, 0, 0},
+    {9017.0 / 3168.0, -355.0 / 33.0, 46732.0 / 5247.0, 49.0 / 176.0, -5103.0 / 18656.0, 0, 0},
+    {35.0 / 384.0, 0, 500.0 / 1113.0, 125.0 / 192.0, -2187.0 / 6784.0, 11.0 / 84.0, 0}};
+// b - b*, the weights of the error estimate
+__device__ constexpr double k_E[7] = {35.0 / 384.0 - 5179.0 / 57600.0, 0, 500.0 / 1113.0 - 7571.0 / 16695.0,
+                                      125.0 / 192.0 - 393.0 / 640.0, -2187.0 / 6784.0 - -92097.0 / 339200.0,
+                                      11.0 / 84.0 - 187.0 / 2100.0, 0 - 1.0 / 40.0};
 
 struct Tones {
     int n;
     int mode;          // 0: sum of tones; 1/2/3: single/dual/triple combo of G:40-78 at amplitude A
     double A;
     double f[BD_MAX_BUBBLE_TONES], a[BD_MAX_BUBBLE_TONES], phi[BD_MAX_BUBBLE_TONES];
+    // what the fast path's drive needs of them, fixed for a whole integration
+    double w[BD_MAX_BUBBLE_TONES];         // 2 pi f
+    double aw[BD_MAX_BUBBLE_TONES][9];     // a w^m
+    double wmax;                           // largest |w|
+    __device__ void derive() {
+        wmax = 0.0;
+        for (int k = 0; k < n; ++k) {
+            w[k] = 2.0 * BD_PI_D * f[k];
+            wmax = fmax(wmax, fabs(w[k]));
+            double wm = a[k];
+            for (int m = 0; m < 9; ++m) { aw[k][m] = wm; wm *= w[k]; }
+        }
+    }
 };
+
+// |x| <= y for y >= 0 (false for NaN) and the larger of |x| and |y| (|x| if y is NaN)
+// on the integer units: a double compare holds its quarter of an SM for 64 cycles a warp, like
+// every FP64 instruction here.
+__device__ __forceinline__ bool abs_le(double x, double y) {
+    return (unsigned long long)(__double_as_longlong(x) & 0x7fffffffffffffffLL) <= (unsigned long long)__double_as_longlong(y);
+}
+__device__ __forceinline__ double abs_max(double x, double y) {
+    const long long a = __double_as_longlong(x) & 0x7fffffffffffffffLL, b = __double_as_longlong(y) & 0x7fffffffffffffffLL;
+    return __longlong_as_double(a > b || b > 0x7ff0000000000000LL ? a : b);
+}
 
 // --------------------------------------------------------------- reference RHS
 // G:40-179 in the reference's operation order (pow calls kept).
@@ -176,7 +214,7 @@ __device__ __forceinline__ void drive_at(const Tones& d, const double* s0, const
     P = 0.0;
     Pdt = 0.0;
     for (int k = 0; k < d.n; ++k) {
-        const double w = 2.0 * BD_PI_D * d.f[k];
+        const double w = d.w[k];
         const double th = w * dt;
         double ss, cc;
         if (fabs(th) <= 0.25) small_sincos(th, ss, cc);
@@ -223,20 +261,15 @@ struct DriveSeries {
 
 __device__ __forceinline__ bool drive_series(const Tones& d, const double* s0, const double* c0, double h,
                                              DriveSeries& S) {
-    double wmax = 0.0;
-    for (int k = 0; k < d.n; ++k) wmax = fmax(wmax, 2.0 * BD_PI_D * fabs(d.f[k]));
-    if (wmax * fabs(h) > 0.02) return false;
+    if (!abs_le(d.wmax * fabs(h), 0.02)) return false;
     double D[9];
 #pragma unroll
     for (int m = 0; m < 9; ++m) D[m] = 0.0;
     for (int k = 0; k < d.n; ++k) {
-        const double w = 2.0 * BD_PI_D * d.f[k];
-        double wm = d.a[k];
 #pragma unroll
         for (int m = 0; m < 9; ++m) {
-            const double v = (m & 1) ? c0[k] : s0[k];
+            const double v = (m & 1) ? c0[k] : s0[k], wm = d.aw[k][m];
             D[m] = fma(((m & 2) ? -wm : wm), v, D[m]);
-            wm *= w;
         }
     }
     double fact = 1.0;
@@ -267,7 +300,7 @@ __device__ __forceinline__ RhsBase rhs_base(const GilK& g, double pin0, double R
     b.iI = 1.0 / b.I;
     const double lI = log(b.I);
     b.Ip = exp(g.n1n * lI);                // I^{(n-1)/n}
-    b.Ipmh = exp(-0.5 * g.n1n * lI);       // I^{-(n-1)/(2n)}
+    b.Ipmh = exp(g.mn1n2 * lI);            // I^{-(n-1)/(2n)}
     b.Ipm = b.Ip * b.iI;                   // I^{-1/n}
     return b;
 }
@@ -277,7 +310,7 @@ __device__ __forceinline__ RhsBase rhs_base(const GilK& g, double pin0, double R
 __device__ __forceinline__ Rhs series_rhs(const GilK& g, const RhsBase& b, double pin0, double R0, double R,
                                           double U, double Tau, double q, double P, double Pdt) {
     const double dr = (R - b.R) * b.iR;
-    if (!(fabs(dr) <= 1e-3)) return fast_rhs(g, pin0, R0, R, U, Tau, q, P, Pdt);
+    if (!abs_le(dr, 1e-3)) return fast_rhs(g, pin0, R0, R, U, Tau, q, P, Pdt);
     const double iR = b.iR * (1.0 - dr * (1.0 - dr * (1.0 - dr * (1.0 - dr * (1.0 - dr * (1.0 - dr))))));
     const double l1 = log1p_s(dr);
     const double pin = b.pin * (1.0 + expm1_s(-g.gamma3 * l1));
@@ -286,11 +319,11 @@ __device__ __forceinline__ Rhs series_rhs(const GilK& g, const RhsBase& b, doubl
     const double iv = 1.0 / v;
     const double I = u * iv;
     const double e = (I - b.I) * b.iI;
-    if (!(fabs(e) <= 1e-3)) return fast_rhs(g, pin0, R0, R, U, Tau, q, P, Pdt);
+    if (!abs_le(e, 1e-3)) return fast_rhs(g, pin0, R0, R, U, Tau, q, P, Pdt);
     const double lI = log1p_s(e);
     const double Ip = b.Ip * (1.0 + expm1_s(g.n1n * lI));
-    const double Ipmh = b.Ipmh * (1.0 + expm1_s(-0.5 * g.n1n * lI));
-    const double Ipm = b.Ipm * (1.0 + expm1_s(-(1.0 - g.n1n) * lI));
+    const double Ipmh = b.Ipmh * (1.0 + expm1_s(g.mn1n2 * lI));
+    const double Ipm = b.Ipm * (1.0 + expm1_s(g.mn1 * lI));
     const double x = R0 * iR;
     const double x3 = x * x * x;
     const double el = -g.G4_3 * (1.0 - x3) - g.mu4 * U * iR;
@@ -359,7 +392,7 @@ __device__ bool dp_attempt(const GilK& g, const OdeK& o, const Tones& d, double 
     } else {
         // fast path: transcendentals and the drive expanded around the step start
         double s0[BD_MAX_BUBBLE_TONES], c0[BD_MAX_BUBBLE_TONES];
-        for (int k = 0; k < d.n; ++k) sincos(2.0 * BD_PI_D * d.f[k] * L.t + d.phi[k], &s0[k], &c0[k]);
+        for (int k = 0; k < d.n; ++k) sincos(d.w[k] * L.t + d.phi[k], &s0[k], &c0[k]);
         DriveSeries ds;
         const bool dser = drive_series(d, s0, c0, h, ds);
         double Pb, Pdb;
@@ -372,18 +405,21 @@ __device__ bool dp_attempt(const GilK& g, const OdeK& o, const Tones& d, double 
             L.have_k1 = true;
         }
         for (int c = 0; c < 4; ++c) K[0][c] = L.k1[c];
+        double P = 0.0, Pd = 0.0;
 #pragma unroll
         for (int i = 1; i < 7; ++i) {
             double ys[4];
             for (int c = 0; c < 4; ++c) {
                 double acc = 0.0;
 #pragma unroll
-                for (int j = 0; j < i; ++j) acc += c_A[i][j] * K[j][c];
+                for (int j = 0; j < i; ++j)
+                    if (k_A[i][j] != 0.0) acc += k_A[i][j] * K[j][c];
                 ys[c] = y[c] + h * acc;
             }
-            double P, Pd;
-            if (dser) ds.eval(c_C[i] * h, P, Pd);
-            else drive_at(d, s0, c0, c_C[i] * h, P, Pd);
+            if (i < 6) {                       // stage 7 sits at the time of stage 6
+                if (dser) ds.eval(c_C[i] * h, P, Pd);
+                else drive_at(d, s0, c0, c_C[i] * h, P, Pd);
+            }
             Rhs r = series_rhs(g, B, pin0, R0, ys[0], ys[1], ys[2], ys[3], P, Pd);
             K[i][0] = r.dR; K[i][1] = r.dU; K[i][2] = r.dT; K[i][3] = r.dq;
             if (i == 6)
@@ -392,7 +428,8 @@ __device__ bool dp_attempt(const GilK& g, const OdeK& o, const Tones& d, double 
         for (int c = 0; c < 4; ++c) {
             double e = 0.0;
 #pragma unroll
-            for (int j = 0; j < 7; ++j) e += (c_B[j] - c_BB[j]) * K[j][c];
+            for (int j = 0; j < 7; ++j)
+                if (k_E[j] != 0.0) e += k_E[j] * K[j][c];
             E[c] = h * e;
         }
     }
@@ -418,7 +455,7 @@ __device__ bool dp_attempt(const GilK& g, const OdeK& o, const Tones& d, double 
         // reference-arithmetic path keeps G's FP64 expressions)
         float S = 0.0f;
         for (int c = 0; c < 4; ++c) {
-            const double sc = o.atol + o.rtol * fmax(fabs(y[c]), fabs(Yn[c]));
+            const double sc = o.atol + o.rtol * abs_max(y[c], Yn[c]);
             const float r = (float)E[c] / (float)sc;
             S = fmaf(r, r, S);
         }
@@ -448,6 +485,7 @@ __device__ __forceinline__ void load_tones(const bd_bubble& b, Tones& d) {
     d.A = 0.0;
     d.n = min(max(b.n_tones, 0), BD_MAX_BUBBLE_TONES);
     for (int k = 0; k < d.n; ++k) { d.f[k] = b.f[k]; d.a[k] = b.a[k]; d.phi[k] = b.phi[k]; }
+    d.derive();
 }
 
 __device__ __forceinline__ void lane_reset(Lane& L, double R0, double h0) {
@@ -620,6 +658,7 @@ __global__ void __launch_bounds__(128) gilmore_threshold_kernel(const double* __
             } else {
                 d.n = 3; d.mode = 3; d.f[0] = f1; d.f[1] = f2; d.f[2] = f3; d.a[0] = d.a[1] = d.a[2] = A / sqrt(3.0);
             }
+            d.derive();
             running = true;
             steps_this = 0;
         }
@@ -657,6 +696,8 @@ static GilK make_gilk(const bd_gilmore_medium* m) {
     g.irho = 1.0 / m->rho; g.ilam = 1.0 / m->lambda; g.i3lam = 1.0 / (3.0 * m->lambda);
     g.nrho = m->n / (m->rho * (m->n - 1.0));
     g.iCinf = 1.0 / m->C_inf;
+    g.mn1n2 = -0.5 * g.n1n;
+    g.mn1 = -(1.0 - g.n1n);
     return g;
 }
 
@@ -687,9 +728,14 @@ static void launch_run(bd_context* ctx, const bd_gilmore_medium* m, long long n,
     const OdeK o = make_odek(ode);
     const int grid = persistent_grid(ctx, (const void*)gilmore_persistent_kernel);
     // with no more bubbles than resident lanes there is nothing to steal: full
-    // warps of the static kernel do the same work (and give the same bits)
+    // warps of the static kernel do the same work (and give the same bits).  One
+    // warp a block spreads them over the SM quarters: 12,000 bubbles in 94 blocks of
+    // four warps left 58 SMs idle and slowed the FP64 units of the others (76 cycles
+    // an instruction with all four quarters busy, 64 with three): 12,000 bubbles over 2 ns
+    // took 432 ms, 370 with one-warp blocks and the stages trimmed above
     if (ode->schedule == BD_SCHEDULE_STATIC || n <= (long long)grid * 128) {
-        gilmore_static_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(d_b, n, g, o, d_r);
+        const unsigned T = n <= (long long)grid * 128 ? 32 : 128;
+        gilmore_static_kernel<<<(unsigned)((n + T - 1) / T), T, 0, st>>>(d_b, n, g, o, d_r);
         BD_LAUNCHED(ctx);
         return;
     }
