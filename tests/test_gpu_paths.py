@@ -1,0 +1,228 @@
+"""The paths a size, a row length or a step count selects, against the general
+ones: device rows padded to 16 bytes, short z chunks, accumulators added several
+steps at a time, the one-pass Mur faces, the heat step's paired doses and its
+integer dose add, bubbles in one-warp blocks.  Wherever both paths perform the
+same operations on every value the comparison is bit for bit."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from bubbledynamics_gb300 import abi, api, presets
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("p_final", "peak", "energy", "Q", "dft_re", "dft_im")
+
+
+def same(a, b, msg):
+    for k in FIELDS:
+        if k in a:
+            np.testing.assert_array_equal(a[k], b[k], err_msg="%s: %s" % (msg, k))
+
+
+def burst(nx, ny, nz, steps):
+    return presets.cfg1(nx, ny, nz, steps, precision=abi.BD_F32)
+
+
+def layers(nx, nz, periods=1, precision=abi.BD_F32):
+    p = presets.ref_W_mini(precision, Nxy=nx, Nz=nz, loop1_periods=1, periods=periods)
+    return p
+
+
+def mapped(nx, ny, nz, steps):
+    """Water and liver mixed cell by cell (0 and 1 relaxation process)."""
+    p = presets.cfg1(nx, ny, nz, steps, precision=abi.BD_F32, heterogeneity=False)
+    p.medium.n_materials = 2
+    p.medium.mat[1] = presets.slab_materials(1.0e6)[2]
+    p.medium.mat[0].n_relax = 0
+    p.set_material_map((np.random.default_rng(3).random((nz, ny, nx)) < 0.5).astype(np.uint8))
+    return p
+
+
+@pytest.mark.parametrize("nx", [33, 34, 35, 61, 65, 67])
+def test_padded_rows_equal_the_plain_kernel(ctx, nx):
+    """Row lengths on either side of the 32- and 64-cell tiles and of every remainder
+    modulo four: the padded two-cell variants and the default give the plain
+    kernel's bits (c map, material map, mirror and Mur faces with the DFT)."""
+    for make in (lambda: burst(nx, 27, 41, 45), lambda: mapped(nx, 27, 41, 45), lambda: layers(nx, 40)):
+        base = None
+        for v in (0, -1, 24, 25, 26, 27, 28):
+            p = make()
+            p.params.tile_variant = v
+            r = ctx.westervelt(p)
+            if v >= 0:
+                assert r["tile_variant"] == v
+            if base is None:
+                base = r
+                assert np.abs(r["p_final"]).max() > 0
+            else:
+                same(r, base, "nx %d, variant %d" % (nx, v))
+
+
+@pytest.mark.parametrize("nz", [8, 9, 15, 17, 50])
+def test_short_chunks_equal_the_plain_kernel(ctx, nz):
+    """Grids that do not fill one wave run in chunks of two planes or more."""
+    base = None
+    for v in (0, 17, 19, 21, 23, -1):
+        p = burst(40, 36, nz, 40)
+        p.params.tile_variant = v
+        r = ctx.westervelt(p)
+        base = base or r
+        same(r, base, "nz %d, variant %d" % (nz, v))
+
+
+@pytest.mark.parametrize("mode", [abi.BD_ENERGY_P2, abi.BD_ENERGY_DPDT2])
+def test_deferred_accumulators_in_any_pieces(ctx, mode):
+    """Windows that open and close between the steps that accumulate, advanced in
+    pieces of every length: the bits of the one-cell kernel, which accumulates
+    every step (variant 17), and of the run in one piece with graphs."""
+    def make(v):
+        p = layers(28, 40)
+        p.params.energy_mode = mode
+        n = p.params.n_steps
+        p.params.peak_start, p.params.peak_end = 3, n - 7
+        p.params.energy_start, p.params.energy_end = 22, 137
+        p.params.dft_start, p.params.dft_len = 101, 61
+        p.params.tile_variant = v
+        return p
+    base = ctx.westervelt(make(17))
+    assert np.abs(base["dft_re"]).max() > 0 and base["energy"].max() > 0
+    for v in (19, 21, 23):
+        same(ctx.westervelt(make(v)), base, "one run, variant %d" % v)
+        p = make(v)
+        with ctx.westervelt_session(p) as s:
+            k, left = 1, p.params.n_steps
+            while left:
+                n = min(k % 13 + 1, left)
+                s.advance(n)
+                left -= n
+                k += 1
+            same(s.finish(), base, "pieces, variant %d" % v)
+
+
+@pytest.mark.parametrize("precision", [abi.BD_F32, abi.BD_F64])
+@pytest.mark.parametrize("n_layers", [1, 2, 5, 8])
+def test_mur_layer_counts(ctx, oracle, precision, n_layers):
+    """The one-pass Mur faces with other layer counts than the reference's three
+    (the x+, y+ and z+ runs meet in the corners): 1e-9 of the FP64 oracle, the
+    1e-5 field tolerance in FP32."""
+    p = layers(26, 44, precision=precision)
+    p.grid.mur_layers = n_layers
+    q = layers(26, 44, precision=abi.BD_F64)
+    q.grid.mur_layers = n_layers
+    got, exp = ctx.westervelt(p), oracle.westervelt(q)
+    for k in ("p_final", "peak", "Q"):
+        a, b = np.asarray(got[k], np.float64), exp[k].reshape(got[k].shape)
+        assert np.linalg.norm(a - b) <= (1e-9 if precision == abi.BD_F64 else 1e-5) * np.linalg.norm(b), k
+
+
+@pytest.mark.parametrize("nx", [33, 35])
+def test_checkpoint_between_padded_and_plain_rows(ctx, nx):
+    """A checkpoint has rows of nx cells whatever the device's: one taken on padded
+    rows continues on the plain kernel's, and the other way round."""
+    whole = ctx.westervelt(layers(nx, 40))
+    for first, second in ((-1, 0), (0, -1)):
+        a, b = layers(nx, 40), layers(nx, 40)
+        a.params.tile_variant, b.params.tile_variant = (first, second)
+        if first == -1:
+            a.params.tile_variant = 28
+        if second == -1:
+            b.params.tile_variant = 28
+        with ctx.westervelt_session(a) as s:
+            s.advance(63)
+            blob = s.checkpoint()
+        with ctx.westervelt_session(b) as s:
+            s.restore(blob)
+            s.advance(a.params.n_steps - 63)
+            same(s.finish(), whole, "%d -> %d" % (first, second))
+
+
+# --------------------------------------------------------------------------- heat
+def thermal(nx, ny, nz, steps, precision=abi.BD_F32, material_map=False):
+    k = presets.ref_T_mini_constants(Nxy=nx, Nz=nz, legs=2)
+    p = presets.make_ref_T(k, precision=precision)
+    p.thermal.ny = ny
+    if material_map:
+        p.set_material_map((np.random.default_rng(5).random((nz, ny, nx)) < 0.5).astype(np.uint8))
+    p.set_spots([0, 3, -2], [0, 1, -4], [steps // 3, steps // 3, steps - 2 * (steps // 3)])
+    Q = presets.gaussian_focus_Q((nz, ny, nx), (nz // 2, ny // 2, nx // 2), (3.0, 2.0, 2.0), 4.0e7)
+    return p, Q
+
+
+@pytest.mark.parametrize("precision", [abi.BD_F32, abi.BD_F64])
+@pytest.mark.parametrize("nx,ny,nz,steps", [(3, 3, 3, 5), (9, 11, 7, 1), (13, 9, 70, 2), (66, 17, 8, 67), (131, 8, 9, 64)])
+def test_heat_run_equals_single_steps(ctx, precision, nx, ny, nz, steps):
+    """Doses added for two steps at once, padded rows and every chunk length, against
+    the same run advanced one step at a time (each step its own dose)."""
+    for material_map in (False, True):
+        p, Q = thermal(nx, ny, nz, steps, precision, material_map)
+        one = ctx.heat(p.thermal, Q, p.traj)
+        s = ctx.heat_slab(p.thermal, Q, p.traj, 0, nz)
+        for _ in range(steps):
+            s.advance(1)
+        got = s.finish()
+        s.close()
+        np.testing.assert_array_equal(one["T"], got["T"])
+        np.testing.assert_array_equal(one["dose"], got["dose"])
+
+
+def test_dose_add_is_the_fp64_sum(ctx):
+    """One step onto doses of every magnitude, sign and kind: the bits of start + increment in
+    double (the increment itself is the dose of the same step from zero)."""
+    nx, ny, nz = 34, 30, 12
+    p, Q = thermal(nx, ny, nz, 1)
+    p.thermal.dose_init = 0
+    inc = ctx.heat(p.thermal, Q, p.traj)["dose"]
+    T0, _ = p.initial_fields()
+    rng = np.random.default_rng(11)
+    n = nx * ny * nz
+    start = np.ldexp(rng.uniform(1.0, 2.0, n), rng.integers(-60, 60, n)) * np.where(rng.random(n) < 0.1, -1.0, 1.0)
+    start *= np.median(inc[1:-1, 1:-1, 1:-1])
+    start[:: 7] = (np.ldexp(1.0, rng.integers(0, 40, n)) * inc.reshape(-1) * (1.0 - 2.0 ** -53))[:: 7]   # next to a carry
+    start[::101], start[1::101], start[2::101] = 0.0, np.inf, np.nan
+    start[3::101], start[4::101], start[5::101] = 5e-324, 1e308, -0.0
+    start = start.reshape(nz, ny, nx)
+    p.set_start(T0, start)
+    got = ctx.heat(p.thermal, Q, p.traj)["dose"]
+    exp = start.copy()
+    exp[1:-1, 1:-1, 1:-1] += inc[1:-1, 1:-1, 1:-1]
+    np.testing.assert_array_equal(got, exp)
+
+
+@pytest.mark.parametrize("nx", [40, 41])
+@pytest.mark.parametrize("steps", [1, 2, 65])
+def test_noalloc_steps_equal_the_run(ctx, nx, steps):
+    """The allocation-free run on vector and scalar rows: the allocating run's
+    temperature bit for bit, its dose to the 2^-47 of a float pair."""
+    torch = pytest.importorskip("torch")
+    p, Q = thermal(nx, 23, 31, steps)
+    th = p.thermal
+    exp = ctx.heat(th, Q, p.traj)
+    sx, sy, _ = api.trajectory_shifts(p.traj)
+    shifts = np.ascontiguousarray(np.stack([sx, sy], axis=1).astype(np.int32))
+    T0, D0 = p.initial_fields()
+    hi = D0.astype(np.float32)
+    pair = np.ascontiguousarray(np.stack([hi, (D0 - hi).astype(np.float32)], axis=-1))
+    theta, q, dose = (torch.from_numpy(a).cuda() for a in ((T0 - th.T_ref).astype(np.float32), Q.astype(np.float32), pair))
+    torch.cuda.synchronize()
+    api.check(ctx.L.bd_heat_run_device_noalloc(ctx.h, C.byref(th), theta.data_ptr(), q.data_ptr(), dose.data_ptr(),
+                                               shifts.ctypes.data, len(sx), None))
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(th.T_ref + theta.cpu().numpy().astype(np.float64), exp["T"])
+    d = dose.cpu().numpy().astype(np.float64).sum(-1)
+    np.testing.assert_allclose(d, exp["dose"], rtol=2.0 ** -44)
+
+
+# --------------------------------------------------------------------------- bubbles
+def test_bubbles_do_not_depend_on_the_batch(ctx):
+    """One-warp blocks (batches that fit the resident lanes) and the one-thread-per-bubble
+    schedule: a bubble's result is the same in a batch of any size."""
+    med, ode = presets.cfg2_medium(), presets.cfg2_ode(t_end=2e-11)
+    b = presets.cfg2_bubbles(257, seed=5)
+    whole, _ = ctx.gilmore(med, b, ode)
+    for n in (1, 31, 32, 33, 129):
+        part, _ = ctx.gilmore(med, b[:n], ode)
+        np.testing.assert_array_equal(part, whole[:n])
+    ode.schedule = abi.BD_SCHEDULE_STATIC
+    np.testing.assert_array_equal(ctx.gilmore(med, b, ode)[0], whole)
