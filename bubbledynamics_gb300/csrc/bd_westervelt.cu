@@ -1552,6 +1552,7 @@ static void adjoint_solve(WvSession& S, const bd_focal_loss* loss, double* loss_
                 a.Hin = Hb[(s + 1) & 1].as<real>();    // written by step s + 1 (zero before the first)
             }
             a.koff = koff;
+            a.rev = (int)(s & 1);
             adj_launch<real>(S, a, cs);
             rot = (rot + 1) % 6;      // lambda_k now sits in the buffer of mu_{k+1}, lambda_4 in the spare
             rrot = (rrot + 1) % 3;
@@ -1829,6 +1830,7 @@ static void adjoint_solve_slabs(std::vector<WvSession*>& sl, const bd_focal_loss
                         a.Hin = P.Hb[(s + 1) & 1].as<real>();    // written by step s + 1
                     }
                     a.koff = koff;
+                    a.rev = (int)(s & 1);
                     adj_launch<real>(S, a, st, part);
                 }
                 if (part != 2)                  // H of this step: ghost planes from the neighbours
