@@ -401,6 +401,28 @@ __global__ void __launch_bounds__(256, FUSE ? 4 : 1) adj_point_kernel(const AdjA
     vstore<real, VEC>(a.H + i0, h);
 }
 
+// Loss of one plane: part[blockIdx.x] = sum of w_L E over the cells of plane
+// iz0 + blockIdx.x.  One block a plane in a fixed order (the same bits on every
+// run and however the planes are split); cells without a weight cost no FP64 add.
+template <class real>
+__global__ void __launch_bounds__(256) adj_loss_kernel(const AdjArgs<real> a, const real* __restrict__ E, int iz0, double* part) {
+    __shared__ double sum[256];
+    const int iz = iz0 + blockIdx.x, dz = iz - a.fz;
+    double v = 0.0;
+    for (int j = threadIdx.x; j < (int)a.plane; j += 256) {
+        const int iy = j / a.nx, dx = j - iy * a.nx - a.fx, dy = iy - a.fy, r2 = dx * dx + dy * dy + dz * dz;
+        if (r2 <= a.frad2) v -= (double)E[iz * a.plane + j];
+        else if (dz == 0 && r2 >= a.srad2 && a.side_w != 0.0) v += a.side_w * (double)E[iz * a.plane + j];
+    }
+    sum[threadIdx.x] = v;
+    __syncthreads();
+    for (int w = 128; w > 0; w >>= 1) {
+        if (threadIdx.x < w) sum[threadIdx.x] += sum[threadIdx.x + w];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) part[blockIdx.x] = sum[0];
+}
+
 // Stencil pass: lambda_0 += (d Lap / d p^s)^T H, the same symmetric
 // 6th-order stencil applied to H with zero outside the grid.  Each thread
 // marches along z over a.zb planes keeping H(iz-3..iz+4) of its column in
