@@ -9,7 +9,7 @@
 //         be lost against 300 K in float), source Q in float, the dose rate
 //         R^(T-43) in float and the dose itself accumulated in double (one
 //         FP64 add per cell and step).  Traffic: theta read + write 8 B, Q 4 B,
-//         dose RMW 16 B.
+//         dose RMW 16 B every other step.
 // The allocation-free entry point keeps its dose as a double-float pair (hi,
 // lo) updated with error-free FP32 sums (its caller-owned buffer format).
 #include <cuda_runtime.h>
@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "bd_internal.h"
+#include "f32x2.cuh"
 
 namespace bd {
 
@@ -37,8 +38,8 @@ struct HeatMat {
 // bytes a cell), and a step's increment follows from its temperature alone, which
 // the next step reads anyway: of two steps the first leaves the dose alone
 // (DOSE_LATER) and the second adds both increments, in order (DOSE_BOTH), at 12 + 28
-// bytes for the two.  256 x 256 x 384: 92 us a step, 106 with DOSE_THIS alone;
-// 213 x 213 x 201: 41 and 45.
+// bytes for the two.  256 x 256 x 384: 87 us a step, 106 with DOSE_THIS alone;
+// 213 x 213 x 201: 40 and 45.
 enum HeatDose { DOSE_LATER = 0, DOSE_THIS = 1, DOSE_BOTH = 2 };
 
 template <class real>
@@ -300,6 +301,86 @@ __global__ void __launch_bounds__(128) heat_step4_kernel(const HeatArgs<float> a
     }
 }
 
+// The four-cell step without the dose (DOSE_LATER) and without a material map: 12
+// bytes a cell, so instructions weigh more than in heat_step4_kernel.  Offsets are
+// formed once and pointers advance, the material of a plane stays in registers until
+// it changes, one cell of each neighbouring vector is read instead of four, and the
+// arithmetic runs on pairs (the same operations, so the same bits).  Held to 64
+// registers, eight blocks a SM: 256 x 256 x 384 90.9 -> 87.3 us a step of a pair,
+// 213 x 213 x 201 41.3 -> 39.7 (ten blocks spill: 92.6 and 42.3).
+__global__ void __launch_bounds__(128, 8) heat_theta4_kernel(const HeatArgs<float> a, int koff) {
+    const int x0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+    const int iy = blockIdx.y * blockDim.y + threadIdx.y;
+    if (x0 >= a.nx || iy < 1 || iy >= a.ny - 1) return;
+    const int bz = a.rev ? gridDim.z - 1 - blockIdx.z : blockIdx.z;
+    const int z0 = max(1, bz * a.zb);
+    const int z1 = min(a.nz - 1, bz * a.zb + a.zb);
+    if (z0 >= z1) return;
+    const int2 sh = a.shifts[*a.step_base + koff];
+    auto ld4 = [](const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); };
+    int iz = a.rev ? z1 - 1 : z0;
+    const int one = a.rev ? -1 : 1;
+    const long long dz = a.rev ? -a.plane : a.plane;
+    const long long i = (long long)iz * a.plane + (long long)iy * a.px + x0;
+    const int NX = a.px;
+    const int ya = iy - sh.y, xa = x0 - sh.x;
+    const bool row = ya >= 0 && ya < a.ny;
+    bool qok[4], upd[4];
+    int qo[4];
+    const int xc = min(max(xa, 0), a.nx - 1);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        qok[k] = row && xa + k >= 0 && xa + k < a.nx;
+        qo[k] = min(max(xa + k, 0), a.nx - 1) - xc;
+        upd[k] = x0 + k >= 1 && x0 + k < a.nx - 1;
+    }
+    const float* pQ = a.Q + (long long)iz * a.plane + (long long)min(max(ya, 0), a.ny - 1) * NX + xc;
+    const float* T = a.Tin + i;
+    float* O = a.Tout + i;
+    const int oL = x0 >= 1 ? -1 : 0, oR = x0 + 4 < NX ? 4 : 0;
+    float4 tm = ld4(T - dz), tc = ld4(T);
+    int mcur = a.plane_mat ? __ldg(a.plane_mat + iz) : 0;
+    HeatMat<float> M = a.mat[mcur];
+    for (int n = z1 - z0; n > 0; --n) {
+        const float4 tp = ld4(T + dz), yu = ld4(T + NX), yd = ld4(T - NX);
+        const float L = __ldg(T + oL), R = __ldg(T + oR);
+        float q[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float v = __ldg(pQ + qo[k]);
+            q[k] = qok[k] ? v : 0.f;
+        }
+        T += dz;
+        pQ += dz;
+        iz += one;
+        const int mnext = n > 1 && a.plane_mat ? __ldg(a.plane_mat + iz) : mcur;
+        const float cv[4] = {tc.x, tc.y, tc.z, tc.w};
+        const float xs[4] = {L + tc.y, tc.x + tc.z, tc.y + tc.w, tc.z + R};
+        const float su[4] = {yu.x, yu.y, yu.z, yu.w}, sd[4] = {yd.x, yd.y, yd.z, yd.w};
+        const float zu[4] = {tp.x, tp.y, tp.z, tp.w}, zd[4] = {tm.x, tm.y, tm.z, tm.w};
+        float tn[4];
+#pragma unroll
+        for (int k = 0; k < 4; k += 2) {
+            const F2 sxy = f2_add(f2_add(f2(xs[k], xs[k + 1]), f2(su[k], su[k + 1])), f2(sd[k], sd[k + 1]));
+            const F2 zz = f2_add(f2(zu[k], zu[k + 1]), f2(zd[k], zd[k + 1]));
+            F2 t = f2_fma(f2(cv[k], cv[k + 1]), f2(M.a0, M.a0), f2_mul(f2(M.kxy, M.kxy), sxy));
+            t = f2_fma(f2(M.kz, M.kz), zz, t);
+            t = f2_fma(f2(M.qc, M.qc), f2(q[k], q[k + 1]), t);
+            f2_split(f2_add(t, f2(M.wTa, M.wTa)), tn[k], tn[k + 1]);
+            tn[k] = upd[k] ? tn[k] : cv[k];
+            tn[k + 1] = upd[k + 1] ? tn[k + 1] : cv[k + 1];
+        }
+        *reinterpret_cast<float4*>(O) = make_float4(tn[0], tn[1], tn[2], tn[3]);
+        O += dz;
+        if (mnext != mcur) {
+            mcur = mnext;
+            M = a.mat[mcur];
+        }
+        tm = tc;
+        tc = tp;
+    }
+}
+
 // Planes per CTA of the FP32 kernels.  A chunk costs its planes plus about 0.7 of
 // a plane's time to start; grids of several waves fill up as CTAs end and pay
 // half a chunk at the end.  Measured per step: 256 x 256 x 384 105.7 / 105.5 /
@@ -325,7 +406,10 @@ static int dose_mode(int64_t k, int64_t cnt) {
 template <bool PAIR>
 static void step4_launch(const HeatArgs<float>& a, int koff, int mode, dim3 grid, cudaStream_t st) {
     const dim3 block(16, 8);
-    if (mode == DOSE_LATER) heat_step4_kernel<PAIR, DOSE_LATER><<<grid, block, 0, st>>>(a, koff);
+    // chunks of two or three planes (small grids) end before what the kernel without
+    // the dose sets up has paid: 72 x 72 x 60 launch by launch 6.7 us a step, 7.2 with it
+    if (mode == DOSE_LATER && !a.matmap && a.zb >= 4) heat_theta4_kernel<<<grid, block, 0, st>>>(a, koff);
+    else if (mode == DOSE_LATER) heat_step4_kernel<PAIR, DOSE_LATER><<<grid, block, 0, st>>>(a, koff);
     else if (mode == DOSE_THIS) heat_step4_kernel<PAIR, DOSE_THIS><<<grid, block, 0, st>>>(a, koff);
     else heat_step4_kernel<PAIR, DOSE_BOTH><<<grid, block, 0, st>>>(a, koff);
 }
