@@ -176,6 +176,10 @@ static WvArgs<real> make_args(WvSession& S, int64_t s) {
     a.dt = (real)g.dt;
     a.kxy180 = (real)(g.dt * g.dt / (g.dx * g.dx) / 180.0);
     a.kz180 = (real)(g.dt * g.dt / (g.dz * g.dz) / 180.0);
+    const double hxy = g.dt * g.dt / (g.dx * g.dx) / 180.0, hz = g.dt * g.dt / (g.dz * g.dz) / 180.0;
+    const double st[7] = {-980.0 * hxy - 490.0 * hz, 270.0 * hxy, -27.0 * hxy, 2.0 * hxy, 270.0 * hz, -27.0 * hz, 2.0 * hz};
+    for (int k = 0; k < 7; ++k) a.st[k] = (real)st[k];
+    a.ke = (real)(S.p.energy_mode == BD_ENERGY_DPDT2 ? 0.25 / g.dt : g.dt);
     a.dt2 = (real)(g.dt * g.dt);
     a.dtdx = (real)(g.dt / g.dx);
     a.dtdz = (real)(g.dt / g.dz);

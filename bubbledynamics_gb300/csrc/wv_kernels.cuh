@@ -33,6 +33,7 @@ struct MatConst {
     real kxy, kz, kd, kn, kr;  // stencil xy and z, diffusivity, nonlinearity, (c dt)^2
     real xr;                   // x / (1 - x), x = 3 kr sum a (semi-implicit relaxation)
     real av[BD_MAX_RELAX];     // a_v
+    real st[sizeof(real) == 8 ? 7 : 1];   // FP64: (c dt / d)^2 times the stencil weights (WvArgs::st)
 };
 
 template <class real>
@@ -98,6 +99,8 @@ struct WvArgs {
     real* __restrict__ dim;
     const real* __restrict__ tw;               // DFT twiddles [dft step][n_dft][2]
     long long peak_start, peak_end, energy_start, energy_end, dft_start, dft_len;
+    real ke;                   // FP64: weight of p^2 (dt) or of (p^{n+1} - p^{n-1})^2 (1 / 4dt) in the energy
+    real st[7];                // FP64: stencil weights over d^2: p; the +-1, +-2, +-3 rings in x and y; the same in z
     int energy_mode, n_dft, dz_lo, dz_hi;
     int relax_scheme;
     int mat_tile;              // 1: the two-cell kernel receives the material map as a TMA tile per plane
@@ -158,9 +161,24 @@ __device__ __forceinline__ bool is_mur_cell(const WvArgs<real>& a, int ix, int i
            (a.mur_zp && iz >= a.nz - a.L) || (a.mur_zm && iz < a.Lzm);
 }
 
+// max(|v|, pk).  FP64 values compare as integers: a double compare takes the FP64
+// unit, 64 cycles a warp, like every FP64 instruction here.
+__device__ __forceinline__ float peak_max(float v, float pk) {
+    const float av = fabsf(v);
+    return av > pk ? av : pk;
+}
+__device__ __forceinline__ double peak_max(double v, double pk) {
+    const long long av = __double_as_longlong(v) & 0x7fffffffffffffffLL;
+    return av <= 0x7ff0000000000000LL && av > __double_as_longlong(pk) ? __longlong_as_double(av) : pk;
+}
+
 // Energy accumulator update: E + p^2 dt, or E + ((p^{n+1}-p^{n-1})/2dt)^2 dt (W:253-257).
 template <class real>
 __device__ __forceinline__ real energy_add(const WvArgs<real>& a, real old, real v, real vm1) {
+    if constexpr (sizeof(real) == 8) {             // three FP64 instructions, no division
+        const real d = a.energy_mode == BD_ENERGY_DPDT2 ? add_(v, -vm1) : v;
+        return fma_(mul_(d, d), a.ke, old);
+    }
     real e;
     if (a.energy_mode == BD_ENERGY_DPDT2) {
         const real dp = div_(add_(v, -vm1), mul_(real(2.0), a.dt));     // W:253
@@ -176,9 +194,7 @@ template <class real>
 __device__ __forceinline__ void accumulate(const WvArgs<real>& a, long long step, long long i, int ix, int iy,
                                            int iz, real v, real vm1) {
     if (step >= a.peak_start && step < a.peak_end) {
-        const real av = fabs(v);
-        const real pk = a.peak[i];
-        a.peak[i] = av > pk ? av : pk;
+        a.peak[i] = peak_max(v, a.peak[i]);
     }
     if (step >= a.energy_start && step < a.energy_end) a.energy[i] = energy_add(a, a.energy[i], v, vm1);
     const long long ds = step - a.dft_start;
@@ -217,8 +233,13 @@ __device__ __forceinline__ void cell_coef(const WvArgs<real>& a, MatConst<real>&
     const real c2 = mul_(c, c);
     const real ic = div_(real(1), c);
     const real ic2 = mul_(ic, ic);
-    M.kxy = mul_(c2, a.kxy180);
-    M.kz = mul_(c2, a.kz180);
+    if constexpr (sizeof(real) == 8) {
+#pragma unroll
+        for (int k = 0; k < 7; ++k) M.st[k] = mul_(c2, a.st[k]);
+    } else {
+        M.kxy = mul_(c2, a.kxy180);
+        M.kz = mul_(c2, a.kz180);
+    }
     M.kd = mul_(M.delta_2dt, ic2);
     M.kn = mul_(M.beta2_rho, ic2);
     M.kr = mul_(c2, a.dt2);
@@ -261,9 +282,6 @@ template <class real, int NRMAX = BD_MAX_RELAX>
 __device__ __forceinline__ real cell_update(const WvArgs<real>& a, const MatConst<real>& M, real pc, real sx1, real sx2,
                                             real sx3, real sy1, real sy2, real sy3, const real* w, real q1, real q2,
                                             real q3, real q4, const real* rc, real* ro) {
-    const real Dxx = d2x180(pc, sx1, sx2, sx3);
-    const real Dyy = d2x180(pc, sy1, sy2, sy3);
-    const real Dzz = d2x180(pc, add_(w[4], w[2]), add_(w[5], w[1]), add_(w[6], w[0]));
     // W:207: 5 p - 18 p1 + 24 p2 - 14 p3 + 3 p4
     const real Dttt = fma_(real(3), q4, fma_(real(-14), q3, fma_(real(24), q2, fma_(real(-18), q1, mul_(real(5), pc)))));
     const real s3 = fma_(real(3), pc, fma_(real(-4), q1, q2));
@@ -275,9 +293,24 @@ __device__ __forceinline__ real cell_update(const WvArgs<real>& a, const MatCons
     // cells per wavelength) and p^{n+1} takes one final rounding: the FP32 field
     // error against FP64 after 3000 cfg1 steps drops from 1.04e-5 to 8.4e-6
     // (summing 2p - p1 + ... directly rounds at the size of p five times).
+    // FP64 is bound by its FP64 instructions: there the weights carry (c dt / d)^2 and
+    // the x and y rings add up first, 19 instructions instead of 24 (and the
+    // relaxation terms go straight into V; 64 x 64 x 201, two processes: 199.8 -> 188.0 us a
+    // step).
     real V = add_(pc, -q1);
-    V = fma_(M.kxy, add_(Dxx, Dyy), V);
-    V = fma_(M.kz, Dzz, V);
+    const real sz1 = add_(w[4], w[2]), sz2 = add_(w[5], w[1]), sz3 = add_(w[6], w[0]);
+    if constexpr (sizeof(real) == 8) {
+        V = fma_(M.st[0], pc, V);
+        V = fma_(M.st[1], add_(sx1, sy1), V);
+        V = fma_(M.st[2], add_(sx2, sy2), V);
+        V = fma_(M.st[3], add_(sx3, sy3), V);
+        V = fma_(M.st[4], sz1, V);
+        V = fma_(M.st[5], sz2, V);
+        V = fma_(M.st[6], sz3, V);
+    } else {
+        V = fma_(M.kxy, add_(d2x180(pc, sx1, sx2, sx3), d2x180(pc, sy1, sy2, sy3)), V);
+        V = fma_(M.kz, d2x180(pc, sz1, sz2, sz3), V);
+    }
     V = fma_(M.kd, Dttt, V);
     V = fma_(M.kn, add_(D1, D2), V);
     real pn;
@@ -291,7 +324,8 @@ __device__ __forceinline__ real cell_update(const WvArgs<real>& a, const MatCons
         for (int v = 0; v < NRMAX; ++v) {
             if (v < M.n_relax) {
                 bv[v] = mul_(M.rb[v], fma_(real(4), rc[v], -ro[v]));
-                G = add_(G, fma_(M.av[v], E, bv[v]));
+                const real g = fma_(M.av[v], E, bv[v]);
+                G = sizeof(real) == 8 && v == 0 ? g : add_(G, g);
             }
         }
         const real Vn = fma_(M.kr, G, V);                        // num = p + Vn
@@ -307,10 +341,12 @@ __device__ __forceinline__ real cell_update(const WvArgs<real>& a, const MatCons
                 // W:227: R = 2dt 2 c_v tau Dttt/(2dt^3) / ((2dt+3tau) c^3) + tau (4 R1 - R2)/(2dt+3tau)
                 const real rn = fma_(M.av[v], Dttt, mul_(M.rb[v], fma_(real(4), rc[v], -ro[v])));
                 ro[v] = rn;
-                sumR = add_(sumR, rn);
+                if constexpr (sizeof(real) == 8) V = fma_(rn, M.kr, V);
+                else sumR = add_(sumR, rn);
             }
         }
-        pn = add_(pc, fma_(sumR, M.kr, V));                                                      // W:234
+        if constexpr (sizeof(real) == 4) V = fma_(sumR, M.kr, V);
+        pn = add_(pc, V);                                                      // W:234
     }
     return pn;
 }
@@ -338,22 +374,23 @@ __global__ void __launch_bounds__(TX* TY) wv_step_kernel(const WvArgs<real> a, c
     const int z0 = blockIdx.z * a.zb;
     const int z1 = min(a.nz, z0 + a.zb);
     const int nx = a.nx;
-    // neighbour offsets and weights along x and y (mirror at index 0, zero ghosts outside)
+    // neighbour offsets along x and y (mirror at index 0) and which are cells (zero ghosts
+    // outside; selected, as weights of 0 and 1 cost six FP64 multiplications a cell)
     int xo[6], yo[6];
-    real xw[6], yw[6];
+    bool xw[6], yw[6];
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
         const int o = k < 3 ? k - 3 : k - 2;   // -3,-2,-1,1,2,3
         int jx = ix + o;
-        real wxk = real(1);
-        if (jx < 0) { if (a.mir_x) jx = -jx; else { jx = ix; wxk = real(0); } }
-        if (jx >= nx) { jx = ix; wxk = real(0); }
-        xo[k] = jx - ix; xw[k] = wxk;
+        xw[k] = true;
+        if (jx < 0) { if (a.mir_x) jx = -jx; else { jx = ix; xw[k] = false; } }
+        if (jx >= nx) { jx = ix; xw[k] = false; }
+        xo[k] = jx - ix;
         int jy = iy + o;
-        real wyk = real(1);
-        if (jy < 0) { if (a.mir_y) jy = -jy; else { jy = iy; wyk = real(0); } }
-        if (jy >= a.ny) { jy = iy; wyk = real(0); }
-        yo[k] = (jy - iy) * a.px; yw[k] = wyk;
+        yw[k] = true;
+        if (jy < 0) { if (a.mir_y) jy = -jy; else { jy = iy; yw[k] = false; } }
+        if (jy >= a.ny) { jy = iy; yw[k] = false; }
+        yo[k] = (jy - iy) * a.px;
     }
     const bool col_in_box = ix <= a.xhi && iy <= a.yhi;
     const real sw_xy = a.wx ? mul_(a.wx[ix], a.wy[iy]) : real(1);
@@ -380,12 +417,13 @@ __global__ void __launch_bounds__(TX* TY) wv_step_kernel(const WvArgs<real> a, c
         } else if (col_in_box && iz >= a.zlo && iz <= a.zhi) {
             const real pc = w[3];
             const real* P = a.p0 + i;
-            const real sx1 = xw[3] * ld(P + xo[3]) + xw[2] * ld(P + xo[2]);
-            const real sx2 = xw[4] * ld(P + xo[4]) + xw[1] * ld(P + xo[1]);
-            const real sx3 = xw[5] * ld(P + xo[5]) + xw[0] * ld(P + xo[0]);
-            const real sy1 = yw[3] * ld(P + yo[3]) + yw[2] * ld(P + yo[2]);
-            const real sy2 = yw[4] * ld(P + yo[4]) + yw[1] * ld(P + yo[1]);
-            const real sy3 = yw[5] * ld(P + yo[5]) + yw[0] * ld(P + yo[0]);
+            const auto nb = [](bool in, const real* p) { const real v = ld(p); return in ? v : real(0); };
+            const real sx1 = nb(xw[3], P + xo[3]) + nb(xw[2], P + xo[2]);
+            const real sx2 = nb(xw[4], P + xo[4]) + nb(xw[1], P + xo[1]);
+            const real sx3 = nb(xw[5], P + xo[5]) + nb(xw[0], P + xo[0]);
+            const real sy1 = nb(yw[3], P + yo[3]) + nb(yw[2], P + yo[2]);
+            const real sy2 = nb(yw[4], P + yo[4]) + nb(yw[1], P + yo[1]);
+            const real sy3 = nb(yw[5], P + yo[5]) + nb(yw[0], P + yo[0]);
             const real q1 = ld(a.p1 + i), q2 = ld(a.p2 + i), q3 = ld(a.p3 + i), q4 = a.p4[i];
             const int m = cell_mat(a, i, iz);
             real rc[BD_MAX_RELAX], ro[BD_MAX_RELAX];
@@ -531,10 +569,7 @@ __global__ void __launch_bounds__(128) wv_mur_kernel(const WvArgs<real> a, const
             if (l >= nl) break;
             const long long i = i0 + l * st;
             F[i] = v[l];
-            if (do_peak) {
-                const real av = fabs(v[l]), pk = a.peak[i];
-                a.peak[i] = av > pk ? av : pk;
-            }
+            if (do_peak) a.peak[i] = peak_max(v[l], a.peak[i]);
             if (do_energy) a.energy[i] = energy_add(a, a.energy[i], v[l], a.energy_mode == BD_ENERGY_DPDT2 ? a.p1[i] : real(0));
         }
         return;

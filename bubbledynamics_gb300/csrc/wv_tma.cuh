@@ -256,7 +256,6 @@ __global__ void __launch_bounds__(TX* TY / CPT) wv_tma_kernel(const WvArgs<real>
     const long long ds = step - a.dft_start;
     const bool do_dft = a.n_dft > 0 && ds >= 0 && ds < a.dft_len;
     const bool single_mat = FL >= 0 && FL != FL_NOC ? (FL & 1) != 0 : (!a.matmap && !a.plane_mat);
-    const bool dpdt = a.energy_mode == BD_ENERGY_DPDT2;
     // the material of single-material problems, in registers
     const MatConst<real> M0 = sK[0];
 
@@ -361,20 +360,8 @@ __global__ void __launch_bounds__(TX* TY / CPT) wv_tma_kernel(const WvArgs<real>
             if (have) {
                 p4z[col[c]] = pn;
                 if (!(murz || murxy[c])) {
-                    if (do_peak) {
-                        const real av = fabs(pn), pk = pkt[k];
-                        pkz[col[c]] = av > pk ? av : pk;
-                    }
-                    if (do_energy) {
-                        real e;
-                        if (dpdt) {
-                            const real dp = div_(add_(pn, -q1), mul_(real(2.0), a.dt));
-                            e = mul_(mul_(dp, dp), a.dt);
-                        } else {
-                            e = mul_(mul_(pn, pn), a.dt);
-                        }
-                        enz[col[c]] = add_(ent[k], e);
-                    }
+                    if (do_peak) pkz[col[c]] = peak_max(pn, pkt[k]);
+                    if (do_energy) enz[col[c]] = energy_add(a, ent[k], pn, q1);
                     if (do_dft && iz >= a.dz_lo && iz < a.dz_hi) {
                         const long long pl = (long long)(iz - a.dz_lo) * a.plane + col[c];
                         const long long stride = (long long)(a.dz_hi - a.dz_lo) * a.plane;
