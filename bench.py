@@ -9,7 +9,7 @@ dx = 0.1875 mm, heterogeneous c, one relaxation process, 20-cell sponge, 1 MHz
              timed with CUDA events on the library's stream
   e2e        K calls of bd_westervelt_run through the C ABI with host buffers:
              c map and source tables uploaded, peak and energy maps read back
-  roofline   algorithmic bytes of the step kernel (56 B/cell) / its event-timed
+  roofline   algorithmic bytes of the step kernel (43.2 B/cell) / its event-timed
              duration, against the measured HBM copy bandwidth
   cpu_baseline  the CPU oracle (OpenMP, all host cores) on a bounded sample
 
@@ -42,7 +42,7 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 CFG1 = dict(nx=128, ny=128, nz=256, n_steps=3000)
-BYTES_PER_CELL = 56          # p^n..p^{n-4} 20 B, p^{n+1} 4, R 12, c 4, peak 8, energy 8
+BYTES_PER_CELL = 43.2        # p^n..p^{n-4} 20 B, p^{n+1} 4, R 12, c 4; peak 8 and energy 8 every fifth step
 METRIC = "Westervelt Gcell-updates/s"
 UNIT = "Gcell-updates/s"
 # dram__bytes_read.sum + dram__bytes_write.sum of one step-kernel launch on the
@@ -255,7 +255,7 @@ def run_westervelt(args, world, rank, local):
     achieved = BYTES_PER_CELL * ncell / (step_us * 1e-6) / 1e9
     roof = {"bound": "hbm", "achieved": achieved, "peak": pk["hbm_gbs"], "unit": "GB/s",
             "frac": achieved / pk["hbm_gbs"], "traffic": NCU_TRAFFIC_BYTES,
-            "algorithmic_bytes": BYTES_PER_CELL * ncell, "peak_kind": pk_kind}
+            "algorithmic_bytes": int(BYTES_PER_CELL * ncell), "peak_kind": pk_kind}
     # ---- end to end through the C ABI with host buffers
     prob = cfg1_problem(tile_variant=args.tile_variant)
     cmap = prob.array("c_map")
@@ -330,7 +330,7 @@ def adjoint_summary(ctx):
     return out
 
 
-HEAT_BYTES_PER_CELL = 28    # theta read + write 8 B, Q 4 B, FP64 dose read + write 16 B
+HEAT_BYTES_PER_CELL = 20    # theta read + write 8 B, Q 4 B, FP64 dose read + write 16 B every other step
 
 
 def cfg3_summary(ctx, n_spots=49):
@@ -384,12 +384,12 @@ def cfg5_summary(ctx, n_steps=12000, n_bubbles=1 << 18, t_end=0.1e-6):
     win_ms = s.last_ms()
     r = s.finish(want=("dft", "peak"))
     s.close()
-    # p ring 24 B + two relaxation processes 24 B + peak 8 B (no c map; the
-    # energy accumulator only inside the window, +8 B, with the DFT's 16 B per
-    # frequency on its planes)
-    b_cell = 56
+    # p ring 24 B + two relaxation processes 24 B + peak 8 B every fifth step (no c
+    # map; the energy accumulator only inside the window, and every fifth step there
+    # the DFT pass: 16 B per frequency and five levels on its planes)
+    b_cell = 48 + 8 / 5
     dft_cells = (p.dft_z_hi - p.dft_z_lo) * g.nx * g.ny
-    win_bytes = (b_cell + 8) * ncell + 16 * p.n_dft * dft_cells
+    win_bytes = (b_cell + 8 / 5) * ncell + (16 * p.n_dft + 20) / 5 * dft_cells
     win_us = win_ms * 1e3 / p.dft_len
     out = {"workload": "cfg5 512x512x768 FP32, %d steps, 9-frequency DFT over the last 10 us (530 steps) "
                        "on %d planes; %d bubbles driven by the local field for %g s" % (n_steps, p.dft_z_hi - p.dft_z_lo,

@@ -92,12 +92,14 @@ struct WvSession {
     PoolBuf step_base, flag, kconst, Qd;
     double tau_max = 0.0;
     double last_ms = 0.0;
-    cudaGraphExec_t graph[4] = {nullptr, nullptr, nullptr, nullptr};   // chunk graphs per accumulator mode (ACC_*)
-    int graph_variant[4] = {-1, -1, -1, -1};
+    // chunk graphs per accumulator mode (ACC_*), without and with the DFT passes
+    cudaGraphExec_t graph[6] = {};
+    int graph_variant[6] = {-1, -1, -1, -1, -1, -1};
+    int64_t graph_launches[6] = {};
     // tensor maps of the TMA variant in use (built per tile shape)
     int maps_tx = 0, maps_ty = 0;
     bool adj_fused = false;     // adjoint: one fused pass per backward step (FP32, nx % 4 == 0)
-    CUtensorMap mP0[5], mQ[5], mR[BD_MAX_RELAX][2], mC, mPeak, mEnergy, mMat, mDre, mDim;
+    CUtensorMap mP0[5], mQ[5], mR[BD_MAX_RELAX][2], mC, mPeak, mEnergy, mMat;
     bool mat_tile = false;      // the material map travels as a TMA tile (nx % 16 == 0)
     // segment view (TMA variants only): the pressure levels of the next step are
     // read from, and p^{n+1} written to, caller-chosen buffers instead of the ring
@@ -176,9 +178,6 @@ static WvArgs<real> make_args(WvSession& S, int64_t s) {
     a.dt = (real)g.dt;
     a.kxy180 = (real)(g.dt * g.dt / (g.dx * g.dx) / 180.0);
     a.kz180 = (real)(g.dt * g.dt / (g.dz * g.dz) / 180.0);
-    const double hxy = g.dt * g.dt / (g.dx * g.dx) / 180.0, hz = g.dt * g.dt / (g.dz * g.dz) / 180.0;
-    const double st[7] = {-980.0 * hxy - 490.0 * hz, 270.0 * hxy, -27.0 * hxy, 2.0 * hxy, 270.0 * hz, -27.0 * hz, 2.0 * hz};
-    for (int k = 0; k < 7; ++k) a.st[k] = (real)st[k];
     a.ke = (real)(S.p.energy_mode == BD_ENERGY_DPDT2 ? 0.25 / g.dt : g.dt);
     a.dt2 = (real)(g.dt * g.dt);
     a.dtdx = (real)(g.dt / g.dx);
@@ -271,11 +270,6 @@ static void build_maps(WvSession& S, int tx, int ty) {
     S.mEnergy = make_map(S, S.energy.p, f, tx, ty);
     if (S.has_cmap) S.mC = make_map(S, S.cmap.p, true, tx, ty);
     if (S.mat_tile) S.mMat = make_map(S, S.matmap.p, false, tx, ty, true);
-    if (f && S.n_dft > 0) {   // the DFT planes of every frequency stacked along z (L2 prefetch only)
-        const long long depth = (long long)S.n_dft * (S.dz_hi - S.dz_lo);
-        S.mDre = make_map(S, S.dre.p, true, tx, ty, false, depth);
-        S.mDim = make_map(S, S.dim.p, true, tx, ty, false, depth);
-    }
     S.maps_tx = tx;
     S.maps_ty = ty;
 }
@@ -342,15 +336,14 @@ static void step_maps(WvSession& S, int64_t s, int tx, int ty, TmaMaps& maps) {
     maps.energy = S.mEnergy;
     if (S.has_cmap) maps.cmap = S.mC;
     if (S.mat_tile) maps.mat = S.mMat;
-    if (S.prec == BD_F32 && S.n_dft > 0) { maps.dre = S.mDre; maps.dim = S.mDim; }
 }
 
 template <class real, int TX, int TY, int CPT, int ZU>
 static void launch_tma_t(WvSession& S, const WvArgs<real>& a, int64_t s, int koff, cudaStream_t st) {
     TmaMaps maps;
     step_maps(S, s, TX, TY, maps);
-    // FP32 kernels with 0, 1 or 2 relaxation processes are compiled for their count;
-    // FP64 and larger counts use the kernel that reads the count at run time
+    // kernels with 0, 1 or 2 relaxation processes are compiled for their count (FP64:
+    // without a c map); the others read the count at run time
     if (sizeof(real) == 4 && S.max_relax == 0) launch_tma_k<real, TX, TY, CPT, 0, ZU>(S, a, maps, koff, st);
     else if (sizeof(real) == 4 && S.max_relax == 1 && S.has_cmap && !S.has_matmap && !S.has_planemat)
         launch_tma_k<real, TX, TY, CPT, 1, ZU, 3>(S, a, maps, koff, st);   // one material, c map (cfg1)
@@ -360,27 +353,27 @@ static void launch_tma_t(WvSession& S, const WvArgs<real>& a, int64_t s, int kof
     else launch_tma_k<real, TX, TY, CPT, -1, ZU>(S, a, maps, koff, st);
 }
 
-// Accumulators step s adds to (the ACC_* modes of the paired kernel): all when
-// its DFT window is open, peak and energy when the energy window is, the peak
-// map only when just the peak window is, none outside every window.
+// Accumulators step s adds to besides the DFT (the ACC_* modes of the paired
+// kernel): peak and energy inside the energy window, the peak map only when just
+// the peak window is open, none outside both.  A mode serves every lower one.
 static int step_acc_mode(const WvSession& S, int64_t s) {
-    if (S.n_dft > 0 && s >= S.p.dft_start && s < S.p.dft_start + S.p.dft_len) return ACC_ALL;
     if (s >= S.p.energy_start && s < S.p.energy_end) return ACC_PE;
-    if (s >= S.p.peak_start && s < S.p.peak_end) return ACC_PEAK;
-    return ACC_NONE;
+    return s >= S.p.peak_start && s < S.p.peak_end ? ACC_PEAK : ACC_NONE;
 }
 
-static int acc_rank(int m) { return m == ACC_ALL ? 3 : m == ACC_PE ? 2 : m == ACC_PEAK ? 1 : 0; }
+static bool step_in_dft(const WvSession& S, int64_t s) {
+    return S.n_dft > 0 && s >= S.p.dft_start && s < S.p.dft_start + S.p.dft_len;
+}
 
-// The mode that serves every step of [s0, s0 + n): all > peak and energy > peak > none.
+// The mode that serves every step of [s0, s0 + n), + 3 if one is inside the DFT window.
 static int range_acc_mode(const WvSession& S, int64_t s0, int64_t n) {
     int m = ACC_NONE;
+    bool dft = false;
     for (int64_t s = s0; s < s0 + n; ++s) {
-        const int k = step_acc_mode(S, s);
-        if (acc_rank(k) > acc_rank(m)) m = k;
-        if (m == ACC_ALL) break;
+        m = std::max(m, step_acc_mode(S, s));
+        dft = dft || step_in_dft(S, s);
     }
-    return m;
+    return m + (dft ? 3 : 0);
 }
 
 // Two x cells per thread (FP32; variant_ok has been checked).
@@ -421,30 +414,44 @@ static void launch_step_t(WvSession& S, const WvArgs<real>& a, int koff, cudaStr
     BD_LAUNCHED(S.ctx);
 }
 
-// The Mur faces of a step (one kernel), after the stencil update.
-template <class real>
-static void launch_mur(WvSession& S, const WvArgs<real>& a, int koff, cudaStream_t st, int acc) {
-    const long long cx = a.mur_xp ? a.nx - a.L : a.nx, cy = a.mur_yp ? a.ny - a.L : a.ny;
-    const long long n = (a.mur_zm ? cx * cy * a.Lzm : 0) + (a.mur_zp ? cx * cy : 0) + (a.mur_xp ? cy * a.nz : 0) +
-                        (a.mur_yp ? (long long)a.nx * a.nz : 0);
-    if (n <= 0) return;
-    const unsigned groups = acc == ACC_ALL && a.n_dft > 0 ? 1 + (a.n_dft + MUR_FREQS - 1) / MUR_FREQS : 1;
-    const WvConst<real>* K = S.kconst.as<WvConst<real>>();
+// A kernel that may start its prologue before the kernel ahead of it has ended.
+template <class... P, class... A>
+static void launch_after(WvSession& S, void (*kern)(P...), long long threads, int block, cudaStream_t st, const A&... args) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((n + 127) / 128), 1, groups);
-    cfg.blockDim = dim3(128);
+    cfg.gridDim = dim3((unsigned)((threads + block - 1) / block));
+    cfg.blockDim = dim3(block);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = S.pdl ? 1 : 0;
-    BD_CUDA(cudaLaunchKernelEx(&cfg, wv_mur_kernel<real>, a, K, koff));
+    BD_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
     BD_LAUNCHED(S.ctx);
 }
 
+// The Mur faces of a step (one kernel), after the stencil update.
 template <class real>
-static void launch_step(WvSession& S, int variant, int64_t s, int koff, cudaStream_t st, int acc, int acc_n, int mur_acc) {
+static void launch_mur(WvSession& S, const WvArgs<real>& a, int koff, cudaStream_t st) {
+    const long long cx = a.mur_xp ? a.nx - a.L : a.nx, cy = a.mur_yp ? a.ny - a.L : a.ny;
+    const long long n = (a.mur_zm ? cx * cy * a.Lzm : 0) + (a.mur_zp ? cx * cy : 0) + (a.mur_xp ? cy * a.nz : 0) +
+                        (a.mur_yp ? (long long)a.nx * a.nz : 0);
+    if (n <= 0) return;
+    launch_after(S, wv_mur_kernel<real>, n, 128, st, a, S.kconst.as<WvConst<real>>(), koff);
+}
+
+// The DFT of step s and the n - 1 before it, after the step (and its Mur faces).
+template <class real>
+static void launch_dft(WvSession& S, int64_t s, int koff, int n, cudaStream_t st) {
+    WvArgs<real> a = make_args<real>(S, s);
+    a.acc_n = n;
+    constexpr int VEC = 16 / sizeof(real);
+    if (S.plane % VEC == 0) launch_after(S, wv_dft_kernel<real, VEC>, S.dcells / VEC, 256, st, a, koff);
+    else launch_after(S, wv_dft_kernel<real, 1>, S.dcells, 256, st, a, koff);
+}
+
+template <class real>
+static void launch_step(WvSession& S, int variant, int64_t s, int koff, cudaStream_t st, int acc, int acc_n) {
     WvArgs<real> a = make_args<real>(S, s);
     a.acc_n = acc_n;
     const Variant& v = kVariants[variant];
@@ -469,7 +476,7 @@ static void launch_step(WvSession& S, int variant, int64_t s, int koff, cudaStre
         case 15: launch_tma_t<real, 32, 8, 1, 1>(S, a, s, koff, st); break;
         default: fail(BD_ERR_INVALID_ARG, "bad tile variant %d", variant);
     }
-    if (S.any_mur) launch_mur<real>(S, a, koff, st, mur_acc);   // its cells accumulate every step
+    if (S.any_mur) launch_mur<real>(S, a, koff, st);   // its cells accumulate peak and energy every step
 }
 
 // Whether the two-cell kernel accumulates in step s for itself and the steps since
@@ -482,27 +489,35 @@ static bool acc_due(const WvSession& S, int64_t s) {
 
 // Issue steps [s, s+n) on the stream (no graph): kernels read *step_base + koff,
 // then one advance kernel moves the counter by n.  The two-cell kernel accumulates
-// several steps at a time; the last step issued leaves nothing pending.  acc < 0:
-// the accumulating steps take the kernel that touches only the accumulators their
-// steps need (step_acc_mode); an ACC_* mode forces that one (a captured chunk).
-static void issue_steps(WvSession& S, int variant, int64_t s, int n, cudaStream_t st, int acc = -1) {
-    int pending = 0, mode = ACC_NONE;
+// several steps at a time, the DFT pass takes every fifth step; the last step issued
+// leaves nothing pending.  mode < 0: the accumulating steps take the kernel that
+// touches only the accumulators their steps need (step_acc_mode); a mode of
+// range_acc_mode forces that one (a captured chunk).
+static void issue_steps(WvSession& S, int variant, int64_t s, int n, cudaStream_t st, int mode = -1) {
+    int pending = 0, acc = ACC_NONE, dft_n = 0;
+    bool dft = false;
     for (int k = 0; k < n; ++k) {
-        const int own = acc >= 0 ? acc : step_acc_mode(S, s + k);
-        if (acc_rank(own) > acc_rank(mode)) mode = own;
+        acc = std::max(acc, mode >= 0 ? mode % 3 : step_acc_mode(S, s + k));
         ++pending;
         const bool now = !kVariants[variant].pair || k == n - 1 || acc_due(S, s + k);
-        const int m = now ? mode : ACC_NONE;
-        if (S.prec == BD_F32) launch_step<float>(S, variant, s + k, k, st, m, now ? pending : 0, own);
-        else launch_step<double>(S, variant, s + k, k, st, m, now ? pending : 0, own);
-        if (now) { pending = 0; mode = ACC_NONE; }
+        if (S.prec == BD_F32) launch_step<float>(S, variant, s + k, k, st, now ? acc : ACC_NONE, now ? pending : 0);
+        else launch_step<double>(S, variant, s + k, k, st, now ? acc : ACC_NONE, now ? pending : 0);
+        if (now) { pending = 0; acc = ACC_NONE; }
+        dft = dft || (mode >= 0 ? mode >= 3 : step_in_dft(S, s + k));
+        ++dft_n;
+        if (k == n - 1 || (s + k) % ACC_STEPS == ACC_STEPS - 1) {
+            if (dft && S.prec == BD_F32) launch_dft<float>(S, s + k, k, dft_n, st);
+            else if (dft) launch_dft<double>(S, s + k, k, dft_n, st);
+            dft_n = 0;
+            dft = false;
+        }
     }
     wv_advance_kernel<<<1, 32, 0, st>>>(S.step_base.as<long long>(), n);
     BD_LAUNCHED(S.ctx);
 }
 
-static void build_graph(WvSession& S, int acc) {
-    cudaGraphExec_t& G = S.graph[acc];
+static void build_graph(WvSession& S, int mode) {
+    cudaGraphExec_t& G = S.graph[mode];
     if (G) { cudaGraphExecDestroy(G); G = nullptr; }
     cudaStream_t cs;
     BD_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
@@ -510,7 +525,7 @@ static void build_graph(WvSession& S, int acc) {
     const int64_t launches_before = S.ctx->launches;
     BD_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
     try {
-        issue_steps(S, S.variant, 0, S.chunk, cs, acc);   // base arrangement: chunk starts at s = 0 mod 10
+        issue_steps(S, S.variant, 0, S.chunk, cs, mode);   // base arrangement: chunk starts at s = 0 mod 10
     } catch (...) {
         cudaStreamEndCapture(cs, &g);
         if (g) cudaGraphDestroy(g);
@@ -518,12 +533,13 @@ static void build_graph(WvSession& S, int acc) {
         throw;
     }
     BD_CUDA(cudaStreamEndCapture(cs, &g));
+    S.graph_launches[mode] = S.ctx->launches - launches_before;
     S.ctx->launches = launches_before;   // captured, not yet launched
     const cudaError_t e = cudaGraphInstantiate(&G, g, 0);
     cudaGraphDestroy(g);
     cudaStreamDestroy(cs);
     BD_CUDA(e);
-    S.graph_variant[acc] = S.variant;
+    S.graph_variant[mode] = S.variant;
 }
 
 static int64_t launches_per_step(const WvSession& S) { return S.any_mur ? 2 : 1; }
@@ -551,7 +567,6 @@ static void advance(WvSession& S, int64_t n, bool use_graph) {
     const int64_t fault = S.p.fault_at_step;
     bool faulted = false;
     if (fault >= 0 && fault >= S.step && fault < end) { end = fault; faulted = true; }
-    const int64_t per = launches_per_step(S) + 0;
     int64_t next_probe = S.p.check_every > 0 ? ((S.step / S.p.check_every) + 1) * S.p.check_every : INT64_MAX;
     while (S.step < end) {
         int64_t todo = end - S.step;
@@ -561,7 +576,7 @@ static void advance(WvSession& S, int64_t n, bool use_graph) {
             const int m = range_acc_mode(S, S.step, S.chunk);
             if (!S.graph[m] || S.graph_variant[m] != S.variant) build_graph(S, m);
             BD_CUDA(cudaGraphLaunch(S.graph[m], st));
-            S.ctx->launches += per * S.chunk + 1;
+            S.ctx->launches += S.graph_launches[m];
             take = S.chunk;
         } else {
             take = std::min<int64_t>(todo, to_align > 0 ? to_align : S.chunk);

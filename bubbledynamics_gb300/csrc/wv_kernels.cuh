@@ -33,7 +33,6 @@ struct MatConst {
     real kxy, kz, kd, kn, kr;  // stencil xy and z, diffusivity, nonlinearity, (c dt)^2
     real xr;                   // x / (1 - x), x = 3 kr sum a (semi-implicit relaxation)
     real av[BD_MAX_RELAX];     // a_v
-    real st[sizeof(real) == 8 ? 7 : 1];   // FP64: (c dt / d)^2 times the stencil weights (WvArgs::st)
 };
 
 template <class real>
@@ -47,7 +46,7 @@ struct WvArgs {
     int zb;                    // z-chunk per CTA
     int px;                    // row pitch in cells
     int rev;                   // two-cell kernel: march from the high end
-    int acc_n;                 // two-cell kernel: steps this one accumulates (itself and acc_n - 1 before it)
+    int acc_n;                 // two-cell and DFT kernels: steps this one accumulates (itself and acc_n - 1 before it)
     long long plane;           // px*ny
     // time levels: p^n (stencil), p^{n-1..n-3}, and the p^{n-4} buffer that receives p^{n+1}
     const real* __restrict__ p0;
@@ -100,7 +99,6 @@ struct WvArgs {
     const real* __restrict__ tw;               // DFT twiddles [dft step][n_dft][2]
     long long peak_start, peak_end, energy_start, energy_end, dft_start, dft_len;
     real ke;                   // FP64: weight of p^2 (dt) or of (p^{n+1} - p^{n-1})^2 (1 / 4dt) in the energy
-    real st[7];                // FP64: stencil weights over d^2: p; the +-1, +-2, +-3 rings in x and y; the same in z
     int energy_mode, n_dft, dz_lo, dz_hi;
     int relax_scheme;
     int mat_tile;              // 1: the two-cell kernel receives the material map as a TMA tile per plane
@@ -189,24 +187,11 @@ __device__ __forceinline__ real energy_add(const WvArgs<real>& a, real old, real
     return add_(old, e);
 }
 
-// Peak / energy / DFT accumulation on the final p^{n+1} of a cell.
+// Peak / energy accumulation on the final p^{n+1} of a cell.
 template <class real>
-__device__ __forceinline__ void accumulate(const WvArgs<real>& a, long long step, long long i, int ix, int iy,
-                                           int iz, real v, real vm1) {
-    if (step >= a.peak_start && step < a.peak_end) {
-        a.peak[i] = peak_max(v, a.peak[i]);
-    }
+__device__ __forceinline__ void accumulate(const WvArgs<real>& a, long long step, long long i, real v, real vm1) {
+    if (step >= a.peak_start && step < a.peak_end) a.peak[i] = peak_max(v, a.peak[i]);
     if (step >= a.energy_start && step < a.energy_end) a.energy[i] = energy_add(a, a.energy[i], v, vm1);
-    const long long ds = step - a.dft_start;
-    if (a.n_dft > 0 && ds >= 0 && ds < a.dft_len && iz >= a.dz_lo && iz < a.dz_hi) {
-        const long long pl = (long long)(iz - a.dz_lo) * a.plane + (long long)iy * a.px + ix;
-        const long long stride = (long long)(a.dz_hi - a.dz_lo) * a.plane;
-        const real* tw = a.tw + ds * a.n_dft * 2;
-        for (int j = 0; j < a.n_dft; ++j) {
-            a.dre[j * stride + pl] = fma_(v, tw[2 * j], a.dre[j * stride + pl]);
-            a.dim[j * stride + pl] = fma_(-v, tw[2 * j + 1], a.dim[j * stride + pl]);
-        }
-    }
 }
 
 template <class real>
@@ -233,13 +218,8 @@ __device__ __forceinline__ void cell_coef(const WvArgs<real>& a, MatConst<real>&
     const real c2 = mul_(c, c);
     const real ic = div_(real(1), c);
     const real ic2 = mul_(ic, ic);
-    if constexpr (sizeof(real) == 8) {
-#pragma unroll
-        for (int k = 0; k < 7; ++k) M.st[k] = mul_(c2, a.st[k]);
-    } else {
-        M.kxy = mul_(c2, a.kxy180);
-        M.kz = mul_(c2, a.kz180);
-    }
+    M.kxy = mul_(c2, a.kxy180);
+    M.kz = mul_(c2, a.kz180);
     M.kd = mul_(M.delta_2dt, ic2);
     M.kn = mul_(M.beta2_rho, ic2);
     M.kr = mul_(c2, a.dt2);
@@ -293,24 +273,19 @@ __device__ __forceinline__ real cell_update(const WvArgs<real>& a, const MatCons
     // cells per wavelength) and p^{n+1} takes one final rounding: the FP32 field
     // error against FP64 after 3000 cfg1 steps drops from 1.04e-5 to 8.4e-6
     // (summing 2p - p1 + ... directly rounds at the size of p five times).
-    // FP64 is bound by its FP64 instructions: there the weights carry (c dt / d)^2 and
-    // the x and y rings add up first, 19 instructions instead of 24 (and the
-    // relaxation terms go straight into V; 64 x 64 x 201, two processes: 199.8 -> 188.0 us a
-    // step).
+    // FP64 is bound by its FP64 instructions: there the x and y rings add up before
+    // they are weighted (two instructions fewer) and the relaxation terms go straight
+    // into V.  Weights that carry kxy and kz save three more (64 x 64 x 201, two
+    // processes: 139 us a step instead of 146), but no longer cancel exactly: five
+    // times the error after 600 steps.
     real V = add_(pc, -q1);
     const real sz1 = add_(w[4], w[2]), sz2 = add_(w[5], w[1]), sz3 = add_(w[6], w[0]);
-    if constexpr (sizeof(real) == 8) {
-        V = fma_(M.st[0], pc, V);
-        V = fma_(M.st[1], add_(sx1, sy1), V);
-        V = fma_(M.st[2], add_(sx2, sy2), V);
-        V = fma_(M.st[3], add_(sx3, sy3), V);
-        V = fma_(M.st[4], sz1, V);
-        V = fma_(M.st[5], sz2, V);
-        V = fma_(M.st[6], sz3, V);
-    } else {
-        V = fma_(M.kxy, add_(d2x180(pc, sx1, sx2, sx3), d2x180(pc, sy1, sy2, sy3)), V);
-        V = fma_(M.kz, d2x180(pc, sz1, sz2, sz3), V);
-    }
+    real Dxy;
+    if constexpr (sizeof(real) == 8)
+        Dxy = fma_(real(2), add_(sx3, sy3), fma_(real(-27), add_(sx2, sy2), fma_(real(270), add_(sx1, sy1), mul_(real(-980), pc))));
+    else Dxy = add_(d2x180(pc, sx1, sx2, sx3), d2x180(pc, sy1, sy2, sy3));
+    V = fma_(M.kxy, Dxy, V);
+    V = fma_(M.kz, d2x180(pc, sz1, sz2, sz3), V);
     V = fma_(M.kd, Dttt, V);
     V = fma_(M.kn, add_(D1, D2), V);
     real pn;
@@ -437,7 +412,7 @@ __global__ void __launch_bounds__(TX* TY) wv_step_kernel(const WvArgs<real> a, c
         if (have) {
             const real vm1 = (a.energy_mode == BD_ENERGY_DPDT2) ? ld(a.p1 + i) : real(0);
             a.p4[i] = pn;
-            if (!mur) accumulate(a, step, i, ix, iy, iz, pn, vm1);
+            if (!mur) accumulate(a, step, i, pn, vm1);
         }
 #pragma unroll
         for (int k = 0; k < 6; ++k) w[k] = w[k + 1];
@@ -457,8 +432,11 @@ __device__ __forceinline__ real mur_cell(real pj, real nb, real pi, real c, real
     return pj + (nb - pi) * mur_k(c, dth);
 }
 
+// steps the two-cell kernel and the DFT pass accumulate at once, at most: their
+// pressures are p^{n+1}..p^{n-3}; the (dp/dt)^2 energy of a step also needs the level
+// two before its own, so it stops at four
+constexpr int ACC_STEPS = 5, ACC_DPDT = 4;
 constexpr int MUR_MAXL = 8;    // layers of an x+, y+ or z+ face
-constexpr int MUR_FREQS = 2;   // DFT frequencies per block of the Mur kernel's DFT groups
 
 // The Mur faces of a step in one pass, in the order z-, z+, x+, y+ of a serial
 // launch of W:88-135.  Every cell's value follows from P^n and from the cells the
@@ -466,12 +444,7 @@ constexpr int MUR_FREQS = 2;   // DFT frequencies per block of the Mur kernel's 
 // layers (or one z- cell, whose neighbour is P^n or the source plane) and, where
 // the run starts on a cell that an earlier face overwrites, forms that cell's
 // value itself.  Three kernels, one per face, whose threads re-read each layer
-// they had just written took 26 us a step on 107 x 107 x 401 cells outside the DFT
-// window and several times that inside it (FP64 64 x 64 x 201, 600 steps, 400 of
-// them in the window: the solve went from 173 to 140 ms).
-// In the DFT window blocks with blockIdx.z > 0 form the same values again and
-// add them to MUR_FREQS frequencies each (one thread adding ten frequencies in
-// turn waited for twenty dependent round trips a layer).
+// they had just written took 26 us a step on 107 x 107 x 401 cells; this one 10.4.
 template <class real>
 __global__ void __launch_bounds__(128) wv_mur_kernel(const WvArgs<real> a, const WvConst<real>* __restrict__ Kp, int koff) {
     const WvConst<real>& K = *Kp;
@@ -561,45 +534,91 @@ __global__ void __launch_bounds__(128) wv_mur_kernel(const WvArgs<real> a, const
             pj = pi;
         }
     } else nl = 1;
-    if (blockIdx.z == 0) {
-        const bool do_peak = step >= a.peak_start && step < a.peak_end;
-        const bool do_energy = step >= a.energy_start && step < a.energy_end;
+    const bool do_peak = step >= a.peak_start && step < a.peak_end;
+    const bool do_energy = step >= a.energy_start && step < a.energy_end;
 #pragma unroll
-        for (int l = 0; l < MUR_MAXL; ++l) {
-            if (l >= nl) break;
-            const long long i = i0 + l * st;
-            F[i] = v[l];
-            if (do_peak) a.peak[i] = peak_max(v[l], a.peak[i]);
-            if (do_energy) a.energy[i] = energy_add(a, a.energy[i], v[l], a.energy_mode == BD_ENERGY_DPDT2 ? a.p1[i] : real(0));
-        }
-        return;
+    for (int l = 0; l < MUR_MAXL; ++l) {
+        if (l >= nl) break;
+        const long long i = i0 + l * st;
+        F[i] = v[l];
+        if (do_peak) a.peak[i] = peak_max(v[l], a.peak[i]);
+        if (do_energy) a.energy[i] = energy_add(a, a.energy[i], v[l], a.energy_mode == BD_ENERGY_DPDT2 ? a.p1[i] : real(0));
     }
-    const long long ds = step - a.dft_start;
-    if (ds < 0 || ds >= a.dft_len) return;
-    const long long stride = (long long)(a.dz_hi - a.dz_lo) * a.plane, off = (long long)a.dz_lo * a.plane;
-    const int j0 = (blockIdx.z - 1) * MUR_FREQS;
-    const real* tw = a.tw + ds * a.n_dft * 2;
+}
+
+template <class real, int VEC>
+struct alignas(VEC * sizeof(real)) Cells {
+    real v[VEC];
+};
+
+// The DFT accumulators of this step and the a.acc_n - 1 before it, whose pressures
+// are still in the ring, oldest first: one stream over the DFT planes, 8 B (FP32) a
+// frequency and cell read and as much written, 20 B of pressures.  Inside the step
+// kernels the accumulators took registers and waited for their loads between two
+// barriers, and the Mur faces added theirs one cell at a time.  FP32 107 x 107 x
+// 401, ten frequencies on 347 planes: a step that accumulated took 253 us instead of
+// 62, one in three or four, and the Mur faces 38 instead of 11 in every step; this
+// pass takes 102 us (the copy bandwidth) every fifth.  FP64 is bound by its two FMAs a
+// frequency, step and cell.  Cells that no step updates hold zeros and add zeros.
+// VEC cells a thread; the twiddles sit in shared memory.
+template <class real, int VEC>
+__global__ void __launch_bounds__(256) wv_dft_kernel(const WvArgs<real> a, int koff) {
+    __shared__ real tw[ACC_STEPS][BD_MAX_DFT][2];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const long long ds = *a.step_base + koff - a.dft_start;
+    unsigned mask = 0;                              // bit m: step - m is inside the window
 #pragma unroll
-    for (int u = 0; u < MUR_FREQS; ++u) {
-        const int j = j0 + u;
-        if (j >= a.n_dft) break;
-        real* dr = a.dre + j * stride - off;
-        real* di = a.dim + j * stride - off;
-        const real tr = tw[2 * j], ti = tw[2 * j + 1];
-        real r[MUR_MAXL], m[MUR_MAXL];
+    for (int m = 0; m < ACC_STEPS; ++m)
+        if (m < a.acc_n && ds - m >= 0 && ds - m < a.dft_len) mask |= 1u << m;
+    if (mask == 0) return;
+    for (int e = threadIdx.x; e < ACC_STEPS * a.n_dft; e += blockDim.x) {
+        const int m = e / a.n_dft, j = e - m * a.n_dft;
+        if (!(mask >> m & 1u)) continue;
+        const real* t = a.tw + ((ds - m) * a.n_dft + j) * 2;
+        tw[m][j][0] = t[0];
+        tw[m][j][1] = t[1];
+    }
+    __syncthreads();
+    const long long n = (long long)(a.dz_hi - a.dz_lo) * a.plane;
+    const long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) * VEC;
+    if (i >= n) return;
+    const real* const lev[ACC_STEPS] = {a.p4, a.p0, a.p1, a.p2, a.p3};   // p^{n+1} (written by the step), p^n, ...
+    using Vec = Cells<real, VEC>;
+    auto at = [](const real* p) { return *reinterpret_cast<const Vec*>(p); };
+    Vec x[ACC_STEPS];
 #pragma unroll
-        for (int l = 0; l < MUR_MAXL; ++l) {        // every load before any store
-            const int z = iz + l * dzl;
-            if (l < nl && z >= a.dz_lo && z < a.dz_hi) { r[l] = dr[i0 + l * st]; m[l] = di[i0 + l * st]; }
-        }
+    for (int m = 0; m < ACC_STEPS; ++m)
+        if (mask >> m & 1u) x[m] = at(lev[m] + a.dz_lo * a.plane + i);
+    constexpr int G = 4;                            // frequencies whose loads are issued together
+    for (int j = 0; j < a.n_dft; j += G) {
+        Vec r[G], q[G];
 #pragma unroll
-        for (int l = 0; l < MUR_MAXL; ++l) {
-            const int z = iz + l * dzl;
-            if (l < nl && z >= a.dz_lo && z < a.dz_hi) {
-                dr[i0 + l * st] = fma_(v[l], tr, r[l]);
-                di[i0 + l * st] = fma_(-v[l], ti, m[l]);
+        for (int u = 0; u < G; ++u)
+            if (j + u < a.n_dft) {
+                r[u] = at(a.dre + (j + u) * n + i);
+                q[u] = at(a.dim + (j + u) * n + i);
             }
+#pragma unroll
+        for (int m = ACC_STEPS - 1; m >= 0; --m) {
+            if (!(mask >> m & 1u)) continue;
+#pragma unroll
+            for (int u = 0; u < G; ++u)
+                if (j + u < a.n_dft) {
+                    const real c = tw[m][j + u][0], s = tw[m][j + u][1];
+#pragma unroll
+                    for (int k = 0; k < VEC; ++k) {
+                        r[u].v[k] = fma_(x[m].v[k], c, r[u].v[k]);
+                        q[u].v[k] = fma_(-x[m].v[k], s, q[u].v[k]);
+                    }
+                }
         }
+#pragma unroll
+        for (int u = 0; u < G; ++u)
+            if (j + u < a.n_dft) {
+                *reinterpret_cast<Vec*>(a.dre + (j + u) * n + i) = r[u];
+                *reinterpret_cast<Vec*>(a.dim + (j + u) * n + i) = q[u];
+            }
     }
 }
 

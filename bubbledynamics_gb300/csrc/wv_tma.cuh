@@ -24,14 +24,10 @@
 namespace bd {
 
 constexpr int TMA_NP = 8;   // p^n plane slots (>= 7)
-// accumulator modes of the paired step kernel: all (peak, energy and the DFT),
-// none, the peak map only, peak and energy without the DFT
-constexpr int ACC_ALL = 0, ACC_NONE = 1, ACC_PEAK = 2, ACC_PE = 3;
+// accumulator modes of the paired step kernel: none, the peak map only, peak and
+// energy (the DFT has a pass of its own)
+constexpr int ACC_NONE = 0, ACC_PEAK = 1, ACC_PE = 2;
 constexpr int TMA_NQ = 3;   // pointwise slots
-// steps the two-cell kernel accumulates at once, at most: their pressures are
-// p^{n+1}..p^{n-3}; the (dp/dt)^2 energy of a step also needs the level two before
-// its own, so it stops at four
-constexpr int ACC_STEPS = 5, ACC_DPDT = 4;
 constexpr int FL_NOC = 4;   // kernel flags: no c map, materials by plane or cell
 
 struct TmaMaps {
@@ -41,7 +37,7 @@ struct TmaMaps {
     CUtensorMap ro[BD_MAX_RELAX];       // R^{n-2}
     CUtensorMap cmap, peak, energy;
     CUtensorMap mat;                    // box (TX, TY, 1) on the per-cell material map (uint8), when staged
-    CUtensorMap dre, dim;               // box (TX, TY, 1) on the DFT accumulators as (nx, ny, n_dft x planes)
+
 };
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) {
@@ -108,14 +104,6 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, u
         "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
         ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
         : "memory");
-}
-
-// Prefetch of one tile into L2 (no shared memory, no barrier): a hint for the
-// loads that follow.
-__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* map, int x, int y, int z) {
-    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];"
-                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z)
-                 : "memory");
 }
 
 // Shared-memory layout.  NRMAX is the number of relaxation processes the slot
@@ -253,8 +241,6 @@ __global__ void __launch_bounds__(TX* TY / CPT) wv_tma_kernel(const WvArgs<real>
     const bool fix_x = a.mir_x && x0 == 0, fix_y = a.mir_y && y0 == 0;
     const bool do_peak = step >= a.peak_start && step < a.peak_end;
     const bool do_energy = step >= a.energy_start && step < a.energy_end;
-    const long long ds = step - a.dft_start;
-    const bool do_dft = a.n_dft > 0 && ds >= 0 && ds < a.dft_len;
     const bool single_mat = FL >= 0 && FL != FL_NOC ? (FL & 1) != 0 : (!a.matmap && !a.plane_mat);
     // the material of single-material problems, in registers
     const MatConst<real> M0 = sK[0];
@@ -362,29 +348,6 @@ __global__ void __launch_bounds__(TX* TY / CPT) wv_tma_kernel(const WvArgs<real>
                 if (!(murz || murxy[c])) {
                     if (do_peak) pkz[col[c]] = peak_max(pn, pkt[k]);
                     if (do_energy) enz[col[c]] = energy_add(a, ent[k], pn, q1);
-                    if (do_dft && iz >= a.dz_lo && iz < a.dz_hi) {
-                        const long long pl = (long long)(iz - a.dz_lo) * a.plane + col[c];
-                        const long long stride = (long long)(a.dz_hi - a.dz_lo) * a.plane;
-                        const real* tw = a.tw + ds * a.n_dft * 2;
-                        real* dr = a.dre + pl;
-                        real* di = a.dim + pl;
-                        int j = 0;
-                        // four frequencies at a time: their eight loads are issued before any store
-                        for (; j + 4 <= a.n_dft; j += 4) {
-                            real r[4], m[4];
-#pragma unroll
-                            for (int u = 0; u < 4; ++u) { r[u] = dr[(j + u) * stride]; m[u] = di[(j + u) * stride]; }
-#pragma unroll
-                            for (int u = 0; u < 4; ++u) {
-                                dr[(j + u) * stride] = fma_(pn, tw[2 * (j + u)], r[u]);
-                                di[(j + u) * stride] = fma_(-pn, tw[2 * (j + u) + 1], m[u]);
-                            }
-                        }
-                        for (; j < a.n_dft; ++j) {
-                            dr[j * stride] = fma_(pn, tw[2 * j], dr[j * stride]);
-                            di[j * stride] = fma_(-pn, tw[2 * j + 1], di[j * stride]);
-                        }
-                    }
                 }
             }
         }

@@ -120,16 +120,13 @@ __device__ __forceinline__ F2 cell_update2(const WvArgs<float>& a, const Coef2<N
 // for 24 resident warps per SM (at most 85 registers a thread).  The cell update is
 // cell_update(), so the results are the plain kernel's bits.
 //
-// ACC: which accumulators the step may touch.  ACC_ALL: peak, energy and DFT
-// (each still gated by its window); ACC_PE: peak and energy (a step outside the
-// DFT window: no DFT code, so fewer registers); ACC_PEAK: only the peak map (a
-// step outside the energy and DFT windows: the energy tile is not loaded, 4 B
-// less per cell); ACC_NONE: none (outside every window, e.g. the recompute of
-// the adjoint: neither tile is loaded, 8 B less per cell).  Planes on which
+// ACC: which accumulators the step may touch.  ACC_PE: peak and energy (each still
+// gated by its window); ACC_PEAK: only the peak map (the energy tile is not loaded,
+// 4 B less per cell); ACC_NONE: none (outside the windows, or a step that a later
+// one accumulates for: neither tile is loaded, 8 B less per cell).  Planes on which
 // every cell of the tile is updated take a copy of the cell code without the
-// per-cell conditions, except in ACC_ALL, where the larger DFT code of that
-// copy would cost registers (and spills) in the whole kernel.
-template <int TX, int TY, int NREL, int ZU, int FL, int NQ, int ACC = ACC_ALL>
+// per-cell conditions.
+template <int TX, int TY, int NREL, int ZU, int FL, int NQ, int ACC = ACC_PE>
 __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kernel(const WvArgs<float> a,
                                                                  const WvConst<float>* __restrict__ Kp, int koff,
                                                                  const __grid_constant__ TmaMaps maps,
@@ -182,23 +179,12 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
         mbar_expect_tx(bar, L::PW * L::PH * (unsigned)sizeof(real));
         tma_load_3d(pslot(q), &maps.p0, bar, x0 - 4, y0 - 3, plane);
     };
-    // steps inside the DFT window: the producer also asks L2 for the plane's
-    // accumulator tiles when it issues the plane's pointwise tiles, so the
-    // accumulators' read-modify-writes find them there (set once the step is known)
-    bool pf_dft = false;
     auto issueQ = [&](int r) {
         if (r >= zbn) return;
         const int plane = zof(r);
-        if (pf_dft && plane >= a.dz_lo && plane < a.dz_hi) {
-            const int ndz = a.dz_hi - a.dz_lo;
-            for (int j = 0; j < a.n_dft; ++j) {
-                tma_prefetch_3d(&maps.dre, x0, y0, j * ndz + plane - a.dz_lo);
-                tma_prefetch_3d(&maps.dim, x0, y0, j * ndz + plane - a.dz_lo);
-            }
-        }
         uint64_t* bar = &barQ[r % NQ];
         unsigned char* q = qslot(r);
-        constexpr int acc_tiles = ACC == ACC_ALL || ACC == ACC_PE ? 2 : ACC == ACC_PEAK ? 1 : 0;
+        constexpr int acc_tiles = ACC == ACC_PE ? 2 : ACC == ACC_PEAK ? 1 : 0;
         mbar_expect_tx(bar, (unsigned)((4 + acc_tiles + 2 * nrel) * L::QTB + (has_c ? L::QTF : 0) +
                                        (a.mat_tile ? L::QT : 0)));
         for (int k = 0; k < 4; ++k) tma_load_3d(q + k * L::QTB, &maps.q[k], bar, x0, y0, plane);
@@ -207,7 +193,7 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
             tma_load_3d(q + (4 + NRMAX + v) * L::QTB, &maps.ro[v], bar, x0, y0, plane);
         }
         if constexpr (ACC != ACC_NONE) tma_load_3d(q + L::K_PEAK * L::QTB, &maps.peak, bar, x0, y0, plane);
-        if constexpr (ACC == ACC_ALL || ACC == ACC_PE)
+        if constexpr (ACC == ACC_PE)
             tma_load_3d(q + L::K_ENERGY * L::QTB, &maps.energy, bar, x0, y0, plane);
         if (has_c) tma_load_3d(q + L::NQR * L::QTB, &maps.cmap, bar, x0, y0, plane);
         if (a.mat_tile) tma_load_3d(q + L::NQR * L::QTB + L::QTF, &maps.mat, bar, x0, y0, plane);
@@ -225,8 +211,6 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
     // read only after this wait (a no-op for an ordinary launch).
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const long long step = *a.step_base + koff;
-    if constexpr (ACC == ACC_ALL && sizeof(real) == 4)
-        pf_dft = a.n_dft > 0 && step >= a.dft_start && step - a.acc_n + 1 < a.dft_start + a.dft_len;
     if (tid == 0) {
         for (int q = 0; q < TMA_NP; ++q) issueP(q);
         for (int r = 0; r < NQ; ++r) issueQ(r);
@@ -257,24 +241,19 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
     // every cell of the tile inside the grid and the update box and on no x / y
     // Mur layer: the planes of the tile inside the z range take the code without
     // per-cell conditions (the same operations on every cell, so the same bits)
-    bool tile_fast = false;
-    if constexpr (ACC != ACC_ALL) {
-        const bool mine = active[0] && active[1] && inbox[0] && inbox[1] && !murxy[0] && !murxy[1];
-        tile_fast = __syncthreads_and(mine) != 0;      // also: the slots of the three planes before the first are free again
-    } else {
-        __syncthreads();                               // the slots of the three planes before the first are free again
-    }
+    const bool mine = active[0] && active[1] && inbox[0] && inbox[1] && !murxy[0] && !murxy[1];
+    const bool tile_fast = __syncthreads_and(mine) != 0;   // also: the slots of the three planes before the first are free again
     if (tid == 0)
         for (int q = TMA_NP; q < TMA_NP + 3; ++q) issueP(q);
 
     const bool fix_x = a.mir_x && x0 == 0, fix_y = a.mir_y && y0 == 0;
-    // Deferred accumulation: a step's peak, energy and DFT terms follow from its
+    // Deferred accumulation: a step's peak and energy terms follow from its
     // pressure alone, which stays in the ring, so one step in four or five adds its
     // own terms and those of the steps since the last such step, oldest first (the
     // same operations on every accumulator, so the same bits), and the steps between
     // leave the accumulators alone.  Bit m: step - m is inside the window.
     const int acc_n = ACC == ACC_NONE ? 0 : a.acc_n;
-    unsigned peak_m = 0, energy_m = 0, dft_m = 0;
+    unsigned peak_m = 0, energy_m = 0;
     if constexpr (ACC != ACC_NONE) {
 #pragma unroll
         for (int m = 0; m < ACC_STEPS; ++m) {
@@ -282,13 +261,10 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
             if (m >= acc_n) continue;
             if (t >= a.peak_start && t < a.peak_end) peak_m |= 1u << m;
             if (t >= a.energy_start && t < a.energy_end) energy_m |= 1u << m;
-            if (a.n_dft > 0 && t >= a.dft_start && t < a.dft_start + a.dft_len) dft_m |= 1u << m;
         }
     }
     const bool do_peak = peak_m != 0;
-    const bool do_energy = (ACC == ACC_ALL || ACC == ACC_PE) && energy_m != 0;
-    const bool do_dft = ACC == ACC_ALL && dft_m != 0;
-    const long long ds = step - a.dft_start;
+    const bool do_energy = ACC == ACC_PE && energy_m != 0;
     const bool single_mat = FL >= 0 && FL != FL_NOC ? (FL & 1) != 0 : (!a.matmap && !a.plane_mat);
     const bool dpdt = a.energy_mode == BD_ENERGY_DPDT2;
 
@@ -463,64 +439,11 @@ __global__ void __launch_bounds__(TX* TY / 2, 1536 / (TX * TY)) wv_tma_pair_kern
                     if (acc[1]) enz[col + 1] = e1;
                 }
             }
-            if (do_dft && iz >= a.dz_lo && iz < a.dz_hi) {
-                const long long pl = (long long)(iz - a.dz_lo) * a.plane + col;
-                const long long stride = (long long)(a.dz_hi - a.dz_lo) * a.plane;
-                const real* tw = a.tw + ds * a.n_dft * 2;
-                real* dr = a.dre + pl;
-                real* di = a.dim + pl;
-                auto add = [&](F2& r, F2& i, int j) {
-#pragma unroll
-                    for (int m = ACC_STEPS - 1; m >= 0; --m) {
-                        if (!(dft_m >> m & 1u)) continue;
-                        const float2 t = __ldg(reinterpret_cast<const float2*>(tw + 2 * (j - m * a.n_dft)));
-                        r = f2_fma(lev[m], f2(t.x), r);
-                        i = f2_fma(lev[m], f2(-t.y), i);
-                    }
-                };
-                if (acc_pair) {
-                    // both cells accumulate: one pair load and store per accumulator, the
-                    // loads of four frequencies before any store
-                    int j = 0;
-                    for (; j + 4 <= a.n_dft; j += 4) {
-                        F2 r[4], i[4];
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) { r[u] = ld2(dr + (j + u) * stride); i[u] = ld2(di + (j + u) * stride); }
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            add(r[u], i[u], j + u);
-                            st2(dr + (j + u) * stride, r[u]);
-                            st2(di + (j + u) * stride, i[u]);
-                        }
-                    }
-                    for (; j < a.n_dft; ++j) {
-                        F2 r = ld2(dr + j * stride), i = ld2(di + j * stride);
-                        add(r, i, j);
-                        st2(dr + j * stride, r);
-                        st2(di + j * stride, i);
-                    }
-                } else if (acc[0] || acc[1]) {
-                    for (int j = 0; j < a.n_dft; ++j) {
-                        real *pr = dr + j * stride, *pi = di + j * stride;
-                        F2 r = f2(acc[0] ? pr[0] : 0.0f, acc[1] ? pr[1] : 0.0f), i = f2(acc[0] ? pi[0] : 0.0f, acc[1] ? pi[1] : 0.0f);
-                        add(r, i, j);
-                        float r0, r1, i0, i1;
-                        f2_split(r, r0, r1);
-                        f2_split(i, i0, i1);
-                        if (acc[0]) { pr[0] = r0; pi[0] = i0; }
-                        if (acc[1]) { pr[1] = r1; pi[1] = i1; }
-                    }
-                }
-            }
             }
         }
         };
-        if constexpr (ACC != ACC_ALL) {
-            if (tile_fast && zin && !murz) cells(std::true_type{});
-            else cells(std::false_type{});
-        } else {
-            cells(std::false_type{});
-        }
+        if (tile_fast && zin && !murz) cells(std::true_type{});
+        else cells(std::false_type{});
 #pragma unroll
         for (int j = 0; j < 6; ++j) w[j] = w[j + 1];
     }

@@ -226,3 +226,35 @@ def test_bubbles_do_not_depend_on_the_batch(ctx):
         np.testing.assert_array_equal(part, whole[:n])
     ode.schedule = abi.BD_SCHEDULE_STATIC
     np.testing.assert_array_equal(ctx.gilmore(med, b, ode)[0], whole)
+
+
+# --------------------------------------------------------------------------- DFT pass
+@pytest.mark.parametrize("precision", [abi.BD_F32, abi.BD_F64])
+@pytest.mark.parametrize("nx,n_dft", [(27, 1), (28, 4), (29, 5), (26, 16)])
+def test_dft_pass(ctx, oracle, precision, nx, n_dft):
+    """The DFT pass on odd and even planes (scalar and 16-byte accesses; the FP32 rows are
+    padded), every remainder of its groups of four frequencies, a window that opens and
+    closes inside a group of steps and planes that start off a 16-byte boundary: the
+    bits of the run advanced one step at a time, and the FP64 oracle (1e-9 of the
+    largest accumulator in FP64, the 1e-5 field tolerance in FP32)."""
+    def make(precision):
+        p = layers(nx, 40, precision=precision)
+        w = p.params
+        w.n_dft = n_dft
+        for j in range(n_dft):
+            w.dft_freq[j] = 1.0e6 * (j + 1)
+        w.dft_start, w.dft_len = w.n_steps - 77, 73
+        w.dft_z_lo, w.dft_z_hi = 3, 36
+        return p
+    whole = ctx.westervelt(make(precision), want=("p_final", "dft"))
+    p = make(precision)
+    with ctx.westervelt_session(p) as s:
+        for _ in range(p.params.n_steps):
+            s.advance(1)
+        same(s.finish(want=("p_final", "dft")), whole, "step by step")
+    exp = oracle.westervelt(make(abi.BD_F64))
+    tol = 1e-9 if precision == abi.BD_F64 else 1e-5
+    for k in ("dft_re", "dft_im"):
+        a, b = np.asarray(whole[k], np.float64), np.asarray(exp[k]).reshape(whole[k].shape)
+        assert np.abs(b).max() > 0
+        assert np.linalg.norm(a - b) <= tol * np.sqrt(np.linalg.norm(exp["dft_re"]) ** 2 + np.linalg.norm(exp["dft_im"]) ** 2), k
