@@ -1,5 +1,5 @@
-// Device side of the Westervelt solver: one fused kernel per time step plus
-// the Mur boundary passes, all templated on the storage/arithmetic type.
+// Device side of the Westervelt solver: one fused kernel per time step, one pass over the
+// Mur faces and one over the DFT planes, templated on the storage/arithmetic type.
 //
 // Reference: W:139-236 (interior update), W:62-85 (source plane), W:88-135
 // (Mur), W:242-265 (water power), W:268-345 (harmonic power via FFT; here an

@@ -258,3 +258,21 @@ def test_dft_pass(ctx, oracle, precision, nx, n_dft):
         a, b = np.asarray(whole[k], np.float64), np.asarray(exp[k]).reshape(whole[k].shape)
         assert np.abs(b).max() > 0
         assert np.linalg.norm(a - b) <= tol * np.sqrt(np.linalg.norm(exp["dft_re"]) ** 2 + np.linalg.norm(exp["dft_im"]) ** 2), k
+
+
+@pytest.mark.parametrize("n_relax", [0, 1, 2, 3])
+def test_fp64_kernels_by_relaxation_count(ctx, n_relax):
+    """The FP64 TMA kernels compiled for 0, 1 and 2 relaxation processes, and the one that
+    reads the count, give the plain kernel's bits (plane materials, Mur, the DFT)."""
+    base = None
+    for v in (0, 8, 9, 16, 17, 18, -1):
+        p = layers(28, 40, precision=abi.BD_F64)
+        for m in range(p.medium.n_materials):
+            mt = p.medium.mat[m]
+            for k in range(mt.n_relax, n_relax):
+                mt.relax_tau[k], mt.relax_c[k] = 1.0e-8 * (k + 1), 1.0
+            mt.n_relax = n_relax if m % 2 == 0 else min(n_relax, 1)
+        p.params.tile_variant = v
+        r = ctx.westervelt(p)
+        base = base or r
+        same(r, base, "%d processes, variant %d" % (n_relax, v))
