@@ -167,6 +167,22 @@ def test_heat_run_equals_single_steps(ctx, precision, nx, ny, nz, steps):
         np.testing.assert_array_equal(one["dose"], got["dose"])
 
 
+@pytest.mark.parametrize("nx,ny,nz", [(66, 600, 40), (67, 599, 41), (253, 160, 83)])
+def test_heat_dose_free_kernel(ctx, nx, ny, nz):
+    """Grids large enough for chunks of four planes and more, whose steps without the dose
+    take their own kernel: the bits of single steps, which the general kernel runs."""
+    p, Q = thermal(nx, ny, nz, 5)
+    one = ctx.heat(p.thermal, Q, p.traj)
+    s = ctx.heat_slab(p.thermal, Q, p.traj, 0, nz)
+    for _ in range(5):
+        s.advance(1)
+    got = s.finish()
+    s.close()
+    np.testing.assert_array_equal(one["T"], got["T"])
+    np.testing.assert_array_equal(one["dose"], got["dose"])
+    assert one["T"].max() > p.thermal.T_ref
+
+
 def test_dose_add_is_the_fp64_sum(ctx):
     """One step onto doses of every magnitude, sign and kind: the bits of start + increment in
     double (the increment itself is the dose of the same step from zero)."""
@@ -252,6 +268,7 @@ def test_dft_pass(ctx, oracle, precision, nx, n_dft):
         for _ in range(p.params.n_steps):
             s.advance(1)
         same(s.finish(want=("p_final", "dft")), whole, "step by step")
+    same(ctx.westervelt_slabs(make(precision), 2, want=("p_final", "dft")), whole, "two slabs (rows of nx cells)")
     exp = oracle.westervelt(make(abi.BD_F64))
     tol = 1e-9 if precision == abi.BD_F64 else 1e-5
     for k in ("dft_re", "dft_im"):
