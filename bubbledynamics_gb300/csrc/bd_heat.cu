@@ -38,8 +38,8 @@ struct HeatMat {
 // bytes a cell), and a step's increment follows from its temperature alone, which
 // the next step reads anyway: of two steps the first leaves the dose alone
 // (DOSE_LATER) and the second adds both increments, in order (DOSE_BOTH), at 12 + 28
-// bytes for the two.  256 x 256 x 384: 87 us a step, 106 with DOSE_THIS alone;
-// 213 x 213 x 201: 40 and 45.
+// bytes for the two.  256 x 256 x 384: 86 us a step, 106 with DOSE_THIS alone;
+// 213 x 213 x 201: 38 and 45.
 enum HeatDose { DOSE_LATER = 0, DOSE_THIS = 1, DOSE_BOTH = 2 };
 
 template <class real>
@@ -381,17 +381,18 @@ __global__ void __launch_bounds__(128, 8) heat_theta4_kernel(const HeatArgs<floa
     }
 }
 
-// Planes per CTA of the FP32 kernels.  A chunk costs its planes plus about 0.7 of
-// a plane's time to start; grids of several waves fill up as CTAs end and pay
-// half a chunk at the end.  Measured per step: 256 x 256 x 384 105.7 / 105.5 /
-// 117.2 us in chunks of 8 / 24 / 32 planes, 213 x 213 x 201 45.0 / 47.8 / 52.7 us
-// in 4 / 24 / 32, 96 x 96 x 78 5.5 / 10.1 / 30.5 us in 2 / 8 / 32, 72 x 72 x 60
-// 7.1 / 11.2 / 29.9 us (launch by launch) in 2 / 8 / 32.
-static int march_zb(bd_context* ctx, long long tiles, int nz, int per_sm) {
+// Planes per CTA of the FP32 kernels, at most `most`.  A chunk costs its planes plus
+// about 0.7 of a plane's time to start; grids of several waves fill up as CTAs end and
+// pay half a chunk at the end.  The four-cell kernels stop at six planes: 256 x 256 x
+// 384 85.5 / 86.4 / 88.3 / 87.3 us a step in chunks of 6 / 8 / 24 / 43 planes, 213 x
+// 213 x 201 38.2 / 40.8 / 39.7 / 43.2 in 6 / 8 / 19 / 24, 150 x 150 x 120 12.8 / 13.0 /
+// 17.2 in 6 / 8 / 16, 96 x 96 x 78 5.5 / 6.5 / 9.2 in 2 / 4 / 8, 72 x 72 x 60 (launch
+// by launch) 6.7 / 7.1 / 8.1 in 1 / 2 / 4.
+static int march_zb(bd_context* ctx, long long tiles, int nz, int per_sm, int most) {
     const double slots = (double)ctx->sm_count * std::max(per_sm, 1);
     int best = 1;
     double cost = 1e300;
-    for (int zb = 1; zb <= std::min(nz, 64); ++zb) {
+    for (int zb = 1; zb <= std::min(nz, most); ++zb) {
         const double waves = (double)(tiles * ((nz + zb - 1) / zb)) / slots;
         const double c = (waves > 1.0 ? waves + 0.5 : 1.0) * (zb + 0.7);
         if (c < cost) { cost = c; best = zb; }
@@ -430,7 +431,7 @@ static int step4_zb(bd_context* ctx, int px, int ny, int nz) {
         BD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_step4_kernel<false, DOSE_BOTH>, 128, 0));
         return n;
     }();
-    return march_zb(ctx, (long long)((px / 4 + 15) / 16) * ((ny + 7) / 8), nz, per_sm);
+    return march_zb(ctx, (long long)((px / 4 + 15) / 16) * ((ny + 7) / 8), nz, per_sm, 6);
 }
 static int scalar_zb(bd_context* ctx, int nx, int ny, int nz) {
     static const int per_sm = [] {
@@ -438,7 +439,7 @@ static int scalar_zb(bd_context* ctx, int nx, int ny, int nz) {
         BD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_step_kernel<float, DOSE_BOTH>, 256, 0));
         return n;
     }();
-    return march_zb(ctx, (long long)((nx + 31) / 32) * ((ny + 7) / 8), nz, per_sm);
+    return march_zb(ctx, (long long)((nx + 31) / 32) * ((ny + 7) / 8), nz, per_sm, 64);
 }
 
 // Initial fields and outputs are formed on the device: the callers' arrays are
