@@ -674,6 +674,9 @@ struct HeatPlan {
         }
         if (has_mm) {
             mm.alloc(ctx, plane * nz);
+            // the four-cell kernels read the materials of a whole vector and index their table
+            // with each: the cells between rows are material 0, not what the block last held
+            if (px != nx) BD_CUDA(cudaMemsetAsync(mm.p, 0, (size_t)plane * nz, q));
             BD_CUDA(cudaMemcpy2DAsync(mm.p, px, th->material_map, nx, nx, (size_t)ny * nz, cudaMemcpyHostToDevice, q));
         }
         BD_CUDA(cudaMemsetAsync(sb.p, 0, 64, q));

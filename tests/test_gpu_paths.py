@@ -183,6 +183,26 @@ def test_heat_dose_free_kernel(ctx, nx, ny, nz):
     assert one["T"].max() > p.thermal.T_ref
 
 
+@pytest.mark.parametrize("nx", [13, 14, 15])
+def test_material_map_on_padded_rows(nx):
+    """The cells between padded rows hold a material of the table whatever the block of the
+    map last held: its bytes are 255 here (an FP64 run of no steps whose fields are all
+    ones), an index far outside.  The bits of the run on a fresh context."""
+    ny, nz = 10, 9                                           # 16 x 10 x 9 bytes
+    p, Q = thermal(nx, ny, nz, 5, material_map=True)
+    with api.Context(0) as c:
+        fresh = c.heat(p.thermal, Q, p.traj)
+    ones, _ = thermal(5, 6, 6, 3, abi.BD_F64)                # 180 doubles
+    ones.set_spots([0], [0], [0])
+    fill = np.full(180, 2 ** 64 - 1, np.uint64).view(np.float64).reshape(6, 6, 5)
+    ones.set_start(fill, fill)
+    with api.Context(0) as c:
+        c.heat(ones.thermal, fill, ones.traj)
+        got = c.heat(p.thermal, Q, p.traj)
+    np.testing.assert_array_equal(got["T"], fresh["T"])
+    np.testing.assert_array_equal(got["dose"], fresh["dose"])
+
+
 def test_dose_add_is_the_fp64_sum(ctx):
     """One step onto doses of every magnitude, sign and kind: the bits of start + increment in
     double (the increment itself is the dose of the same step from zero)."""
