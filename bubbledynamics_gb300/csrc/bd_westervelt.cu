@@ -668,6 +668,16 @@ static void autotune(WvSession& S) {
     g_tuned[key] = best_v;
 }
 
+// A host array to the device, in the order of the session's stream; the array has
+// been read when this returns.  (cudaMemcpy takes the legacy stream, which the
+// session's non-blocking stream is not ordered with, and may return before a copy
+// from pageable memory has reached the device: a kernel launched next could read
+// what the block held before.)
+static void to_device(WvSession& S, void* dev, const void* host, size_t bytes) {
+    BD_CUDA(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, S.ctx->stream));
+    BD_CUDA(cudaStreamSynchronize(S.ctx->stream));
+}
+
 template <class real>
 static void upload_consts(WvSession& S, const bd_medium* m) {
     WvConst<real> K;
@@ -687,7 +697,7 @@ static void upload_consts(WvSession& S, const bd_medium* m) {
         }
     }
     S.kconst.alloc(S.ctx, sizeof K);
-    BD_CUDA(cudaMemcpy(S.kconst.p, &K, sizeof K, cudaMemcpyHostToDevice));
+    to_device(S, S.kconst.p, &K, sizeof K);
     const WvArgs<real> a = make_args<real>(S, 0);    // dt, dx, dz and the relaxation scheme
     wv_derive_kernel<real><<<1, 32, 0, S.ctx->stream>>>(a, S.kconst.as<WvConst<real>>());
     BD_LAUNCHED(S.ctx);
@@ -696,7 +706,7 @@ static void upload_consts(WvSession& S, const bd_medium* m) {
 template <class T>
 static void upload(WvSession& S, PoolBuf& b, const std::vector<T>& v) {
     b.alloc(S.ctx, v.size() * sizeof(T));
-    if (!v.empty()) BD_CUDA(cudaMemcpy(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+    if (!v.empty()) to_device(S, b.p, v.data(), v.size() * sizeof(T));
 }
 
 // Rows of nx cells to or from rows of px cells.
@@ -715,7 +725,7 @@ template <class T>
 static void field_in(WvSession& S, void* dev, const void* host, long long rows) {
     const size_t bytes = (size_t)rows * S.nx * sizeof(T);
     if (S.px == S.nx) {
-        BD_CUDA(cudaMemcpy(dev, host, bytes, cudaMemcpyHostToDevice));
+        to_device(S, dev, host, bytes);
         return;
     }
     cudaStream_t st = S.ctx->stream;
@@ -889,7 +899,7 @@ static void setup(WvSession& S, bd_context* ctx, const bd_grid* g, const bd_medi
             if (m->plane_material[iz] < 0 || m->plane_material[iz] >= m->n_materials)
                 fail(BD_ERR_INVALID_ARG, "plane_material entry out of range");
         S.planemat.alloc(ctx, S.nz * 4);
-        BD_CUDA(cudaMemcpy(S.planemat.p, m->plane_material, S.nz * 4, cudaMemcpyHostToDevice));
+        to_device(S, S.planemat.p, m->plane_material, S.nz * 4);
     }
     S.n_materials = m->n_materials;
     S.mats.assign(m->mat, m->mat + m->n_materials);
@@ -1268,7 +1278,7 @@ static void ck_load(WvSession& S, const void* blob, size_t bytes) {
         real_in(S, S.dim.p, in, drows); in += (size_t)drows * S.nx * S.esz;
     }
     long long st = h.step;
-    BD_CUDA(cudaMemcpy(S.step_base.p, &st, sizeof st, cudaMemcpyHostToDevice));
+    to_device(S, S.step_base.p, &st, sizeof st);
     S.step = h.step;
 }
 

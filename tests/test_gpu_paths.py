@@ -138,6 +138,27 @@ def test_checkpoint_between_padded_and_plain_rows(ctx, nx):
             same(s.finish(), whole, "%d -> %d" % (first, second))
 
 
+@pytest.mark.parametrize("precision", [abi.BD_F32, abi.BD_F64])
+def test_constants_of_successive_solves(precision):
+    """Solves of two media in turn on one context, whose constants take the block that the
+    solve before left: each gives the bits of a fresh context, so every upload is in
+    place before the kernel that derives the coefficients reads it."""
+    def make(k):
+        p = layers(24, 40, precision=precision)
+        for m in range(p.medium.n_materials):
+            p.medium.mat[m].c0 *= 1.0 + 0.01 * k
+        p.params.n_steps = 20
+        return p
+    fresh = []
+    for k in (0, 1):
+        with api.Context(0) as c:
+            fresh.append(c.westervelt(make(k), want=("p_final",)))
+    assert np.abs(fresh[0]["p_final"] - fresh[1]["p_final"]).max() > 0
+    with api.Context(0) as c:
+        for i in range(24):
+            same(c.westervelt(make(i % 2), want=("p_final",)), fresh[i % 2], "solve %d" % i)
+
+
 # --------------------------------------------------------------------------- heat
 def thermal(nx, ny, nz, steps, precision=abi.BD_F32, material_map=False):
     k = presets.ref_T_mini_constants(Nxy=nx, Nz=nz, legs=2)
