@@ -819,6 +819,10 @@ static void setup(WvSession& S, bd_context* ctx, const bd_grid* g, const bd_medi
     S.any_mur = false;
     for (int f = 0; f < 6; ++f) if (g->face[f] == BD_FACE_MUR) S.any_mur = true;
     if (S.any_mur && (g->mur_layers < 1 || g->mur_layers > 8)) fail(BD_ERR_INVALID_ARG, "mur_layers must be 1..8");
+    // a run of layers starts from the cell next to it (the z- run ends at the source plane, where there is one)
+    auto fills = [&](int f, int n) { return g->face[f] == BD_FACE_MUR && g->mur_layers >= n; };
+    if (fills(1, S.nx) || fills(3, S.ny) || fills(5, S.nz) || (S.s.kind == BD_SRC_NONE && fills(4, S.nz)))
+        fail(BD_ERR_INVALID_ARG, "%d Mur layers leave no cell of an axis to start from", g->mur_layers);
     if (m->n_materials < 1 || m->n_materials > BD_MAX_MATERIALS) fail(BD_ERR_INVALID_ARG, "n_materials out of range");
     S.max_relax = 0;
     for (int k = 0; k < m->n_materials; ++k) {

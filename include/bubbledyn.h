@@ -91,7 +91,8 @@ typedef struct bd_grid {
     double dx, dz;              /* dy == dx [m] */
     double dt;                  /* time step [s] (W:416) */
     int32_t face[6];            /* bd_face_kind of x-, x+, y-, y+, z-, z+ */
-    int32_t mur_layers;         /* Mur layers on MUR faces; 3 in W:108-133 (z- uses source_iz layers) */
+    int32_t mur_layers;         /* Mur layers on MUR faces, 1..8 and fewer than the axis has cells;
+                                 * 3 in W:108-133 (z- uses source_iz layers) */
     int32_t sponge_cells;       /* damping layer width on OPEN faces (0 = none) */
     double sponge_strength;     /* w(d) = exp(-strength*(d/W)^2) applied each step */
 } bd_grid;

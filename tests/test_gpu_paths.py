@@ -117,6 +117,23 @@ def test_mur_layer_counts(ctx, oracle, precision, n_layers):
         assert np.linalg.norm(a - b) <= (1e-9 if precision == abi.BD_F64 else 1e-5) * np.linalg.norm(b), k
 
 
+@pytest.mark.parametrize("face", [1, 3, 4, 5])
+def test_mur_layers_that_fill_an_axis_are_refused(ctx, face):
+    """Eight layers on an axis of eight cells have no inner neighbour: the run would read cells
+    in front of (z-: behind) the field.  Nine cells are enough."""
+    def make(cells):
+        nx, ny, nz = (cells if face == 1 else 12), (cells if face == 3 else 12), (cells if face > 3 else 24)
+        p = presets.cfg1(nx, ny, nz, 4, heterogeneity=False)
+        p.grid.face[face] = abi.BD_FACE_MUR
+        p.grid.mur_layers = 8
+        p.source.kind = abi.BD_SRC_NONE
+        return p
+    with pytest.raises(api.BDError) as e:
+        ctx.westervelt(make(8))
+    assert e.value.status == abi.BD_ERR_INVALID_ARG and "Mur layers" in str(e.value)
+    assert not ctx.westervelt(make(9), want=("p_final",))["p_final"].any()
+
+
 @pytest.mark.parametrize("nx", [33, 35])
 def test_checkpoint_between_padded_and_plain_rows(ctx, nx):
     """A checkpoint has rows of nx cells whatever the device's: one taken on padded
