@@ -438,10 +438,15 @@ static void launch_after(WvSession& S, void (*kern)(P...), long long threads, in
     BD_LAUNCHED(S.ctx);
 }
 
-// The Mur faces of a step (one kernel), after the stencil update.
+// The Mur faces of a step, after the stencil update: one kernel, and one before it for
+// the z faces where their layers meet.
 template <class real>
-static void launch_mur(WvSession& S, const WvArgs<real>& a, int koff, cudaStream_t st) {
+static void launch_mur(WvSession& S, WvArgs<real> a, int koff, cudaStream_t st) {
     const long long cx = a.mur_xp ? a.nx - a.L : a.nx, cy = a.mur_yp ? a.ny - a.L : a.ny;
+    if (a.mur_zm && a.mur_zp && a.Lzm + a.L >= a.nz) {
+        launch_after(S, wv_mur_z_kernel<real>, cx * cy, 128, st, a, S.kconst.as<WvConst<real>>(), koff);
+        a.mur_zm = a.mur_zp = 0;                    // to wv_mur_kernel the z faces are cells like any other
+    }
     const long long n = (a.mur_zm ? cx * cy * a.Lzm : 0) + (a.mur_zp ? cx * cy : 0) + (a.mur_xp ? cy * a.nz : 0) +
                         (a.mur_yp ? (long long)a.nx * a.nz : 0);
     if (n <= 0) return;

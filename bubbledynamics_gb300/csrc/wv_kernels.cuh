@@ -438,9 +438,42 @@ __device__ __forceinline__ real mur_cell(real pj, real nb, real pi, real c, real
 constexpr int ACC_STEPS = 5, ACC_DPDT = 4;
 constexpr int MUR_MAXL = 8;    // layers of an x+, y+ or z+ face
 
+// The z faces where their layers leave no plane between them (Lzm + L >= nz): the z+
+// run then starts on a z- cell, the last z- cell reads the first z+ one, or cells
+// belong to both.  One thread takes a column, z- first as a serial launch of W:101-113,
+// so the order is fixed; wv_mur_kernel follows with the x+ and y+ faces.  A cell of
+// both runs accumulates its final value.
+template <class real>
+__global__ void __launch_bounds__(128) wv_mur_z_kernel(const WvArgs<real> a, const WvConst<real>* __restrict__ Kp, int koff) {
+    const WvConst<real>& K = *Kp;
+    const int L = a.L;
+    const int cx = a.mur_xp ? a.nx - L : a.nx, cy = a.mur_yp ? a.ny - L : a.ny;   // columns outside the x+ / y+ layers
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (t >= (long long)cx * cy) return;
+    const long long step = *a.step_base + koff;
+    const long long col = (t / cx) * a.px + t % cx;
+    const real* Pn = a.p0;
+    real* F = a.p4;
+    auto put = [&](long long i, real v, bool last) {
+        F[i] = v;
+        if (last) accumulate(a, step, i, v, a.energy_mode == BD_ENERGY_DPDT2 ? a.p1[i] : real(0));
+    };
+    for (int iz = 0; iz < a.Lzm; ++iz) {
+        const long long i = (long long)iz * a.plane + col, j = i + a.plane;
+        put(i, mur_cell(Pn[j], iz + 1 < a.Lzm ? Pn[j] : F[j], Pn[i], cell_c(a, K, i, cell_mat(a, i, iz)), a.dtdz), iz < a.nz - L);
+    }
+    for (int iz = a.nz - L; iz < a.nz; ++iz) {
+        const long long i = (long long)iz * a.plane + col, j = i - a.plane;
+        put(i, mur_cell(Pn[j], F[j], Pn[i], cell_c(a, K, i, cell_mat(a, i, iz)), a.dtdz), true);
+    }
+}
+
 // The Mur faces of a step in one pass, in the order z-, z+, x+, y+ of a serial
 // launch of W:88-135.  Every cell's value follows from P^n and from the cells the
-// stencil update wrote, which this kernel only reads: a thread takes one run of
+// stencil update wrote, which this kernel only reads (the two z runs do not meet,
+// Lzm + L < nz; where they do, wv_mur_z_kernel has formed them): a thread takes one run of
 // layers (or one z- cell, whose neighbour is P^n or the source plane) and, where
 // the run starts on a cell that an earlier face overwrites, forms that cell's
 // value itself.  Three kernels, one per face, whose threads re-read each layer

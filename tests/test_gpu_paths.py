@@ -117,6 +117,30 @@ def test_mur_layer_counts(ctx, oracle, precision, n_layers):
         assert np.linalg.norm(a - b) <= (1e-9 if precision == abi.BD_F64 else 1e-5) * np.linalg.norm(b), k
 
 
+@pytest.mark.parametrize("precision", [abi.BD_F32, abi.BD_F64])
+@pytest.mark.parametrize("nz,n_layers,plane", [(12, 3, 8), (12, 4, 8), (16, 8, 8), (12, 4, 10), (13, 8, 12)])
+def test_mur_z_runs_that_meet(ctx, oracle, precision, nz, n_layers, plane):
+    """Mur on both z faces, z- up to a source plane on either side of the first z+ layer: one
+    plane between the runs, none, and cells in both.  The oracle's order, 1e-9 of it in
+    FP64 and the 1e-5 field tolerance in FP32, in repeated runs the same bits."""
+    def make(precision):
+        p = layers(26, 40, precision=precision)
+        p.grid.nz, p.grid.mur_layers, p.source.plane_iz = nz, n_layers, plane
+        p.params.q_mode, p.params.n_dft = abi.BD_Q_NONE, 0
+        p.params.n_steps, p.params.peak_start, p.params.peak_end = 60, 5, 50
+        p.params.energy_start, p.params.energy_end = 10, 55
+        return p
+    want = ("p_final", "peak", "energy")
+    got = ctx.westervelt(make(precision), want=want)
+    for _ in range(3):
+        same(ctx.westervelt(make(precision), want=want), got, "again")
+    exp = oracle.westervelt(make(abi.BD_F64))
+    for k in want:
+        a, b = np.asarray(got[k], np.float64), np.asarray(exp[k]).reshape(got[k].shape)
+        assert plane > nz - n_layers or np.abs(b).max() > 0      # a z+ layer over the source plane leaves no wave
+        assert np.linalg.norm(a - b) <= (1e-9 if precision == abi.BD_F64 else 1e-5) * np.linalg.norm(b), k
+
+
 @pytest.mark.parametrize("face", [1, 3, 4, 5])
 def test_mur_layers_that_fill_an_axis_are_refused(ctx, face):
     """Eight layers on an axis of eight cells have no inner neighbour: the run would read cells
