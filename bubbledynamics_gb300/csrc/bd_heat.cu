@@ -81,12 +81,13 @@ __device__ __forceinline__ float2 df_add(float2 d, float x) {
 
 // A positive float widened to double with integer operations (exponent rebias,
 // mantissa shift), so the conversion stays off the FP64 pipe, which the dose
-// add already occupies; exact for normal floats, and values below the float
-// normal range (dose rates under 1e-38) become zero.
+// add already occupies; exact for normal floats, infinities and NaN (a rate above
+// 171 C or of no temperature), and values below the float normal range (dose
+// rates under 1e-38) become zero.
 __device__ __forceinline__ double widen_pos(float x) {
     const int b = __float_as_int(x);
     if (b < 0x00800000) return 0.0;                        // zero or subnormal
-    return __longlong_as_double(((long long)b << 29) + (896LL << 52));
+    return __longlong_as_double(((long long)b << 29) + ((b < 0x7f800000 ? 896LL : 1792LL) << 52));
 }
 
 // The FP64 adder behind a branch: asm volatile keeps the compiler from issuing it
@@ -110,7 +111,8 @@ __device__ __forceinline__ double dose_add(double d, float inc) {
     const int b = __float_as_int(inc);
     const int s = (b >> 23) + 925 - (int)(D >> 52);          // 29 - distance of the exponents
     const long long sum = D + (long long)((unsigned long long)((b & 0x007fffff) | 0x00800000) * (1u << (s & 31)));
-    if ((unsigned)s <= 29u && b >= 0x00800000 && ((sum ^ D) >> 52) == 0) return __longlong_as_double(sum);
+    const bool normal = (unsigned)(b - 0x00800000) < 0x7f000000u;   // positive, and no infinity or NaN
+    if ((unsigned)s <= 29u && normal && ((sum ^ D) >> 52) == 0) return __longlong_as_double(sum);
     return dadd_slow(d, widen_pos(inc));
 }
 

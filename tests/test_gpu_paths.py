@@ -288,6 +288,23 @@ def test_dose_add_is_the_fp64_sum(ctx):
     np.testing.assert_array_equal(got, exp)
 
 
+@pytest.mark.parametrize("steps", [1, 2])
+@pytest.mark.parametrize("kelvin", [600.0, np.inf, np.nan])
+def test_dose_add_of_a_rate_that_is_no_number(ctx, steps, kelvin):
+    """Above 171 C the float rate is infinite: the dose becomes infinite (NaN for a NaN
+    temperature) whatever it was, also between 2^128 and 2^157, where the exponents of an
+    infinite increment and of the dose are as close as those the integer add takes."""
+    nx, ny, nz = 18, 14, 11
+    p, Q = thermal(nx, ny, nz, steps)
+    start = np.ldexp(np.random.default_rng(2).uniform(1.0, 2.0, nx * ny * nz), np.arange(nx * ny * nz) % 60 + 110)
+    start = start.reshape(nz, ny, nx)
+    p.set_start(np.full((nz, ny, nx), kelvin), start)
+    got = ctx.heat(p.thermal, Q, p.traj)["dose"]
+    exp = start.copy()
+    exp[1:-1, 1:-1, 1:-1] = np.nan if np.isnan(kelvin) else np.inf
+    np.testing.assert_array_equal(got, exp)
+
+
 @pytest.mark.parametrize("nx", [40, 41])
 @pytest.mark.parametrize("steps", [1, 2, 65])
 def test_noalloc_steps_equal_the_run(ctx, nx, steps):
