@@ -45,6 +45,8 @@ __device__ __forceinline__ Coef2<NR> coef2_c(const WvArgs<float>& a, const MatCo
             F2 sa = f2(0.0f);
 #pragma unroll
             for (int v = 0; v < NR; ++v) {
+                // ptxas leaves this product alone, which is used again (the bits of two processes
+                // are tested against the plain kernel's); f2_mul1 costs 0.25 % of a step
                 k.av[v] = f2_mul(f2(A.ra_num[v], B.ra_num[v]), ic3);
                 sa = f2_add(sa, k.av[v]);
             }

@@ -158,6 +158,26 @@ def test_mur_layers_that_fill_an_axis_are_refused(ctx, face):
     assert not ctx.westervelt(make(9), want=("p_final",))["p_final"].any()
 
 
+@pytest.mark.parametrize("nx", [40, 41])
+def test_two_processes_with_a_c_map(ctx, nx):
+    """Two relaxation processes in the semi-implicit scheme on a c map, strong enough that a
+    rounding of their coefficients shows: every variant gives the plain kernel's bits."""
+    base = None
+    for v in (0, 17, 18, 19, 21, 23, 24, 26, 28):
+        if nx % 4 and 8 <= v < 24:
+            continue
+        p = burst(nx, 34, 45, 60)
+        mt = p.medium.mat[0]
+        mt.n_relax = 2
+        for k, (c, tau) in enumerate(((60.0, 1.0e-7), (45.0, 3.0e-8))):
+            mt.relax_c[k], mt.relax_tau[k] = c, tau
+        p.params.tile_variant = v
+        r = ctx.westervelt(p)
+        base = base or r
+        assert 0 < np.abs(base["p_final"]).max() < 1e8
+        same(r, base, "nx %d, variant %d" % (nx, v))
+
+
 @pytest.mark.parametrize("nx", [33, 35])
 def test_checkpoint_between_padded_and_plain_rows(ctx, nx):
     """A checkpoint has rows of nx cells whatever the device's: one taken on padded
