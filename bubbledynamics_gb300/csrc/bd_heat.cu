@@ -392,9 +392,10 @@ __global__ void __launch_bounds__(128, 8) heat_theta4_kernel(const HeatArgs<floa
 // by launch) 6.7 / 7.1 / 8.1 in 1 / 2 / 4.
 static int march_zb(bd_context* ctx, long long tiles, int nz, int per_sm, int most) {
     const double slots = (double)ctx->sm_count * std::max(per_sm, 1);
-    int best = 1;
+    const int least = (nz + 65534) / 65535;       // a grid has up to 65,535 chunks
+    int best = least;
     double cost = 1e300;
-    for (int zb = 1; zb <= std::min(nz, most); ++zb) {
+    for (int zb = least; zb <= std::min(nz, most); ++zb) {
         const double waves = (double)(tiles * ((nz + zb - 1) / zb)) / slots;
         const double c = (waves > 1.0 ? waves + 0.5 : 1.0) * (zb + 0.7);
         if (c < cost) { cost = c; best = zb; }

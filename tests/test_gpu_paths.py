@@ -265,6 +265,17 @@ def test_heat_dose_free_kernel(ctx, nx, ny, nz):
     assert one["T"].max() > p.thermal.T_ref
 
 
+def test_heat_run_of_many_planes(ctx):
+    """More planes than the four-cell kernel's six-plane chunks could number in a grid's z extent."""
+    nx, ny, nz, steps = 6, 5, 400001, 3
+    p, Q = thermal(nx, ny, nz, steps)
+    q, _ = thermal(nx, ny, nz, steps, abi.BD_F64)
+    got, exp = ctx.heat(p.thermal, Q, p.traj)["T"], ctx.heat(q.thermal, Q, q.traj)["T"]
+    rise = np.abs(exp - q.initial_fields()[0]).max()
+    assert rise > 1e-3
+    assert np.abs(got - exp).max() <= 1e-5 * rise + 1e-9
+
+
 @pytest.mark.parametrize("nx", [13, 14, 15])
 def test_material_map_on_padded_rows(nx):
     """The cells between padded rows hold a material of the table whatever the block of the
