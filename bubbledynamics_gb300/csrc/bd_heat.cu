@@ -589,7 +589,12 @@ struct HeatPlan {
     int64_t step = 0;                              // steps done
     static constexpr int leg_cap = 4096;
     std::vector<int64_t> leg_end;
-    PoolBuf pm, mm, shd, sb, stage;                // stage: doubles of the largest slab, for conversions
+    PoolBuf pm, mm, shd, sb;
+    // doubles of a host array on their way to or from FP32 or padded rows, `group` planes
+    // at a time: one buffer for a whole slab would take 8 B a cell next to the 20 of the run
+    PoolBuf stage;
+    int group = 1;
+    static constexpr long long kStageBytes = 32 << 20;
     std::vector<HeatSlab> sl;
     HeatArgs<float> af{};
     HeatArgs<double> ad{};
@@ -648,7 +653,7 @@ struct HeatPlan {
         T_ref = f64 ? 0.0 : th->T_ref;
         esz = f64 ? 8 : 4;
         std::vector<HeatSlab>(owned.size()).swap(sl);
-        long long most = 0;
+        int most = 0;
         for (size_t k = 0; k < owned.size(); ++k) {
             HeatSlab& S = sl[k];
             S.zb = owned[k].first;
@@ -657,8 +662,9 @@ struct HeatPlan {
             S.hi = S.ze < nz ? S.ze + 1 : nz;
             S.nzl = S.hi - S.lo;
             S.nl = plane * S.nzl;
-            most = std::max(most, hplane * S.nzl);
+            most = std::max(most, S.nzl);
         }
+        group = (int)std::clamp<long long>(kStageBytes / (hplane * 8), 1, most);
         cudaStream_t q = ctx->stream;
         // whatever ends this block, the copies from the callers' arrays and from sh are done by then
         struct Drain {
@@ -667,7 +673,7 @@ struct HeatPlan {
         } drain{q};
         shd.alloc(ctx, sh.size() * sizeof(int2));
         sb.alloc(ctx, 64);
-        if (!f64) stage.alloc(ctx, most * 8);
+        if (!f64) stage.alloc(ctx, group * hplane * 8);
         BD_CUDA(cudaMemcpyAsync(shd.p, sh.data(), sh.size() * sizeof(int2), cudaMemcpyHostToDevice, q));
         has_pm = th->plane_material != nullptr;
         has_mm = th->material_map != nullptr;
@@ -693,44 +699,49 @@ struct HeatPlan {
         for (HeatSlab& S : sl) {
             S.Ta.alloc(ctx, S.nl * esz); S.Tb.alloc(ctx, S.nl * esz); S.Qd.alloc(ctx, S.nl * esz);
             S.TDd.alloc(ctx, S.nl * 8);
-            const long long o = hplane * S.lo, cells = hplane * S.nzl;
-            const int* spm = has_pm ? pm.as<int>() + S.lo : nullptr;
-            const uint8_t* smm = has_mm ? mm.as<uint8_t>() + plane * S.lo : nullptr;
-            const unsigned blocks = (unsigned)((cells + 255) / 256);
             // FP64 rows are not padded: its arrays are copied straight in, the FP32 ones through the staging buffer
-            const double* src = nullptr;
-            if (th->T_start) {
-                void* to = f64 ? S.Tb.p : stage.p;
-                BD_CUDA(cudaMemcpyAsync(to, th->T_start + o, cells * 8, cudaMemcpyHostToDevice, q));
-                src = static_cast<const double*>(to);
-            }
-            if (f64 && src) {
-                BD_CUDA(cudaMemcpyAsync(S.Ta.p, S.Tb.p, cells * 8, cudaMemcpyDeviceToDevice, q));
-            } else if (f64) {
-                heat_init_T_kernel<double><<<blocks, 256, 0, q>>>(S.Ta.as<double>(), S.Tb.as<double>(), nullptr, in, spm,
-                                                                  smm, nx, px, plane, cells, 0.0);
-                BD_LAUNCHED(ctx);
-            } else {
-                heat_init_T_kernel<float><<<blocks, 256, 0, q>>>(S.Ta.as<float>(), S.Tb.as<float>(), src, in, spm, smm,
-                                                                 nx, px, plane, cells, T_ref);
-                BD_LAUNCHED(ctx);
-            }
-            if (f64) {
-                BD_CUDA(cudaMemcpyAsync(S.Qd.p, Q + o, cells * 8, cudaMemcpyHostToDevice, q));
-            } else {
-                BD_CUDA(cudaMemcpyAsync(stage.p, Q + o, cells * 8, cudaMemcpyHostToDevice, q));
-                heat_narrow_kernel<<<blocks, 256, 0, q>>>(S.Qd.as<float>(), stage.as<double>(), nx, px, cells);
-                BD_LAUNCHED(ctx);
-            }
-            src = nullptr;
-            if (th->dose_start) {
-                void* to = f64 ? S.TDd.p : stage.p;
-                BD_CUDA(cudaMemcpyAsync(to, th->dose_start + o, cells * 8, cudaMemcpyHostToDevice, q));
-                src = static_cast<const double*>(to);
-            }
-            if (!(f64 && src)) {
-                heat_init_dose_kernel<<<blocks, 256, 0, q>>>(S.TDd.as<double>(), src, in, spm, smm, nx, px, plane, cells);
-                BD_LAUNCHED(ctx);
+            const int per = f64 ? S.nzl : group;
+            for (int z = 0; z < S.nzl; z += per) {
+                const int planes = std::min(per, S.nzl - z);
+                const long long o = hplane * (S.lo + z), cells = hplane * planes, at = plane * z;
+                const int* spm = has_pm ? pm.as<int>() + S.lo + z : nullptr;
+                const uint8_t* smm = has_mm ? mm.as<uint8_t>() + plane * (S.lo + z) : nullptr;
+                const unsigned blocks = (unsigned)((cells + 255) / 256);
+                const double* src = nullptr;
+                if (th->T_start) {
+                    void* to = f64 ? S.Tb.p : stage.p;
+                    BD_CUDA(cudaMemcpyAsync(to, th->T_start + o, cells * 8, cudaMemcpyHostToDevice, q));
+                    src = static_cast<const double*>(to);
+                }
+                if (f64 && src) {
+                    BD_CUDA(cudaMemcpyAsync(S.Ta.p, S.Tb.p, cells * 8, cudaMemcpyDeviceToDevice, q));
+                } else if (f64) {
+                    heat_init_T_kernel<double><<<blocks, 256, 0, q>>>(S.Ta.as<double>(), S.Tb.as<double>(), nullptr, in,
+                                                                      spm, smm, nx, px, plane, cells, 0.0);
+                    BD_LAUNCHED(ctx);
+                } else {
+                    heat_init_T_kernel<float><<<blocks, 256, 0, q>>>(S.Ta.as<float>() + at, S.Tb.as<float>() + at, src, in,
+                                                                     spm, smm, nx, px, plane, cells, T_ref);
+                    BD_LAUNCHED(ctx);
+                }
+                if (f64) {
+                    BD_CUDA(cudaMemcpyAsync(S.Qd.p, Q + o, cells * 8, cudaMemcpyHostToDevice, q));
+                } else {
+                    BD_CUDA(cudaMemcpyAsync(stage.p, Q + o, cells * 8, cudaMemcpyHostToDevice, q));
+                    heat_narrow_kernel<<<blocks, 256, 0, q>>>(S.Qd.as<float>() + at, stage.as<double>(), nx, px, cells);
+                    BD_LAUNCHED(ctx);
+                }
+                src = nullptr;
+                if (th->dose_start) {
+                    void* to = f64 ? S.TDd.p : stage.p;
+                    BD_CUDA(cudaMemcpyAsync(to, th->dose_start + o, cells * 8, cudaMemcpyHostToDevice, q));
+                    src = static_cast<const double*>(to);
+                }
+                if (!(f64 && src)) {
+                    heat_init_dose_kernel<<<blocks, 256, 0, q>>>(S.TDd.as<double>() + at, src, in, spm, smm, nx, px, plane,
+                                                                 cells);
+                    BD_LAUNCHED(ctx);
+                }
             }
         }
         BD_CUDA(cudaStreamSynchronize(q));
@@ -862,17 +873,19 @@ struct HeatPlan {
         cudaStream_t s = ctx->stream;
         for (const HeatSlab& S : sl) {
             const PoolBuf& src = newest(S, steps);
-            const long long off = plane * (S.zb - S.lo), cnt = hplane * (S.ze - S.zb);
-            const double* from = static_cast<const double*>(src.p) + off;
-            if (!f64) {
-                heat_widen_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, s>>>(
-                    stage.as<double>(), static_cast<const float*>(src.p) + off, nx, px, cnt, T_ref);
-                BD_LAUNCHED(ctx);
-                from = stage.as<double>();
+            host_populate(dst + hplane * S.zb, hplane * (S.ze - S.zb) * 8);   // while the steps before this copy run
+            const int per = f64 ? S.ze - S.zb : group;
+            for (int z = S.zb; z < S.ze; z += per) {
+                const long long off = plane * (z - S.lo), cnt = hplane * std::min(per, S.ze - z);
+                const double* from = static_cast<const double*>(src.p) + off;
+                if (!f64) {
+                    heat_widen_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, s>>>(
+                        stage.as<double>(), static_cast<const float*>(src.p) + off, nx, px, cnt, T_ref);
+                    BD_LAUNCHED(ctx);
+                    from = stage.as<double>();
+                }
+                BD_CUDA(cudaMemcpyAsync(dst + hplane * z, from, cnt * 8, cudaMemcpyDeviceToHost, s));
             }
-            double* d = dst + hplane * S.zb;
-            host_populate(d, cnt * 8);   // while the steps before this copy run
-            BD_CUDA(cudaMemcpyAsync(d, from, cnt * 8, cudaMemcpyDeviceToHost, s));
         }
         BD_CUDA(cudaStreamSynchronize(s));
     }
@@ -880,16 +893,18 @@ struct HeatPlan {
     void copy_dose(double* dst) {
         cudaStream_t s = ctx->stream;
         for (const HeatSlab& S : sl) {
-            const long long off = plane * (S.zb - S.lo), cnt = hplane * (S.ze - S.zb);
-            const double* from = S.TDd.as<double>() + off;
-            if (px != nx) {
-                heat_compact_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, s>>>(stage.as<double>(), from, nx, px, cnt);
-                BD_LAUNCHED(ctx);
-                from = stage.as<double>();
+            host_populate(dst + hplane * S.zb, hplane * (S.ze - S.zb) * 8);
+            const int per = px == nx ? S.ze - S.zb : group;
+            for (int z = S.zb; z < S.ze; z += per) {
+                const long long off = plane * (z - S.lo), cnt = hplane * std::min(per, S.ze - z);
+                const double* from = S.TDd.as<double>() + off;
+                if (px != nx) {
+                    heat_compact_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, s>>>(stage.as<double>(), from, nx, px, cnt);
+                    BD_LAUNCHED(ctx);
+                    from = stage.as<double>();
+                }
+                BD_CUDA(cudaMemcpyAsync(dst + hplane * z, from, cnt * 8, cudaMemcpyDeviceToHost, s));
             }
-            double* d = dst + hplane * S.zb;
-            host_populate(d, cnt * 8);
-            BD_CUDA(cudaMemcpyAsync(d, from, cnt * 8, cudaMemcpyDeviceToHost, s));
         }
         BD_CUDA(cudaStreamSynchronize(s));
     }

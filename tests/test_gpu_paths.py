@@ -265,6 +265,52 @@ def test_heat_dose_free_kernel(ctx, nx, ny, nz):
     assert one["T"].max() > p.thermal.T_ref
 
 
+def device_bytes(torch):
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def test_heat_run_memory():
+    """An FP32 heating run holds 20 bytes a cell (two temperatures and the source in float, the
+    dose in double) and a staging buffer of bounded size."""
+    torch = pytest.importorskip("torch")
+    with api.Context(0) as c:
+        p, Q = thermal(34, 30, 12, 2)
+        c.heat(p.thermal, Q, p.traj)                  # kernels loaded
+        nx, ny, nz = 253, 250, 300
+        p, Q = thermal(nx, ny, nz, 2)
+        before = device_bytes(torch)
+        s = c.heat_slab(p.thermal, Q, p.traj, 0, nz)
+        held = before - device_bytes(torch)
+        s.close()
+    assert held <= 20 * 256 * ny * nz + (48 << 20)
+
+
+def test_fields_through_several_staging_groups(ctx):
+    """Source, start fields and results of a grid of several staging buffers: two steps
+    match FP64 (the FP32 tolerance, 1e-5) and two slabs give the same bits; with no steps the
+    start comes back, its temperatures in float around T_ref."""
+    nx, ny, nz, steps = 255, 254, 150, 2
+    p, Q = thermal(nx, ny, nz, steps)
+    rng = np.random.default_rng(8)
+    T0, D0 = 300.0 + 40.0 * rng.random((nz, ny, nx)), rng.random((nz, ny, nx))
+    p.set_start(T0, D0)
+    got = ctx.heat(p.thermal, Q, p.traj, n_slabs=1)
+    two = ctx.heat(p.thermal, Q, p.traj, n_slabs=2)
+    np.testing.assert_array_equal(got["T"], two["T"])
+    np.testing.assert_array_equal(got["dose"], two["dose"])
+    q, _ = thermal(nx, ny, nz, steps, abi.BD_F64)
+    q.set_start(T0, D0)
+    exp = ctx.heat(q.thermal, Q, q.traj)
+    assert np.abs(got["T"] - exp["T"]).max() <= 1e-5 * 40.0
+    np.testing.assert_allclose(got["dose"], exp["dose"], rtol=1e-5)
+    q = presets.ThermalProblem("start", p.thermal, p.traj, p._keep)
+    q.set_spots([0], [0], [0])
+    back = ctx.heat(q.thermal, Q, q.traj)
+    np.testing.assert_array_equal(back["dose"], D0)
+    np.testing.assert_array_equal(back["T"], p.thermal.T_ref + (T0 - p.thermal.T_ref).astype(np.float32).astype(np.float64))
+
+
 def test_heat_run_of_many_planes(ctx):
     """More planes than the four-cell kernel's six-plane chunks could number in a grid's z extent."""
     nx, ny, nz, steps = 6, 5, 400001, 3
