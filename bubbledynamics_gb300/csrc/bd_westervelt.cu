@@ -725,36 +725,50 @@ __global__ void wv_repitch_kernel(T* __restrict__ dst, const T* __restrict__ src
     else dst[i] = src[j];
 }
 
+// Rows that pass through S.stage at a time: 32 MB of them, so that a checkpoint's DFT
+// planes need no second copy of all accumulators.
+template <class T>
+static long long stage_rows(WvSession& S, long long rows) {
+    const size_t row = (size_t)S.nx * sizeof(T);
+    const long long group = std::clamp<long long>((32 << 20) / row, 1, rows);
+    if (S.stage.bytes < group * row) S.stage.alloc(S.ctx, group * row);
+    return group;
+}
+
 // rows = number of nx-cell rows moved between a host array and a field
 template <class T>
 static void field_in(WvSession& S, void* dev, const void* host, long long rows) {
-    const size_t bytes = (size_t)rows * S.nx * sizeof(T);
     if (S.px == S.nx) {
-        to_device(S, dev, host, bytes);
+        to_device(S, dev, host, (size_t)rows * S.nx * sizeof(T));
         return;
     }
     cudaStream_t st = S.ctx->stream;
-    if (S.stage.bytes < bytes) S.stage.alloc(S.ctx, bytes);
-    BD_CUDA(cudaMemcpyAsync(S.stage.p, host, bytes, cudaMemcpyHostToDevice, st));
-    const long long n = rows * S.nx;
-    wv_repitch_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(static_cast<T*>(dev), S.stage.as<T>(), S.nx, S.px, n, 1);
-    BD_LAUNCHED(S.ctx);
+    const long long group = stage_rows<T>(S, rows);
+    for (long long r = 0; r < rows; r += group) {
+        const long long n = std::min(group, rows - r) * S.nx;
+        BD_CUDA(cudaMemcpyAsync(S.stage.p, static_cast<const T*>(host) + r * S.nx, n * sizeof(T), cudaMemcpyHostToDevice, st));
+        wv_repitch_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(static_cast<T*>(dev) + r * S.px, S.stage.as<T>(), S.nx,
+                                                                           S.px, n, 1);
+        BD_LAUNCHED(S.ctx);
+    }
     BD_CUDA(cudaStreamSynchronize(st));      // the host array has been read
 }
 
 template <class T>
 static void field_out(WvSession& S, void* host, const void* dev, long long rows) {
-    const size_t bytes = (size_t)rows * S.nx * sizeof(T);
     if (S.px == S.nx) {
-        BD_CUDA(cudaMemcpy(host, dev, bytes, cudaMemcpyDeviceToHost));
+        BD_CUDA(cudaMemcpy(host, dev, (size_t)rows * S.nx * sizeof(T), cudaMemcpyDeviceToHost));
         return;
     }
     cudaStream_t st = S.ctx->stream;
-    if (S.stage.bytes < bytes) S.stage.alloc(S.ctx, bytes);
-    const long long n = rows * S.nx;
-    wv_repitch_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(S.stage.as<T>(), static_cast<const T*>(dev), S.nx, S.px, n, 0);
-    BD_LAUNCHED(S.ctx);
-    BD_CUDA(cudaMemcpyAsync(host, S.stage.p, bytes, cudaMemcpyDeviceToHost, st));
+    const long long group = stage_rows<T>(S, rows);
+    for (long long r = 0; r < rows; r += group) {
+        const long long n = std::min(group, rows - r) * S.nx;
+        wv_repitch_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(S.stage.as<T>(), static_cast<const T*>(dev) + r * S.px,
+                                                                           S.nx, S.px, n, 0);
+        BD_LAUNCHED(S.ctx);
+        BD_CUDA(cudaMemcpyAsync(static_cast<T*>(host) + r * S.nx, S.stage.p, n * sizeof(T), cudaMemcpyDeviceToHost, st));
+    }
     BD_CUDA(cudaStreamSynchronize(st));
 }
 

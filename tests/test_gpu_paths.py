@@ -406,6 +406,44 @@ def test_noalloc_steps_equal_the_run(ctx, nx, steps):
     np.testing.assert_allclose(d, exp["dose"], rtol=2.0 ** -44)
 
 
+# --------------------------------------------------------------------------- staging
+def test_checkpoint_memory_of_padded_rows():
+    """A checkpoint of padded rows goes through a staging buffer of bounded size, not one of all
+    the DFT accumulators."""
+    torch = pytest.importorskip("torch")
+    p = layers(131, 200)
+    w = p.params
+    w.n_dft, w.dft_z_lo, w.dft_z_hi, w.dft_len, w.dft_start = 10, 0, 200, 20, 1
+    w.tile_variant = 26
+    with api.Context(0) as c, c.westervelt_session(p) as s:
+        s.advance(20)
+        before = device_bytes(torch)
+        s.checkpoint()
+        held = before - device_bytes(torch)
+    assert held <= 48 << 20
+
+
+def test_fields_through_several_staging_pieces(ctx):
+    """Fields of padded rows larger than the staging buffer, in and out: the c map, the results
+    and a checkpoint's blob are those of the plain kernel's rows."""
+    out, blobs = [], []
+    c = (1500.0 * (1.0 + 0.01 * np.random.default_rng(6).random((160, 250, 251)))).astype(np.float32)   # 40 MB a field
+    p = presets.cfg1(251, 250, 160, 12, heterogeneity=False)
+    p.set_c_map(c)
+    for v in (0, 26):
+        p.params.tile_variant = v
+        with ctx.westervelt_session(p) as s:
+            s.advance(12)
+            blobs.append(s.checkpoint())
+            out.append(s.finish(want=("p_final", "peak", "energy")))
+    assert np.abs(out[0]["p_final"]).max() > 0
+    same(out[1], out[0], "results")
+    assert bytes(blobs[1]) == bytes(blobs[0])
+    with ctx.westervelt_session(p) as s:
+        s.restore(blobs[0])
+        same(s.finish(want=("p_final", "peak", "energy")), out[0], "restored")
+
+
 # --------------------------------------------------------------------------- bubbles
 def test_bubbles_do_not_depend_on_the_batch(ctx):
     """One-warp blocks (batches that fit the resident lanes) and the one-thread-per-bubble
