@@ -458,6 +458,21 @@ def test_bubbles_do_not_depend_on_the_batch(ctx):
     np.testing.assert_array_equal(ctx.gilmore(med, b, ode)[0], whole)
 
 
+def test_bubbles_across_the_launch_shapes(ctx):
+    """A batch larger than the resident lanes of any occupancy (2,048 threads a SM), on the
+    persistent kernel and on four-warp blocks of the static one, against one-warp blocks."""
+    torch = pytest.importorskip("torch")
+    n = 2048 * torch.cuda.get_device_properties(0).multi_processor_count + 1
+    med, ode = presets.cfg2_medium(), presets.cfg2_ode(t_end=1e-12)
+    b = presets.cfg2_bubbles(n, seed=5)
+    ends = np.concatenate([b[:150], b[-107:]])
+    small, _ = ctx.gilmore(med, ends, ode)
+    for schedule in (abi.BD_SCHEDULE_PERSISTENT, abi.BD_SCHEDULE_STATIC):
+        ode.schedule = schedule
+        r, _ = ctx.gilmore(med, b, ode)
+        np.testing.assert_array_equal(np.concatenate([r[:150], r[-107:]]), small)
+
+
 # --------------------------------------------------------------------------- DFT pass
 @pytest.mark.parametrize("precision", [abi.BD_F32, abi.BD_F64])
 @pytest.mark.parametrize("nx,n_dft", [(27, 1), (28, 4), (29, 5), (26, 16)])
