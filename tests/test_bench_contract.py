@@ -33,3 +33,25 @@ def test_reference_arm_json_line():
     assert d["cpu_baseline"]["kind"] == "reference" and d["cpu_baseline"]["value"] == d["value"]
     assert d["e2e"]["value"] == d["value"] and d["e2e"]["h2d_bytes_per_step"] == 0
     assert d["config"]["workload"]
+
+
+@pytest.mark.parametrize("cause", ["no sources", "no compiler"])
+def test_reference_arm_without_the_reference_reports_no_number(monkeypatch, capsys, cause):
+    """Where the reference's kernels cannot be built, the arm says so and times nothing in
+    their place."""
+    import argparse
+
+    import bench
+    from oracle import build as ob
+
+    def build_ref(*a, **k):
+        if cause == "no sources":
+            return None
+        raise RuntimeError("command failed: g++\nsecond line")
+    monkeypatch.setattr(ob, "build_ref", build_ref)
+    bench.run_reference(argparse.Namespace(gpus=1, steps=1, warmup=1), 1, 0)
+    lines = capsys.readouterr().out.splitlines()
+    assert len(lines) == 1
+    d = json.loads(lines[0])
+    assert d["impl"] == "reference" and d["unavailable"] and "\n" not in d["unavailable"]
+    assert "value" not in d and "e2e" not in d
