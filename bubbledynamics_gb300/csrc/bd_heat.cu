@@ -3,8 +3,8 @@
 // slab (bd_heat_slab_*) and bd_trajectory_shifts.  Replaces T:52-105 (kernel)
 // and T:323-573 (host loop).
 //
-// BD_F64: temperature in double, dose increment pow(4|2, T-43) dt exactly as
-//         T:99-102 (reference-faithful mode).
+// BD_F64: temperature in double, dose increment (4|2)^(T-43) dt of T:99-102 with both
+//         powers from one exp2 (pow and exp2 agree to their last bits).
 // BD_F32: theta = T - T_ref in float (the per-step change of about 1e-4 K would
 //         be lost against 300 K in float), source Q in float, the dose rate
 //         R^(T-43) in float and the dose itself accumulated in double (one
@@ -128,6 +128,8 @@ __device__ __forceinline__ float heat_cell(const HeatMat<float>& M, float tc, fl
     return __fadd_rn(t, M.wTa);
 }
 
+// One cell a thread: the FP64 runs (a dose in double), and in FP32 the rows of the
+// allocation-free run that are no whole vectors (a dose of float pairs, no material map).
 template <class real, int DOSE>
 __global__ void heat_step_kernel(const HeatArgs<real> a, int koff) {
     const int ix = blockIdx.x * blockDim.x + threadIdx.x;
@@ -148,7 +150,9 @@ __global__ void heat_step_kernel(const HeatArgs<real> a, int koff) {
     // one cell: T:85-87 (plus the Pennes term -w dt (T - T_art), zero in the reference)
     auto cell = [&](int iz, real tmv, real tcv, real tpv, real sxy, real q) {
         const long long i = (long long)iz * a.plane + col;
-        const int m = a.matmap ? a.matmap[i] : (a.plane_mat ? __ldg(a.plane_mat + iz) : 0);
+        int m = a.plane_mat ? __ldg(a.plane_mat + iz) : 0;
+        if constexpr (sizeof(real) == 8)
+            if (a.matmap) m = a.matmap[i];
         const HeatMat<real>& M = a.mat[m];
         real tn;
         if constexpr (sizeof(real) == 8) tn = tcv * M.a0 + M.kxy * sxy + M.kz * (tpv + tmv) + M.qc * q + M.wTa;
@@ -169,15 +173,9 @@ __global__ void heat_step_kernel(const HeatArgs<real> a, int koff) {
         } else {
             const float inc0 = __fmul_rn(dose_rate((float)tcv + a.T_refm43), (float)a.dt);
             const float inc = __fmul_rn(dose_rate((float)tn + a.T_refm43), (float)a.dt);   // x = T_C - 43
-            if (a.TD) {
-                double d = a.TD[i];
-                if (DOSE == DOSE_BOTH) d = dose_add(d, inc0);
-                a.TD[i] = dose_add(d, inc);
-            } else {
-                float2 d = a.TDf[i];
-                if (DOSE == DOSE_BOTH) d = df_add(d, inc0);
-                a.TDf[i] = df_add(d, inc);
-            }
+            float2 d = a.TDf[i];
+            if (DOSE == DOSE_BOTH) d = df_add(d, inc0);
+            a.TDf[i] = df_add(d, inc);
         }
     };
     auto sxy_at = [&](int iz) {
@@ -425,6 +423,9 @@ static void step_launch(const HeatArgs<real>& a, int koff, int mode, dim3 grid, 
     else heat_step_kernel<real, DOSE_BOTH><<<grid, block, 0, st>>>(a, koff);
 }
 
+static dim3 step_grid(int nx, int ny, int nz, int zb) {
+    return dim3((nx + 31) / 32, (ny + 7) / 8, (nz + zb - 1) / zb);
+}
 static dim3 step4_grid(int px, int ny, int nz, int zb) {
     return dim3((px / 4 + 15) / 16, (ny + 7) / 8, (nz + zb - 1) / zb);
 }
@@ -571,12 +572,12 @@ struct HeatSlab {
     int zb = 0, ze = 0, lo = 0, hi = 0, nzl = 0, zbk = 32;
     long long nl = 0;                              // local cells
     PoolBuf Ta, Tb, Qd, TDd;
-    dim3 grid, grid4;
+    dim3 grid;
 };
 
 struct HeatPlan {
     bd_context* ctx = nullptr;
-    bool f64 = false, vec4 = false, use_graph = true, has_pm = false, has_mm = false;
+    bool f64 = false, use_graph = true, has_pm = false, has_mm = false;
     int nx = 0, ny = 0, nz = 0, n_legs = 0;
     // device rows hold px cells: FP32 rows are padded to whole 16-byte vectors, so
     // that odd row lengths take the four-cell kernel too (213 x 213 x 201: 45 us a
@@ -745,26 +746,15 @@ struct HeatPlan {
             }
         }
         BD_CUDA(cudaStreamSynchronize(q));
-        vec4 = !f64;
         for (HeatSlab& S : sl) {
-            S.zbk = vec4 ? step4_zb(ctx, px, ny, S.nzl) : 32;
-            S.grid = dim3((nx + 31) / 32, (ny + 7) / 8, (S.nzl + S.zbk - 1) / S.zbk);
-            S.grid4 = step4_grid(px, ny, S.nzl, S.zbk);
+            S.zbk = f64 ? 32 : step4_zb(ctx, px, ny, S.nzl);
+            S.grid = f64 ? step_grid(nx, ny, S.nzl, S.zbk) : step4_grid(px, ny, S.nzl, S.zbk);
         }
         // material constants (T:212-217, plus the Pennes term)
         std::memset(&af, 0, sizeof af);
         std::memset(&ad, 0, sizeof ad);
-        for (int k = 0; k < th->n_materials; ++k) {
-            const bd_thermal_material& mt = th->mat[k];
-            const double kk = mt.k_t / (mt.rho * mt.c_t);
-            const double kxy = th->dt * kk / (th->dx * th->dx), kz = th->dt * kk / (th->dz * th->dz);
-            const double w = mt.perfusion * th->dt;
-            const double a0 = 1.0 - 4.0 * kxy - 2.0 * kz - w;
-            const double qc = th->dt / (mt.rho * mt.c_t);
-            const double wTa = w * (mt.T_art - T_ref);
-            af.mat[k] = HeatMat<float>{(float)a0, (float)kxy, (float)kz, (float)qc, (float)wTa};
-            ad.mat[k] = HeatMat<double>{a0, kxy, kz, qc, wTa};
-        }
+        heat_materials<float>(th, T_ref, af.mat);
+        heat_materials<double>(th, T_ref, ad.mat);
         step = 0;
     }
 
@@ -819,7 +809,7 @@ struct HeatPlan {
                 } else {
                     HeatArgs<float> a = af;
                     fill<HeatArgs<float>, float>(a, S, a_to_b);
-                    step4_launch<false>(a, k, mode, S.grid4, st);
+                    step4_launch<false>(a, k, mode, S.grid, st);
                 }
                 BD_LAUNCHED(ctx);
             }
@@ -1160,15 +1150,14 @@ bd_status bd_heat_run_device_noalloc(bd_context* ctx, const bd_thermal* th, floa
         // the caller's rows are not padded: whole-vector rows and 16-byte aligned buffers take the four-cell kernel
         const bool vec = nx % 4 == 0 && (reinterpret_cast<uintptr_t>(d_theta) | reinterpret_cast<uintptr_t>(d_dose)) % 16 == 0;
         a.zb = vec ? step4_zb(ctx, nx, ny, nz) : scalar_zb(ctx, nx, ny, nz);
-        const dim3 grid((nx + 31) / 32, (ny + 7) / 8, (nz + a.zb - 1) / a.zb);
-        const dim3 grid4 = step4_grid(nx, ny, nz, a.zb);
+        const dim3 grid = vec ? step4_grid(nx, ny, nz, a.zb) : step_grid(nx, ny, nz, a.zb);
         for (int64_t k = 0; k < n_steps; ++k) {
             const bool even = k % 2 == 0;                    // even steps read the caller's field
             a.rev = even ? 0 : 1;
             a.Tin = even ? d_theta : sc.theta;
             a.Tout = even ? sc.theta : d_theta;
             const int mode = dose_mode(k, n_steps);
-            if (vec) step4_launch<true>(a, (int)k, mode, grid4, s);
+            if (vec) step4_launch<true>(a, (int)k, mode, grid, s);
             else step_launch(a, (int)k, mode, grid, s);
             BD_LAUNCHED(ctx);
         }

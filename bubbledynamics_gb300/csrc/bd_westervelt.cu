@@ -100,7 +100,7 @@ struct WvSession {
     int maps_tx = 0, maps_ty = 0;
     bool adj_fused = false;     // adjoint: one fused pass per backward step (FP32, nx % 4 == 0)
     CUtensorMap mP0[5], mQ[5], mR[BD_MAX_RELAX][2], mC, mPeak, mEnergy, mMat;
-    bool mat_tile = false;      // the material map travels as a TMA tile (nx % 16 == 0)
+    bool mat_tile = false;      // the material map travels as a TMA tile (px % 16 == 0)
     // segment view (TMA variants only): the pressure levels of the next step are
     // read from, and p^{n+1} written to, caller-chosen buffers instead of the ring
     bool pdl = true;            // launch TMA step kernels with programmatic dependent launch
@@ -226,10 +226,10 @@ static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 }
 
 static CUtensorMap make_map(const WvSession& S, const void* base, bool is_float, int bx, int by,
-                            bool is_u8 = false, long long depth = 0) {
+                            bool is_u8 = false) {
     CUtensorMap m;
     const size_t esz = is_u8 ? 1 : is_float ? 4 : 8;
-    cuuint64_t dims[3] = {(cuuint64_t)S.nx, (cuuint64_t)S.ny, (cuuint64_t)(depth > 0 ? depth : S.nz)};
+    cuuint64_t dims[3] = {(cuuint64_t)S.nx, (cuuint64_t)S.ny, (cuuint64_t)S.nz};
     cuuint64_t strides[2] = {(cuuint64_t)S.px * esz, (cuuint64_t)S.px * S.ny * esz};
     cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, 1};
     cuuint32_t estr[3] = {1, 1, 1};
@@ -554,8 +554,6 @@ static void build_graph(WvSession& S, int mode) {
     BD_CUDA(e);
     S.graph_variant[mode] = S.variant;
 }
-
-static int64_t launches_per_step(const WvSession& S) { return S.any_mur ? 2 : 1; }
 
 static void probe(WvSession& S) {
     unsigned* f = S.flag.as<unsigned>();
@@ -903,7 +901,7 @@ static void setup(WvSession& S, bd_context* ctx, const bd_grid* g, const bd_medi
     S.has_matmap = m->material_map != nullptr;
     S.has_planemat = m->plane_material != nullptr;
     // the paired kernel takes the material map as a uint8 TMA tile when its rows
-    // (nx bytes) are a multiple of 16 bytes, else per cell through the cache
+    // (px bytes) are a multiple of 16 bytes, else per cell through the cache
     S.mat_tile = S.has_matmap && S.px % 16 == 0;
     if (S.has_cmap) {
         S.cmap.alloc(ctx, S.ncell * 4);
@@ -1525,7 +1523,7 @@ static void adjoint_solve(WvSession& S, const bd_focal_loss* loss, double* loss_
         for (int k = 0; k < 5; ++k)
             BD_CUDA(cudaMemcpyAsync(seg[4 - k].p, S.P[(head_of(s0) + k) % 5].p, f, cudaMemcpyDeviceToDevice, st));
         if (use_graphs && seg_direct && s1 - s0 == Kc)
-            captured(rec_graphs, (int)(s0 & 1), Kc * (launches_per_step(S) + 1),
+            captured(rec_graphs, (int)(s0 & 1), 2 * Kc,       // a step and its counter's advance (open faces: no Mur)
                      [&](cudaStream_t cs) { segment_steps(cs, s0, s1); });
         else
             segment_steps(st, s0, s1);

@@ -37,7 +37,6 @@ struct TmaMaps {
     CUtensorMap ro[BD_MAX_RELAX];       // R^{n-2}
     CUtensorMap cmap, peak, energy;
     CUtensorMap mat;                    // box (TX, TY, 1) on the per-cell material map (uint8), when staged
-
 };
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) {

@@ -15,7 +15,8 @@ struct PairCall {
     bool* pdl;                          // programmatic dependent launch (cleared if unavailable)
     cudaStream_t st;
     int tx, ty, zu, nq;                 // tile, planes per barrier, pointwise ring slots
-    int kind;                           // 0: no relaxation, 1: one process + one material + c map, 2: one, 3: two
+    int kind;                           // 0: no relaxation, 1: one process + one material + c map, 2: one, 3: two;
+                                        // 4, 5, 6: 0, 2, 3 without a c map
     int acc;                            // accumulators the step may touch (ACC_*)
 };
 
