@@ -243,8 +243,10 @@ static CUtensorMap make_map(const WvSession& S, const void* base, bool is_float,
     return m;
 }
 
+// Rows of whole 16-byte vectors, the float c map's too (FP64: nx a multiple of four
+// with one, of two without).
 static bool tma_eligible(const WvSession& S) {
-    return (S.px * S.esz) % 16 == 0 && S.nx >= 8;
+    return (S.px * S.esz) % 16 == 0 && !(S.has_cmap && S.px % 4 != 0) && S.nx >= 8;
 }
 
 // The two-cell variants are compiled for FP32 fields with at most two

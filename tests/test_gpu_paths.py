@@ -60,6 +60,25 @@ def test_padded_rows_equal_the_plain_kernel(ctx, nx):
                 same(r, base, "nx %d, variant %d" % (nx, v))
 
 
+@pytest.mark.parametrize("nx", [44, 45, 46])
+def test_fp64_rows_with_a_c_map(ctx, nx):
+    """FP64 rows of 16-byte vectors whose float c map's rows are none (nx = 46): the default
+    is the plain kernel there, a TMA variant is refused, and the bits are the same."""
+    def make(v):
+        p = presets.cfg1(nx, 27, 41, 40, precision=abi.BD_F64)
+        p.params.tile_variant = v
+        return p
+    base = ctx.westervelt(make(0))
+    assert np.abs(base["p_final"]).max() > 0
+    same(ctx.westervelt(make(-1)), base, "default")
+    if nx % 4 == 0:
+        same(ctx.westervelt(make(17)), base, "variant 17")
+    else:
+        with pytest.raises(api.BDError) as e:
+            ctx.westervelt(make(17))
+        assert e.value.status == abi.BD_ERR_INVALID_ARG
+
+
 @pytest.mark.parametrize("nz", [8, 9, 15, 17, 50])
 def test_short_chunks_equal_the_plain_kernel(ctx, nz):
     """Grids that do not fill one wave run in chunks of two planes or more."""
