@@ -382,12 +382,14 @@ __global__ void __launch_bounds__(128, 8) heat_theta4_kernel(const HeatArgs<floa
 }
 
 // Planes per CTA of the FP32 kernels, at most `most`.  A chunk costs its planes plus
-// about 0.7 of a plane's time to start; grids of several waves fill up as CTAs end and
-// pay half a chunk at the end.  The four-cell kernels stop at six planes: 256 x 256 x
+// some of a plane's time to start; grids of several waves fill up as CTAs end and
+// pay part of a chunk at the end.  The four-cell kernels stop at six planes: 256 x 256 x
 // 384 85.5 / 86.4 / 88.3 / 87.3 us a step in chunks of 6 / 8 / 24 / 43 planes, 213 x
 // 213 x 201 38.2 / 40.8 / 39.7 / 43.2 in 6 / 8 / 19 / 24, 150 x 150 x 120 12.8 / 13.0 /
 // 17.2 in 6 / 8 / 16, 96 x 96 x 78 5.5 / 6.5 / 9.2 in 2 / 4 / 8, 72 x 72 x 60 (launch
-// by launch) 6.7 / 7.1 / 8.1 in 1 / 2 / 4.
+// by launch) 6.7 / 7.1 / 8.1 in 1 / 2 / 4.  The 0.7 and 0.5 are round numbers between
+// these times: up to six planes, each size's fastest chunk is the rule's for any
+// 0.7 to 1.2 of a plane and 0.3 to 0.5 of a chunk.
 static int march_zb(bd_context* ctx, long long tiles, int nz, int per_sm, int most) {
     const double slots = (double)ctx->sm_count * std::max(per_sm, 1);
     const int least = (nz + 65534) / 65535;       // a grid has up to 65,535 chunks

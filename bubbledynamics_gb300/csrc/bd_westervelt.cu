@@ -789,7 +789,11 @@ static double frac(double x) { return x - std::floor(x); }
 // plus about six planes' time to fill the pipeline, and a plane more the more
 // warps share an SM.  48 x 48 x 80, 80 x 80 x 96 and 112 x 112 x 128 (one
 // relaxation process, c map): 6.4, 11.0 and 18.4 us a step; the one-cell kernel in
-// 16-plane chunks took 17.6, 19.1 and 25.8.
+// 16-plane chunks took 17.6, 19.1 and 25.8.  The constants were fitted by hand to
+// those times.  Against each of the three tiles over 25 grids of 0.05 to 2 M cells and
+// 150 steps the tile named here is the fastest or within 3 % of it on 17, within 12 %
+// on 24 and 29 % off on one (78 x 71 x 232: 22.5 us a step where 32 x 16 takes 17.5);
+// 5 % of the cost, below what it can tell apart, keeps the larger tile.
 static int untuned_variant(const WvSession& S) {
     if (!tma_eligible(S)) return 0;
     if (S.prec != BD_F32 || S.max_relax > 2) return 17;
